@@ -3,8 +3,13 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <condition_variable>
 #include <cstddef>
 #include <cstring>
+#include <deque>
+#include <exception>
+#include <functional>
+#include <mutex>
 #include <string>
 #include <thread>
 
@@ -161,6 +166,87 @@ void plan_region(const BatchInput& in, int g, int64_t first_read, int64_t first_
   }
 }
 
+// The process's helper threads. They are started when a loop asks for them, wait for the next one, and
+// end after two idle seconds (starting a loop's threads anew took 10-20 us each, 100-200 us of the
+// planning of a batch of a few regions). They run host code only and make no CUDA call. Never destroyed:
+// a helper that waits when the process exits holds nothing. Loops of several callers share the helpers;
+// a caller works on its own loop beside them and never waits for one that has not begun on it, so a
+// process forked from one with helpers, or one that cannot start any, runs its loops by itself.
+class Helpers {
+ public:
+  static Helpers& get() {
+    static Helpers* const h = new Helpers;
+    return *h;
+  }
+
+  // Runs work() on the calling thread and on up to `more` helpers at once; returns when all are done. An
+  // exception of any of them is thrown here, after the others have ended.
+  void run(int more, const std::function<void()>& work) {
+    Job job{&work, 0, nullptr};
+    {
+      std::lock_guard<std::mutex> lock(m_);
+      try {
+        for (int i = 0; i < more; ++i) tickets_.push_back(&job);
+        const int wanted = std::min(static_cast<int>(tickets_.size()), kMost);
+        while (idle_ + starting_ < wanted && total_ < kMost) {
+          std::thread([this] { help(); }).detach();
+          ++total_;
+          ++starting_;
+        }
+      } catch (const std::exception&) {
+        // Fewer helpers than asked for: the caller does what they would have done.
+      }
+    }
+    wake_.notify_all();
+    do_work(job);
+    std::unique_lock<std::mutex> lock(m_);
+    tickets_.erase(std::remove(tickets_.begin(), tickets_.end(), &job), tickets_.end());
+    done_.wait(lock, [&] { return job.active == 0; });
+    if (job.error) std::rethrow_exception(job.error);
+  }
+
+ private:
+  struct Job {
+    const std::function<void()>* work;
+    int active;
+    std::exception_ptr error;
+  };
+  static constexpr int kMost = 64;
+
+  void do_work(Job& job) {
+    try {
+      (*job.work)();
+    } catch (...) {
+      std::lock_guard<std::mutex> lock(m_);
+      if (!job.error) job.error = std::current_exception();
+    }
+  }
+
+  void help() {
+    std::unique_lock<std::mutex> lock(m_);
+    --starting_;
+    for (;;) {
+      ++idle_;
+      const bool some = wake_.wait_for(lock, std::chrono::seconds(2), [&] { return !tickets_.empty(); });
+      --idle_;
+      if (!some) break;
+      Job* const job = tickets_.front();
+      tickets_.pop_front();
+      ++job->active;
+      lock.unlock();
+      do_work(*job);
+      lock.lock();
+      if (--job->active == 0) done_.notify_all();
+    }
+    --total_;
+  }
+
+  std::mutex m_;
+  std::condition_variable wake_, done_;
+  std::deque<Job*> tickets_;
+  int idle_ = 0, starting_ = 0, total_ = 0;
+};
+
 // Runs fn(i) for i in [0, n) on up to `threads` threads, the calling thread among them. Each thread
 // takes the next item when it finishes one, so uneven items (regions of 8 to 256 reads) balance.
 template <class F>
@@ -171,15 +257,10 @@ void parallel_for(int64_t n, int threads, F&& fn) {
     return;
   }
   std::atomic<int64_t> next{0};
-  auto work = [&] {
+  Helpers::get().run(threads - 1, [&] {
     for (int64_t i = next.fetch_add(1, std::memory_order_relaxed); i < n; i = next.fetch_add(1, std::memory_order_relaxed))
       fn(i);
-  };
-  std::vector<std::thread> pool;
-  pool.reserve(static_cast<size_t>(threads) - 1);
-  for (int t = 1; t < threads; ++t) pool.emplace_back(work);
-  work();
-  for (auto& th : pool) th.join();
+  });
 }
 
 int host_threads() { return std::max(1, static_cast<int>(std::thread::hardware_concurrency())); }

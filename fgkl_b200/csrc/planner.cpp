@@ -273,6 +273,8 @@ SortedHaps SortedHaps::make_pd(const std::vector<HapView>& haps, const std::vect
   s.codes.resize(n);
   s.pd_bits.resize(n);
   std::vector<uint8_t> first, later;
+  // Code of each (base, ALT bits) seen, -1 before: one load a column instead of a search of the sets.
+  std::vector<int16_t> code_of(256 * 16, -1);
   for (size_t k = 0; k < n; ++k) {
     const int32_t i = s.order[k];
     const HapView& h = haps[i];
@@ -283,16 +285,16 @@ SortedHaps SortedHaps::make_pd(const std::vector<HapView>& haps, const std::vect
     s.codes[k].resize(h.len);
     for (int32_t j = 0; j < h.len && !s.too_many_sets; ++j) {
       const MatchSet set = MatchSet::of(h.bases[j], f[j]);
-      auto it = std::find(s.match_sets.begin(), s.match_sets.end(), set);
-      if (it == s.match_sets.end()) {
+      int16_t& code = code_of[set.base * 16 + (set.alts >> 3)];
+      if (code < 0) {
         if (s.match_sets.size() >= 256) {
           s.too_many_sets = true;
           break;
         }
+        code = static_cast<int16_t>(s.match_sets.size());
         s.match_sets.push_back(set);
-        it = s.match_sets.end() - 1;
       }
-      s.codes[k][j] = static_cast<uint8_t>(it - s.match_sets.begin());
+      s.codes[k][j] = static_cast<uint8_t>(code);
     }
     first.assign(static_cast<size_t>(h.len), 0);
     later.assign(static_cast<size_t>(h.len), 0);
