@@ -22,7 +22,8 @@ constexpr int kWarpsPerBlock = 4;
 __host__ __device__ constexpr int warps_index(int warps) { return warps <= 1 ? 0 : (warps == 2 ? 1 : 2); }
 
 // ---------------------------------------------------------------------------------------------
-// Arithmetic policies.
+// Arithmetic policies. up and down move a value one lane within groups of G lanes (the first, respectively
+// last, lane of a group receives its own).
 // ---------------------------------------------------------------------------------------------
 
 struct PackedF32 {
@@ -43,11 +44,13 @@ struct PackedF32 {
     else
       v.x = s;
   }
+  template <int G = 32>
   __device__ __forceinline__ static V up(V v) {
-    return make_float2(__shfl_up_sync(kFull, v.x, 1), __shfl_up_sync(kFull, v.y, 1));
+    return make_float2(__shfl_up_sync(kFull, v.x, 1, G), __shfl_up_sync(kFull, v.y, 1, G));
   }
+  template <int G = 32>
   __device__ __forceinline__ static V down(V v) {
-    return make_float2(__shfl_down_sync(kFull, v.x, 1), __shfl_down_sync(kFull, v.y, 1));
+    return make_float2(__shfl_down_sync(kFull, v.x, 1, G), __shfl_down_sync(kFull, v.y, 1, G));
   }
   __device__ __forceinline__ static V sel(bool m0, bool m1, V a, V b) {
     return make_float2(m0 ? a.x : b.x, m1 ? a.y : b.y);
@@ -68,8 +71,14 @@ struct OneF32 {
   __device__ __forceinline__ static V splat(S s) { return s; }
   __device__ __forceinline__ static S get(const V& v, int) { return v; }
   __device__ __forceinline__ static void put(V& v, int, S s) { v = s; }
-  __device__ __forceinline__ static V up(V v) { return __shfl_up_sync(kFull, v, 1); }
-  __device__ __forceinline__ static V down(V v) { return __shfl_down_sync(kFull, v, 1); }
+  template <int G = 32>
+  __device__ __forceinline__ static V up(V v) {
+    return __shfl_up_sync(kFull, v, 1, G);
+  }
+  template <int G = 32>
+  __device__ __forceinline__ static V down(V v) {
+    return __shfl_down_sync(kFull, v, 1, G);
+  }
   __device__ __forceinline__ static V sel(bool m0, bool, V a, V b) { return m0 ? a : b; }
   __device__ __forceinline__ static V max(V a, V b) { return fmaxf(a, b); }
 };
@@ -87,8 +96,14 @@ struct OneF64 {
   __device__ __forceinline__ static V splat(S s) { return s; }
   __device__ __forceinline__ static S get(const V& v, int) { return v; }
   __device__ __forceinline__ static void put(V& v, int, S s) { v = s; }
-  __device__ __forceinline__ static V up(V v) { return __shfl_up_sync(kFull, v, 1); }
-  __device__ __forceinline__ static V down(V v) { return __shfl_down_sync(kFull, v, 1); }
+  template <int G = 32>
+  __device__ __forceinline__ static V up(V v) {
+    return __shfl_up_sync(kFull, v, 1, G);
+  }
+  template <int G = 32>
+  __device__ __forceinline__ static V down(V v) {
+    return __shfl_down_sync(kFull, v, 1, G);
+  }
   __device__ __forceinline__ static V sel(bool m0, bool, V a, V b) { return m0 ? a : b; }
   __device__ __forceinline__ static V max(V a, V b) { return fmax(a, b); }
 };
@@ -120,7 +135,7 @@ struct Consts<true> {
 struct ReadRef {
   int64_t off;  // first byte in the read arrays
   int len;      // 0 = empty component
-  int pad;      // 32 * R - len
+  int pad;      // rows of the lanes that hold the read (32 * R, or G * R for groups of G lanes) - len
 };
 
 __device__ __forceinline__ double err_prob(const BatchView& v, int q) { return __ldg(v.err_prob + (q > 254 ? 254 : q)); }

@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <cmath>
 #include <condition_variable>
 #include <cstddef>
 #include <cstring>
@@ -65,8 +66,12 @@ int single_rows(int len) {
   return rows;
 }
 
+}  // namespace
+
 struct RegionPlan {
-  ProgramBuild prog;
+  SortedHaps set;
+  ForwardPlan fwd;
+  std::vector<ProgramBuild> progs;
   std::vector<HapInfo> haps;
   std::vector<uint8_t> seq;        // prior codes of the distinct sorted haplotypes, concatenated
   std::vector<uint32_t> pd_seq;    // PD: their forward entries (code and deletion bits)
@@ -79,6 +84,8 @@ struct RegionPlan {
   bool extra_codes = false;  // a haplotype byte outside ACGTN: the region runs on the FP64 kernel
   bool generic = false;      // PD: more read bytes than class bits, or more than 256 match sets
 };
+
+namespace {
 
 // PD regions: the reads' distinct bytes become classes 0..30 (first-seen order) and each match-set
 // code the bit set of classes it accepts, so the kernel's prior is one bit test per row.
@@ -114,10 +121,10 @@ void plan_region(const BatchInput& in, int g, int64_t first_read, int64_t first_
     out.read_bases += static_cast<uint64_t>(in.read_off[first_read + r + 1] - in.read_off[first_read + r]);
   if (n_haps == 0 || n_reads == 0) return;
   const bool pd = in.hap_flags != nullptr;
-  SortedHaps s;
+  SortedHaps& s = out.set;
   try {
     s = pd ? SortedHaps::make_pd(views, flags) : SortedHaps::make(views, share);
-    emit_program(s, share && !pd, out.prog);
+    out.fwd = forward_plan(s, share && !pd);
   } catch (const std::exception& e) {
     out.error = e.what();
     return;
@@ -163,6 +170,17 @@ void plan_region(const BatchInput& in, int g, int64_t first_read, int64_t first_
     h.src = src;
     h.len = s.bases[k].len;
     h.pad_[0] = h.pad_[1] = h.pad_[2] = 0;
+  }
+}
+
+// Emits a planned region's programs: its segments in `chunks` runs at most.
+void emit_region(RegionPlan& plan, int chunks) {
+  const std::vector<int32_t> bounds = split_segments(plan.fwd, chunks);
+  plan.progs.resize(bounds.size() - 1);
+  try {
+    for (size_t c = 0; c + 1 < bounds.size(); ++c) emit_program(plan.set, plan.fwd, bounds[c], bounds[c + 1], plan.progs[c]);
+  } catch (const std::exception& e) {
+    plan.error = e.what();
   }
 }
 
@@ -459,11 +477,75 @@ int plan_region_cells(const BatchInput& in, const EngineConfig& cfg, uint64_t* c
       if (rp.generic || len > static_cast<uint64_t>(kMaxBlockRead))
         c += len * distinct_len;
       else
-        c += len * (rp.prog.fwd_columns + rp.prog.bwd_columns);
+        c += len * (rp.fwd.fwd_columns + rp.fwd.bwd_columns);
     }
     cells[g] = rp.error.empty() ? c : 0;
   });
   return FGKL_OK;
+}
+
+// How a batch's first pass is spread: see choose_split.
+int Engine::SplitRule::chunks(const ForwardPlan& p) const {
+  const uint64_t steps = p.steps(), n = p.segs.size();
+  if (steps <= limit || n < 2) return 1;
+  return static_cast<int>(std::min<uint64_t>(n, (steps + limit - 1) / limit));
+}
+
+// Chooses the forms and the split of the first pass. A task's wavefront steps are serial, so a batch with
+// few tasks leaves most of the GPU idle while the longest run: there the reads go one to a warp and each
+// region's segments are spread over several programs, at the cost of the prefixes that these recompute
+// (one region of 64 reads x 16 PD haplotypes: 1.38 -> 0.30 ms with a haplotype a program). A batch with
+// tasks enough for every resident warp keeps one program a region and the forms with the most reads a
+// warp. In between, the step limit is the one that makes the estimate -- the larger of the mean steps a
+// warp gets and the longest program -- smallest (16 uneven regions: 1,400 steps and 0.78 ms; 600 steps
+// 1.11 ms, 3,000 steps 0.98 ms).
+Engine::SplitRule Engine::choose_split(const BatchInput& in, const EngineConfig& cfg, const std::vector<int64_t>& first_read,
+                                       const std::vector<RegionPlan>& plans) const {
+  const int N = in.num_regions;
+  const double warps = 8.0 * sms_;
+  const bool pd = in.hap_flags != nullptr;
+  SplitRule rule;
+  struct Work {
+    double steps, tasks, segs, prefix;
+  };
+  std::vector<Work> work;
+  work.reserve(static_cast<size_t>(N));
+  double reads_steps = 0;  // one read a warp
+  for (int g = 0; g < N; ++g) {
+    const RegionPlan& rp = plans[g];
+    if (rp.fwd.segs.empty()) continue;
+    uint64_t prefix = 0;
+    for (const auto& s : rp.fwd.segs) prefix += static_cast<uint64_t>(s.start);
+    work.push_back({static_cast<double>(rp.fwd.steps()), static_cast<double>(in.region_reads[g]), static_cast<double>(rp.fwd.segs.size()),
+                    static_cast<double>(prefix) / static_cast<double>(rp.fwd.segs.size())});
+    reads_steps += work.back().steps * work.back().tasks;
+  }
+  int reads_per_warp = 1;
+  if (pd && !cfg.double_precision) {
+    if (tuning_.reads_per_warp == 2 && reads_steps / 2 >= kFullSteps * warps) reads_per_warp = rule.pd_reads = 2;
+  } else if (!cfg.double_precision && reads_steps / kQuadReads >= kFullSteps * warps) {
+    rule.quads = true;
+    reads_per_warp = kQuadReads;
+  }
+  for (Work& w : work) w.tasks = std::ceil(w.tasks / reads_per_warp);
+  double total = 0, best = -1;
+  for (const Work& w : work) total += w.steps * w.tasks;
+  for (const double part : {16.0, 4.0, 2.0, 1.4, 1.0, 0.7, 0.5, 0.25, 0.1, 0.02}) {
+    const double limit = std::max(32.0, total / warps * part);
+    double sum = 0, longest = 0;
+    for (const Work& w : work) {
+      const double k = std::min(w.segs, std::max(1.0, std::ceil(w.steps / limit)));
+      const double each = w.steps / k + (k > 1 ? w.prefix + 32 : 0);
+      sum += each * k * w.tasks;
+      longest = std::max(longest, each);
+    }
+    const double time = std::max(sum / warps, longest);
+    if (best < 0 || time < 0.97 * best) {
+      best = time;
+      rule.limit = static_cast<uint64_t>(limit);
+    }
+  }
+  return rule;
 }
 
 int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
@@ -546,14 +628,22 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   parallel_for(N, host_threads(),
                [&](int64_t g) { plan_region(in, static_cast<int>(g), first_read[g], first_hap[g], share, plans[g]); });
 
+  const bool pd = in.hap_flags != nullptr;
+  const SplitRule split = choose_split(in, cfg, first_read, plans);
+  parallel_for(N, host_threads(), [&](int64_t g) {
+    RegionPlan& rp = plans[g];
+    if (rp.error.empty() && !rp.haps.empty()) emit_region(rp, split.chunks(rp.fwd));
+    rp.set = SortedHaps();  // freed here, on the threads that plan
+  });
+
   for (int g = 0; g < N; ++g)
     if (!plans[g].error.empty()) return fail(FGKL_E_UNSUPPORTED, "region " + std::to_string(g) + ": " + plans[g].error);
-  const bool pd = in.hap_flags != nullptr;
 
   planned_.host_plan_ms = ms_since(t_start);
   const auto t_pack = std::chrono::steady_clock::now();
   // Section offsets. Each stream gets kStreamPad zero entries on both sides.
   std::vector<Region> regions(static_cast<size_t>(N));
+  std::vector<Program> progs;
   int64_t n_haps = 0, n_stream = kStreamPad, n_segs = 0, n_sweeps = 0, n_seq = 0, n_pd_seq = 0, n_sigs = 0;
   int max_slots = 1, max_nodes = 1, max_segs = 1;
   std::vector<int64_t> queue_cap(kQueueBins, 0);
@@ -562,25 +652,32 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
     const RegionPlan& rp = plans[g];
     Region& R = regions[g];
     std::memset(&R, 0, sizeof R);
-    Program& p = R.prog;
+    R.prog = static_cast<int32_t>(progs.size());
+    R.n_progs = static_cast<int32_t>(rp.progs.size());
+    R.whole_steps = static_cast<int32_t>(std::min<uint64_t>(rp.fwd.steps(), INT32_MAX / 4));
     auto put_stream = [&](const std::vector<uint32_t>& v, int32_t& off, int32_t& len) {
       off = static_cast<int32_t>(n_stream);
       len = v.empty() ? 0 : static_cast<int32_t>(v.size()) - 1;  // the last entry only carries post events
       n_stream += static_cast<int64_t>(v.size()) + kStreamPad;
     };
-    put_stream(rp.prog.fwd, p.fwd_off, p.fwd_len);
-    put_stream(rp.prog.bwd, p.bwd_off, p.bwd_len);
-    p.seg_off = static_cast<int32_t>(n_segs);
-    p.n_segs = static_cast<int32_t>(rp.prog.segs.size());
-    n_segs += p.n_segs;
-    p.sweep_off = static_cast<int32_t>(n_sweeps);
-    p.n_sweeps = static_cast<int32_t>(rp.prog.sweeps.size());
-    n_sweeps += p.n_sweeps;
-    p.n_slots = rp.prog.n_slots;
-    p.n_nodes = rp.prog.n_nodes;
-    max_slots = std::max(max_slots, rp.prog.n_slots);
-    max_nodes = std::max(max_nodes, rp.prog.n_nodes);
-    max_segs = std::max(max_segs, p.n_segs);
+    for (const ProgramBuild& pb : rp.progs) {
+      Program p{};
+      put_stream(pb.fwd, p.fwd_off, p.fwd_len);
+      put_stream(pb.bwd, p.bwd_off, p.bwd_len);
+      p.seg_off = static_cast<int32_t>(n_segs);
+      p.n_segs = static_cast<int32_t>(pb.segs.size());
+      n_segs += p.n_segs;
+      p.sweep_off = static_cast<int32_t>(n_sweeps);
+      p.n_sweeps = static_cast<int32_t>(pb.sweeps.size());
+      n_sweeps += p.n_sweeps;
+      p.n_slots = pb.n_slots;
+      p.n_nodes = pb.n_nodes;
+      p.seg_first = pb.seg_first;
+      max_slots = std::max(max_slots, pb.n_slots);
+      max_nodes = std::max(max_nodes, pb.n_nodes);
+      max_segs = std::max(max_segs, p.n_segs);
+      progs.push_back(p);
+    }
     R.hap_off = static_cast<int32_t>(n_haps);
     R.n_haps = in.region_haps[g];
     n_haps += static_cast<int64_t>(rp.haps.size());
@@ -609,16 +706,23 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   // regions' tasks come first: regions are visited in that order (ties by index), which lists each
   // bin's tasks longest first without sorting them.
   constexpr int kKinds = kNumKinds;
+  constexpr int kBinRows = kQuadMaxRows + 1 > kRowBins ? kQuadMaxRows + 1 : kRowBins;  // rows-per-lane values of any kind
   struct BinList {
     std::vector<std::pair<uint64_t, Task>> list;
     uint64_t fwd_cells = 0, bwd_cells = 0;  // forward, backward DP cells
   };
-  std::vector<BinList> by_bin(static_cast<size_t>(kKinds) * kRowBins);
-  auto bin_at = [&](Kind kind, int rows) -> BinList& { return by_bin[static_cast<size_t>(kind) * kRowBins + rows]; };
+  std::vector<BinList> by_bin(static_cast<size_t>(kKinds) * kBinRows);
+  auto bin_at = [&](Kind kind, int rows) -> BinList& { return by_bin[static_cast<size_t>(kind) * kBinRows + rows]; };
   std::vector<int> region_order(static_cast<size_t>(N));
   for (int g = 0; g < N; ++g) region_order[g] = g;
-  auto cost_of = [&](int g) { return plans[g].prog.fwd.size() + plans[g].prog.bwd.size() + 31; };
-  std::stable_sort(region_order.begin(), region_order.end(), [&](int a, int b) { return cost_of(a) > cost_of(b); });
+  auto cost_of = [&](int g) {
+    uint64_t most = 0;
+    for (const ProgramBuild& pb : plans[g].progs) most = std::max(most, pb.steps());
+    return most;
+  };
+  std::vector<uint64_t> region_cost(static_cast<size_t>(N));
+  for (int g = 0; g < N; ++g) region_cost[g] = cost_of(g);
+  std::stable_sort(region_order.begin(), region_order.end(), [&](int a, int b) { return region_cost[a] > region_cost[b]; });
   // Each region's tasks, built in parallel (its reads sorted longest first, then packed), then
   // appended to the bins serially in region order.
   struct RegionTask {
@@ -640,12 +744,21 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
     std::vector<RegionTask>& out = region_tasks[g];
     out.reserve(static_cast<size_t>(n_reads));
     auto one = [&](Kind kind, int rows, size_t i) {
-      out.push_back({kind, rows, len_of(order[i]), Task{g, {static_cast<int32_t>(first_read[g] + order[i]), -1}, rows, -1}, 0});
+      out.push_back({kind, rows, len_of(order[i]), Task{g, {static_cast<int32_t>(first_read[g] + order[i]), -1, -1, -1}, rows, -1, 0}, 0});
     };
     auto two = [&](Kind kind, int rows, size_t i) {
       const int32_t a = static_cast<int32_t>(first_read[g] + order[i]);
       const int32_t b = i + 1 < order.size() ? static_cast<int32_t>(first_read[g] + order[i + 1]) : -1;
-      out.push_back({kind, rows, len_of(order[i]) + (i + 1 < order.size() ? len_of(order[i + 1]) : 0), Task{g, {a, b}, rows, -1}, 0});
+      out.push_back({kind, rows, len_of(order[i]) + (i + 1 < order.size() ? len_of(order[i + 1]) : 0), Task{g, {a, b, -1, -1}, rows, -1, 0}, 0});
+    };
+    auto four = [&](size_t i) {
+      Task t{g, {-1, -1, -1, -1}, quad_rows(len_of(order[i])), -1, 0};
+      int len = 0;
+      for (size_t k = 0; k < kQuadReads && i + k < order.size(); ++k) {
+        t.read[k] = static_cast<int32_t>(first_read[g] + order[i + k]);
+        len += len_of(order[i + k]);
+      }
+      out.push_back({Kind::kQuadF32, t.rows, len, t, 0});
     };
     // One task per distinct sorted haplotype of read order[i], strip-mined over row blocks.
     const RegionPlan& rp = plans[g];
@@ -655,7 +768,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       const uint64_t blocks = static_cast<uint64_t>(long_blocks(len, rows));
       for (int k = 0; k < static_cast<int>(rp.haps.size()); ++k)
         if (rp.haps[k].src == k)
-          out.push_back({kind, rows, len, Task{g, {static_cast<int32_t>(first_read[g] + order[i]), -1}, rows, k},
+          out.push_back({kind, rows, len, Task{g, {static_cast<int32_t>(first_read[g] + order[i]), -1, -1, -1}, rows, k, 0},
                          (static_cast<uint64_t>(rp.haps[k].len) + 32) * blocks * static_cast<uint64_t>(rows)});
     };
     size_t i = 0;
@@ -672,7 +785,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
     } else if (pd) {
       // PD in FP32: reads above 248 bases one per warp, the others in pairs (FP32x2) unless the
       // launch configuration asks for one read per warp.
-      for (; i < order.size() && (packed_rows(len_of(order[i])) > 8 || tuning_.reads_per_warp == 1); ++i)
+      for (; i < order.size() && (packed_rows(len_of(order[i])) > 8 || split.pd_reads == 1); ++i)
         one(Kind::kOneF32Pd, single_rows(len_of(order[i])), i);
       for (; i < order.size(); i += 2) two(Kind::kPackedF32Pd, packed_rows(len_of(order[i])), i);
     } else if (cfg.double_precision || plans[g].extra_codes) {
@@ -682,31 +795,36 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       // (more padding rows, other registers and occupancy; the same bits).
       const bool up = tuning_.rows_extra != 0;
       auto single_up = [&](int rows) { return up && rows + 2 <= max_rows(Kind::kOneF32) ? rows + 2 : rows; };  // even, 10..20
-      auto packed_up = [&](int rows) { return up && rows < 8 ? rows + 1 : rows; };
+      auto short_up = [&](int rows) { return up && rows < 8 ? rows + 1 : rows; };
       for (; i < order.size() && packed_rows(len_of(order[i])) > 8; ++i) one(Kind::kOneF32, single_up(single_rows(len_of(order[i]))), i);
-      for (; i < order.size(); i += 2) two(Kind::kPackedF32, packed_up(packed_rows(len_of(order[i]))), i);
+      for (; i < order.size() && (!split.quads || len_of(order[i]) > kQuadMaxRead); ++i) one(Kind::kShortF32, short_up(packed_rows(len_of(order[i]))), i);
+      for (; i < order.size(); i += kQuadReads) four(i);
     }
   });
   {
     std::vector<size_t> bin_size(by_bin.size(), 0);
     for (const auto& v : region_tasks)
-      for (const RegionTask& t : v) ++bin_size[static_cast<size_t>(t.kind) * kRowBins + t.rows];
+      for (const RegionTask& t : v)
+        bin_size[static_cast<size_t>(t.kind) * kBinRows + t.rows] += t.task.hap >= 0 ? 1 : plans[t.task.region].progs.size();
     for (size_t k = 0; k < by_bin.size(); ++k) by_bin[k].list.reserve(bin_size[k]);
   }
   for (const int g : region_order) {
-    const uint64_t cost_cols = cost_of(g);
-    const uint64_t fcols = plans[g].prog.fwd_columns, bcols = plans[g].prog.bwd_columns;
-    for (const RegionTask& t : region_tasks[g]) {
+    const RegionPlan& rp = plans[g];
+    for (RegionTask& t : region_tasks[g]) {
       BinList& bl = bin_at(t.kind, t.rows);
       if (t.task.hap >= 0) {
         // An unshared strip-mined pair: read length x haplotype length forward cells.
         bl.list.push_back({t.cost, t.task});
-        bl.fwd_cells += static_cast<uint64_t>(plans[g].haps[t.task.hap].len) * static_cast<uint64_t>(t.len);
+        bl.fwd_cells += static_cast<uint64_t>(rp.haps[t.task.hap].len) * static_cast<uint64_t>(t.len);
         continue;
       }
-      bl.list.push_back({cost_cols * static_cast<uint64_t>(t.rows), t.task});
-      bl.fwd_cells += fcols * static_cast<uint64_t>(t.len);
-      bl.bwd_cells += bcols * static_cast<uint64_t>(t.len);
+      for (size_t c = 0; c < rp.progs.size(); ++c) {
+        t.task.prog = regions[g].prog + static_cast<int32_t>(c);
+        bl.list.push_back({rp.progs[c].steps() * static_cast<uint64_t>(t.task.rows), t.task});
+      }
+      // The cells of the plan; prefixes that several programs compute count once.
+      bl.fwd_cells += rp.fwd.fwd_columns * static_cast<uint64_t>(t.len);
+      bl.bwd_cells += rp.fwd.bwd_columns * static_cast<uint64_t>(t.len);
     }
   }
   for (const BinList& bl : by_bin) {
@@ -720,8 +838,8 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   for (const BinList& bl : by_bin) n_tasks_all += bl.list.size();
   tasks.reserve(n_tasks_all);
   for (int kind = 0; kind < kKinds; ++kind)
-    for (int rows = 0; rows < kRowBins; ++rows) {
-      const BinList& bl = by_bin[static_cast<size_t>(kind) * kRowBins + rows];
+    for (int rows = 0; rows < kBinRows; ++rows) {
+      const BinList& bl = by_bin[static_cast<size_t>(kind) * kBinRows + rows];
       const auto& list = bl.list;
       if (list.empty()) continue;
       Bin b{static_cast<Kind>(kind), rows, static_cast<int>(tasks.size()), static_cast<int>(list.size()), 0, 0, 0};
@@ -732,17 +850,22 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
         tasks.push_back(e.second);
         cost += e.first;
       }
-      const bool fp32 = b.kind == Kind::kPackedF32 || b.kind == Kind::kOneF32 || b.kind == Kind::kPackedF32Pd || b.kind == Kind::kOneF32Pd;
+      const bool fp32 = b.kind == Kind::kShortF32 || b.kind == Kind::kOneF32 || b.kind == Kind::kPackedF32Pd || b.kind == Kind::kOneF32Pd;
       b.warps = fp32 ? tuning_.warps_per_block : kWarpsPerBlock;
       int per_sm = 0, threads = 0;
       occupancy(b.kind, b.rows, &per_sm, &threads, b.warps);
+      b.warps = threads / 32;
       if (per_sm <= 0) return fail(FGKL_E_CUDA, "kernel instantiation unavailable on this device");
       const int grid = std::max(sms_, per_sm * sms_ * tuning_.grid_percent / 100);
       b.blocks = std::max(1, std::min((b.n_tasks + b.warps - 1) / b.warps, grid));
       first.push_back({cost, b});
     }
-  // The bin with the most work launches first; the others fill the SMs its tail frees.
-  std::stable_sort(first.begin(), first.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+  // The launch with the most work comes last: its many tasks fill the SMs that the others' last ones leave
+  // (before them, their few and as long tasks ran at the end, by themselves). The launches run one after
+  // another all the same: a grid of each at a time, in proportion to its work, took twice as long (62
+  // against 30 ms for 1,024 uneven regions), as warps of several kernels on an SM share its instruction
+  // caches.
+  std::stable_sort(first.begin(), first.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
   for (auto& f : first) bins_.push_back(f.second);
   // Recomputation queues: room for every (read, distinct haplotype) pair of each rows-per-lane bin.
   // Pairs either pass loses (an FP32 underflow, or a joined FP64 result below the backward range)
@@ -794,13 +917,14 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
     scratch_total = std::max(scratch_total, off);
   }
 
-  // Plan blob: regions | haps | stream | segs | sweeps | code tables | haplotype codes | PD entries | PD signatures.
-  size_t o_regions, o_haps, o_stream, o_segs, o_sweeps, o_codes, o_seq, o_pd_seq, o_sigs, blob_bytes = 0;
+  // Plan blob: regions | programs | haps | stream | segs | sweeps | code tables | haplotype codes | PD entries | PD signatures.
+  size_t o_regions, o_progs, o_haps, o_stream, o_segs, o_sweeps, o_codes, o_seq, o_pd_seq, o_sigs, blob_bytes = 0;
   auto section = [&](size_t bytes, size_t& off) {
     off = align_up(blob_bytes, 16);
     blob_bytes = off + bytes;
   };
   section(regions.size() * sizeof(Region), o_regions);
+  section(progs.size() * sizeof(Program), o_progs);
   section(static_cast<size_t>(n_haps) * sizeof(HapInfo), o_haps);
   section(static_cast<size_t>(n_stream) * sizeof(uint32_t), o_stream);
   section(static_cast<size_t>(n_segs) * sizeof(Segment), o_segs);
@@ -850,6 +974,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   {
     uint8_t* blob = st + s_blob;
     std::memcpy(blob + o_regions, regions.data(), regions.size() * sizeof(Region));
+    if (!progs.empty()) std::memcpy(blob + o_progs, progs.data(), progs.size() * sizeof(Program));
     uint32_t* stream = reinterpret_cast<uint32_t*>(blob + o_stream);
     std::memset(stream, 0, kStreamPad * sizeof(uint32_t));
     std::memset(blob + o_seq + n_seq, 0, 16);
@@ -863,12 +988,16 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
         if (!v.empty()) std::memcpy(stream + off, v.data(), v.size() * sizeof(uint32_t));
         std::memset(stream + off + v.size(), 0, kStreamPad * sizeof(uint32_t));
       };
-      put(rp.prog.fwd, R.prog.fwd_off);
-      put(rp.prog.bwd, R.prog.bwd_off);
-      if (!rp.prog.segs.empty())
-        std::memcpy(blob + o_segs + static_cast<size_t>(R.prog.seg_off) * sizeof(Segment), rp.prog.segs.data(), rp.prog.segs.size() * sizeof(Segment));
-      if (!rp.prog.sweeps.empty())
-        std::memcpy(blob + o_sweeps + static_cast<size_t>(R.prog.sweep_off) * sizeof(Sweep), rp.prog.sweeps.data(), rp.prog.sweeps.size() * sizeof(Sweep));
+      for (size_t c = 0; c < rp.progs.size(); ++c) {
+        const ProgramBuild& pb = rp.progs[c];
+        const Program& p = progs[static_cast<size_t>(R.prog) + c];
+        put(pb.fwd, p.fwd_off);
+        put(pb.bwd, p.bwd_off);
+        if (!pb.segs.empty())
+          std::memcpy(blob + o_segs + static_cast<size_t>(p.seg_off) * sizeof(Segment), pb.segs.data(), pb.segs.size() * sizeof(Segment));
+        if (!pb.sweeps.empty())
+          std::memcpy(blob + o_sweeps + static_cast<size_t>(p.sweep_off) * sizeof(Sweep), pb.sweeps.data(), pb.sweeps.size() * sizeof(Sweep));
+      }
       if (!rp.haps.empty()) std::memcpy(blob + o_codes + static_cast<size_t>(g) * 256, rp.codes, 256);
       else std::memset(blob + o_codes + static_cast<size_t>(g) * 256, 0, 256);
       if (!rp.seq.empty()) std::memcpy(blob + o_seq + R.seq_off, rp.seq.data(), rp.seq.size());
@@ -914,6 +1043,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   view_.gcp = d_reads_ + 4 * read_bytes;
   view_.read_off = d_read_off_;
   view_.regions = reinterpret_cast<const Region*>(d_plan_ + o_regions);
+  view_.progs = reinterpret_cast<const Program*>(d_plan_ + o_progs);
   view_.haps = reinterpret_cast<const HapInfo*>(d_plan_ + o_haps);
   view_.stream = reinterpret_cast<const uint32_t*>(d_plan_ + o_stream);
   view_.segs = reinterpret_cast<const Segment*>(d_plan_ + o_segs);

@@ -79,6 +79,9 @@ struct BatchStats {
   double host_fetch_ms = 0;         // waiting for the kernels and copying results out
 };
 
+struct RegionPlan;   // engine.cpp
+struct ForwardPlan;  // planner.h
+
 // Per region, the DP cells a batched run of `in` computes (forward and backward, as the planner
 // emits them): the cost to balance when regions are split across devices. Host only.
 int plan_region_cells(const BatchInput& in, const EngineConfig& cfg, uint64_t* cells, std::string* error);
@@ -131,8 +134,8 @@ class Engine {
   // over (1: one after another; more: bins overlap, the largest first), each first-pass persistent
   // grid as a percentage of the resident-block limit, how many reads an FP32 PD-HMM warp carries
   // (two in FP32x2 at 8 warps per SM, or one at 12), and the first pass's tile shape: rows per lane
-  // of the plain FP32 reads (the fewest that hold the read, or the next the kernels instantiate)
-  // and warps per block of the FP32 first-pass kernels. None changes a result bit. Applies from the
+  // of the plain FP32 reads that go one to a warp (the fewest that hold the read, or the next the
+  // kernels instantiate) and warps per block of the FP32 first-pass kernels but the quad form's. None changes a result bit. Applies from the
   // next prepare().
   struct Tuning {
     int streams = 8;
@@ -160,6 +163,19 @@ class Engine {
     int queue_bin = 0;   // recomputation bins: the queue bin (queue_bin) the tasks come from
     int warps = 4;       // warps per block
   };
+  // The first pass's forms, and the steps above which a region's program is split.
+  struct SplitRule {
+    bool quads = false;         // plain FP32 reads of at most kQuadMaxRead bases go kQuadReads to a warp
+    int pd_reads = 1;           // FP32 PD-HMM reads of at most 248 bases a warp
+    uint64_t limit = ~uint64_t{0};
+    int chunks(const ForwardPlan& p) const;
+  };
+  // Steps a resident warp gets, on average, from which the forms with several reads a warp are taken:
+  // about two haplotypes'. With 16 uneven regions (1,400 steps) four reads a warp and one read a warp
+  // take the same time (0.78 and 0.76 ms); with 1,024, 29.6 and 41.2 ms.
+  static constexpr double kFullSteps = 600;
+  SplitRule choose_split(const BatchInput& in, const EngineConfig& cfg, const std::vector<int64_t>& first_read,
+                         const std::vector<RegionPlan>& plans) const;
   static constexpr int kAuxStreams = 8;
   Tuning tuning_;
   template <class T>

@@ -8,7 +8,7 @@ namespace fgkl {
 
 // Arithmetic of one kernel instantiation.
 enum class Kind : int {
-  kPackedF32 = 0,  // two reads per lane set, FP32x2 arithmetic, rows-per-lane 1..8
+  kShortF32 = 0,   // one read of at most 248 bases, FP32, rows-per-lane 1..8
   kOneF32 = 1,     // one read, FP32, rows-per-lane 10..20 (even)
   kOneF64 = 2,     // one read, FP64, rows-per-lane 1..8 and 10..20 (even)
   kOneF32Pd = 3,   // PD-HMM, one read, FP32, rows-per-lane 1..8 and 10..20 (even)
@@ -24,8 +24,17 @@ enum class Kind : int {
   // the long kinds, with the prior decided by comparing bytes (any read length).
   kGenericF32Pd = 10,
   kGenericF64Pd = 11,
+  kQuadF32 = 12,   // up to four reads, two on each half of the lanes in FP32x2, rows-per-lane 2..14 (even)
 };
-constexpr int kNumKinds = 12;
+constexpr int kNumKinds = 13;
+// Lanes that hold two reads in the quad form, reads a warp, its largest rows-per-lane and its longest
+// read (the first row of the first lane is padding).
+constexpr int kQuadLanes = 16, kQuadReads = 4;
+constexpr int kQuadMaxRows = 14;
+constexpr int kQuadMaxRead = kQuadLanes * kQuadMaxRows - 1;
+// Rows per lane of a read of `len` bases: even values only. Each value is a launch of its own, which ends
+// with the GPU partly idle; the padding of the odd ones' reads costs less.
+__host__ __device__ constexpr int quad_rows(int len) { return (len / kQuadLanes + 2) / 2 * 2; }
 
 // Longest read a single 32 * R-row block holds (lane 0 is padding: 31 rows per lane x 20).
 constexpr int kMaxBlockRead = 620;
@@ -66,7 +75,7 @@ __host__ __device__ inline int queue_bin(int len, bool generic) {
 }
 __host__ __device__ inline int queue_bin_rows(int bin) { return bin % kRowBins; }
 
-inline bool is_long(Kind k) { return static_cast<int>(k) >= static_cast<int>(Kind::kLongF32); }
+inline bool is_long(Kind k) { return k >= Kind::kLongF32 && k <= Kind::kGenericF64Pd; }
 inline bool is_pd(Kind k) {
   return k == Kind::kOneF32Pd || k == Kind::kOneF64Pd || k == Kind::kPackedF32Pd || k == Kind::kLongF32Pd ||
          k == Kind::kLongF64Pd || k == Kind::kGenericF32Pd || k == Kind::kGenericF64Pd;
@@ -108,6 +117,10 @@ size_t scratch_bytes(Kind k, int rows, int max_slots, int max_nodes, int max_seg
 void occupancy(Kind k, int rows, int* blocks_per_sm, int* threads_per_block, int warps_per_block = 4);
 // Launches one persistent grid of `blocks` blocks.
 cudaError_t launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream, int warps_per_block = 4);
+// The quad form (quad.cpp). Warps per block are its own.
+size_t quad_scratch_bytes(int rows, int max_slots, int max_nodes, int max_segs);
+void quad_occupancy(int rows, int* blocks_per_sm, int* threads_per_block);
+cudaError_t quad_launch(int rows, int blocks, const LaunchArgs& args, cudaStream_t stream);
 // PD-HMM instantiations (pd_kernels.cu).
 size_t pd_scratch_bytes(PdForm form, int rows, int max_slots, int max_segs);
 void pd_occupancy(PdForm form, int rows, int* blocks_per_sm, int* threads_per_block, int warps_per_block = 4);

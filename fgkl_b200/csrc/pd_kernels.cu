@@ -438,14 +438,16 @@ __device__ void pd_finalize(const LaunchArgs& a, const Task& task, const Region&
   unsigned long long lost_count = 0;
   for (int k = lane; k < region.n_haps; k += 32) {
     const HapInfo info = a.v.haps[region.hap_off + k];
-    const double factor = a.v.segs[prog.seg_off + info.seg].factor;
+    const int own = info.seg - prog.seg_first;  // another task's, outside the program's segments
+    if (own < 0 || own >= prog.n_segs) continue;
+    const double factor = a.v.segs[prog.seg_off + own].factor;
 #pragma unroll
     for (int c = 0; c < P::NC; ++c) {
       if (task.read[c] < 0) continue;
       const int read_local = task.read[c] - region.read_off;
       double* dst = a.v.out + region.out_off + static_cast<int64_t>(read_local) * region.n_haps + info.order;
       if (dense && !isnan(*dst)) continue;
-      const double raw = __dmul_rn(sc.seg_raw[info.seg * P::NC + c], factor);
+      const double raw = __dmul_rn(sc.seg_raw[own * P::NC + c], factor);
       bool lost = a.min_accept_plain ? !(raw >= C::kMinAccepted) : (raw != raw);
       if (!P::kDouble) lost |= isinf(raw);
       const double result = lost ? __longlong_as_double(0x7ff8000000000000ll) : log10(raw) - C::kLog10Initial;
@@ -480,7 +482,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (PdMinBlocks<P, R>::value
     if (t >= count) break;
     const Task task = a.tasks[t];
     const Region region = a.v.regions[task.region];
-    const Program prog = region.prog;
+    const Program prog = a.v.progs[task.prog];
     ReadRef rd[P::NC];
 #pragma unroll
     for (int c = 0; c < P::NC; ++c) {

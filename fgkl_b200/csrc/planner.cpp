@@ -347,44 +347,96 @@ void code_table(const SortedHaps& s, uint8_t out[256]) {
   for (int c = 0; c < s.num_codes(); ++c) out[s.byte_of_code(c)] = static_cast<uint8_t>(c);
 }
 
-void emit_program(const SortedHaps& s, bool with_suffix, ProgramBuild& out) {
-  const size_t n = s.bases.size();
-  const double init_f64 = std::ldexp(1.0, 1020);
-  const double init_f32 = std::ldexp(1.0, 120);
+namespace {
+// The last earlier segment of [lo, i) passing column q (segment lo starts at column `lo_start`), or -1.
+int32_t last_writer(const std::vector<ForwardPlan::Seg>& segs, int32_t lo, int32_t lo_start, int32_t i, int32_t q) {
+  for (int32_t j = i - 1; j >= lo; --j)
+    if ((j == lo ? lo_start : segs[j].start) < q && q <= segs[j].stop) return j;
+  return -1;
+}
+}  // namespace
 
-  // ---- forward: one segment per distinct sorted haplotype ----
-  struct Seg {
-    int32_t hap, start, stop, len;
-    Cut cut;
-  };
-  std::vector<Seg> segs;
-  for (size_t k = 0; k < n; ++k) {
+ForwardPlan forward_plan(const SortedHaps& s, bool with_suffix) {
+  ForwardPlan p;
+  for (size_t k = 0; k < s.bases.size(); ++k) {
     if (s.dup[k]) continue;
     const int32_t len = s.bases[k].len;
     const Cut cut = with_suffix ? s.plan.cuts[k] : Cut{-1, -1};
     const int32_t stop = cut.column >= 0 ? cut.column - 1 : len;
     if (stop < s.lcp[k]) throw std::logic_error("cut before the shared prefix");
-    segs.push_back(Seg{static_cast<int32_t>(k), s.lcp[k], stop, len, cut});
+    p.segs.push_back(ForwardPlan::Seg{static_cast<int32_t>(k), s.lcp[k], stop, len, 0, cut});
   }
-  const int32_t m = static_cast<int32_t>(segs.size());
-  // The last earlier segment passing each reader's start column wrote the value it resumes from.
-  std::vector<int32_t> writer(m, -1);
-  for (int32_t i = 1; i < m; ++i) {
-    const int32_t q = segs[i].start;
-    if (q == 0) continue;
-    for (int32_t j = i - 1; j >= 0; --j)
-      if (segs[j].start < q && q <= segs[j].stop) {
-        writer[i] = j;
-        break;
+  const int32_t m = static_cast<int32_t>(p.segs.size());
+  // The last earlier segment passing each reader's start column wrote the value it resumes from; each
+  // sharing tree runs at the constant of its longest haplotype (program.h, Segment).
+  std::vector<int32_t> root(m, 0), tree_len(m, 0);
+  std::map<std::pair<int32_t, int32_t>, bool> slots;  // (writer, column) read later than by the next segment
+  for (int32_t i = 0; i < m; ++i) {
+    auto& g = p.segs[i];
+    root[i] = i;
+    if (g.start > 0) {
+      const int32_t w = last_writer(p.segs, 0, p.segs[0].start, i, g.start);
+      if (w < 0) throw std::logic_error("snapshot read before written");
+      root[i] = root[w];
+      if (w != i - 1) slots[{w, g.start}] = true;
+    }
+    tree_len[root[i]] = std::max(tree_len[root[i]], g.len);
+    p.fwd_columns += static_cast<uint64_t>(g.last() - g.start);
+  }
+  for (int32_t i = 0; i < m; ++i) p.segs[i].tree_len = tree_len[root[i]];
+  if (slots.size() >= (s.pd ? kPdPayloadNone : kPayloadNone))
+    throw std::invalid_argument("too many snapshot slots for the stream payload");
+  if (with_suffix && !s.plan.sweeps.empty()) {
+    p.has_backward = true;
+    for (const auto& sw : s.plan.sweeps) p.bwd_columns += static_cast<uint64_t>(sw.need - sw.resume);
+  }
+  return p;
+}
+
+std::vector<int32_t> split_segments(const ForwardPlan& p, int32_t chunks) {
+  const int32_t m = static_cast<int32_t>(p.segs.size());
+  std::vector<int32_t> bounds{0};
+  if (chunks > 1 && m > 1) {
+    // A chunk costs its segments' columns and the prefix that its first segment resumes from.
+    uint64_t prefix = 0;
+    for (const auto& g : p.segs) prefix += static_cast<uint64_t>(g.start);
+    const double target = (static_cast<double>(p.fwd_columns) + (chunks - 1.0) * static_cast<double>(prefix) / m) / chunks;
+    double cost = p.segs[0].last();
+    for (int32_t i = 1; i < m; ++i) {
+      const double own = p.segs[i].last() - p.segs[i].start;
+      const bool must = m - i <= chunks - static_cast<int32_t>(bounds.size());  // one segment a chunk from here
+      if (static_cast<int32_t>(bounds.size()) < chunks && (must || cost + 0.5 * own > target)) {
+        bounds.push_back(i);
+        cost = p.segs[i].last();
+      } else {
+        cost += own;
       }
+    }
+  }
+  bounds.push_back(m);
+  return bounds;
+}
+
+void emit_program(const SortedHaps& s, const ForwardPlan& plan, int32_t lo, int32_t hi, ProgramBuild& out) {
+  const double init_f64 = std::ldexp(1.0, 1020);
+  const double init_f32 = std::ldexp(1.0, 120);
+  const auto& segs = plan.segs;
+  out.seg_first = lo;
+
+  // ---- forward: the segments of distinct sorted haplotypes lo..hi-1, the first from the origin ----
+  auto start_of_seg = [&](int32_t i) { return i == lo ? 0 : segs[i].start; };
+  std::vector<int32_t> writer(static_cast<size_t>(hi), -1);
+  for (int32_t i = lo + 1; i < hi; ++i) {
+    if (segs[i].start == 0) continue;
+    writer[i] = last_writer(segs, lo, 0, i, segs[i].start);
     if (writer[i] < 0) throw std::logic_error("snapshot read before written");
   }
   // Writes keyed by (writer, column): staged for the next segment, and/or a global slot.
   std::map<std::pair<int32_t, int32_t>, std::pair<bool, int32_t>> writes;
-  for (int32_t i = 1; i < m; ++i)
+  for (int32_t i = lo + 1; i < hi; ++i)
     if (writer[i] >= 0) writes[{writer[i], segs[i].start}] = {false, -1};
   int32_t n_slots = 0;
-  for (int32_t i = 1; i < m; ++i) {
+  for (int32_t i = lo + 1; i < hi; ++i) {
     if (writer[i] < 0) continue;
     auto& w = writes[{writer[i], segs[i].start}];
     if (writer[i] == i - 1)
@@ -394,41 +446,57 @@ void emit_program(const SortedHaps& s, bool with_suffix, ProgramBuild& out) {
   }
   // The writes of each segment in column order (the map iterates by writer, then column), so the
   // column loop below meets them with one comparison a column instead of a lookup.
-  std::vector<std::vector<std::pair<int32_t, std::pair<bool, int32_t>>>> writes_of(static_cast<size_t>(m));
+  std::vector<std::vector<std::pair<int32_t, std::pair<bool, int32_t>>>> writes_of(static_cast<size_t>(hi));
   for (const auto& [key, w] : writes) writes_of[static_cast<size_t>(key.first)].push_back({key.second, w});
+  // Backward nodes the segments join, numbered in the plan's order below.
+  const int32_t plan_nodes = plan.has_backward ? s.plan.nodes : 0;
+  std::vector<int32_t> node_id(static_cast<size_t>(plan_nodes), -1);
+  std::vector<uint8_t> node_used(static_cast<size_t>(plan_nodes), 0);
+  for (int32_t i = lo; i < hi; ++i)
+    if (segs[i].cut.column >= 0) node_used[static_cast<size_t>(segs[i].cut.node)] = 1;
+  // A sweep runs when a node that it writes is used, and then uses its start node.
+  const int32_t n_plan_sweeps = plan.has_backward ? static_cast<int32_t>(s.plan.sweeps.size()) : 0;
+  std::vector<uint8_t> sweep_used(static_cast<size_t>(n_plan_sweeps), 0);
+  bool backward = false;
+  for (uint8_t u : node_used) backward |= u != 0;
+  for (int32_t t = n_plan_sweeps - 1; t >= 0; --t) {
+    for (const auto& w : s.plan.sweeps[t].writes) sweep_used[t] |= node_used[static_cast<size_t>(w.second)];
+    if (sweep_used[t]) node_used[static_cast<size_t>(s.plan.sweeps[t].start)] = 1;
+  }
+  int32_t n_nodes = 0;
+  if (backward) {
+    node_used[0] = 1;
+    for (int32_t k = 0; k < plan_nodes; ++k)
+      if (node_used[k]) node_id[k] = n_nodes++;
+  }
   uint32_t pending = 0;  // post events of the previous column, carried by the next entry
   auto push = [&](std::vector<uint32_t>& v, uint32_t e) {
     v.push_back(e | pending);
     pending = 0;
   };
-  // Each sharing tree runs at the constant of its longest haplotype (program.h, Segment).
-  std::vector<int32_t> root(m, 0), tree_len(m, 0);
-  for (int32_t i = 0; i < m; ++i) {
-    root[i] = segs[i].start > 0 ? root[writer[i]] : i;
-    tree_len[root[i]] = std::max(tree_len[root[i]], segs[i].len);
-  }
-  for (int32_t i = 0; i < m; ++i) {
-    const Seg& g = segs[i];
-    const double t_len = static_cast<double>(tree_len[root[i]]);
+  for (int32_t i = lo; i < hi; ++i) {
+    const auto& g = segs[i];
+    const int32_t start = start_of_seg(i);
+    const double t_len = static_cast<double>(g.tree_len);
     Segment rec{};
     rec.hap = g.hap;
-    rec.node = g.cut.column >= 0 ? g.cut.node : -1;
-    rec.staged = g.start > 0 ? 1 : 0;
+    rec.node = g.cut.column >= 0 ? node_id[static_cast<size_t>(g.cut.node)] : -1;
+    rec.staged = start > 0 ? 1 : 0;
     rec.factor = t_len / static_cast<double>(g.len);
     rec.init_d = init_f64 / t_len;
     rec.init_f = static_cast<float>(init_f32 / t_len);
     rec.next_slot = -1;
-    if (i + 1 < m && writer[i + 1] >= 0 && writer[i + 1] < i) rec.next_slot = writes.at({writer[i + 1], segs[i + 1].start}).second;
+    if (i + 1 < hi && writer[i + 1] >= 0 && writer[i + 1] < i) rec.next_slot = writes.at({writer[i + 1], segs[i + 1].start}).second;
     out.segs.push_back(rec);
     // A cut segment also computes its cut column (stop + 1) as an ordinary column.
-    const int32_t last = g.cut.column >= 0 ? g.cut.column : g.stop;
+    const int32_t last = g.last();
     const auto& mine = writes_of[static_cast<size_t>(i)];
     size_t next_write = 0;
-    out.fwd.reserve(out.fwd.size() + static_cast<size_t>(last - g.start) + 1);
-    for (int32_t j = g.start + 1; j <= last; ++j) {
+    out.fwd.reserve(out.fwd.size() + static_cast<size_t>(last - start) + 1);
+    for (int32_t j = start + 1; j <= last; ++j) {
       const bool is_cut = g.cut.column >= 0 && j == g.cut.column;
       const uint32_t pd_bits = s.pd ? s.pd_bits[g.hap][j - 1] : 0u;
-      push(out.fwd, s.codes[g.hap][j - 1] | pd_bits | (j == g.start + 1 ? EV_BEGIN : 0u) | (is_cut ? EV_ACC : 0u));
+      push(out.fwd, s.codes[g.hap][j - 1] | pd_bits | (j == start + 1 ? EV_BEGIN : 0u) | (is_cut ? EV_ACC : 0u));
       if (!is_cut && next_write < mine.size() && mine[next_write].first == j) {
         const auto& w = mine[next_write++].second;
         const uint32_t none = s.pd ? kPdPayloadNone : kPayloadNone;
@@ -439,21 +507,23 @@ void emit_program(const SortedHaps& s, bool with_suffix, ProgramBuild& out) {
     }
     if (next_write != mine.size()) throw std::logic_error("snapshot column outside its writer");
     pending |= g.cut.column >= 0 ? EV_JOIN : EV_END;
-    out.fwd_columns += static_cast<uint64_t>(last - g.start);
   }
   push(out.fwd, 0);
   out.n_slots = n_slots;
 
-  // ---- backward: node 0 from the all-zero column beyond the end, then the plan's sweeps ----
-  out.n_nodes = 0;
-  if (!with_suffix || s.plan.sweeps.empty()) return;
-  const auto& plan = s.plan;
-  const int32_t S = static_cast<int32_t>(plan.sweeps.size()) + 1;
-  std::vector<int32_t> node_writer(static_cast<size_t>(plan.nodes), -1);
+  // ---- backward: node 0 from the all-zero column beyond the end, then the used sweeps, each as far as
+  // its deepest used node ----
+  out.n_nodes = n_nodes;
+  if (!backward) return;
+  std::vector<int32_t> run;  // the sweeps that run, in the plan's order
+  for (int32_t t = 0; t < n_plan_sweeps; ++t)
+    if (sweep_used[t]) run.push_back(t);
+  const int32_t S = static_cast<int32_t>(run.size()) + 1;
+  std::vector<int32_t> node_writer(static_cast<size_t>(plan_nodes), -1);
   node_writer[0] = 0;
   for (int32_t t = 1; t < S; ++t)
-    for (const auto& w : plan.sweeps[t - 1].writes) node_writer[w.second] = t;
-  auto start_of = [&](int32_t t) { return t == 0 ? -1 : plan.sweeps[t - 1].start; };
+    for (const auto& w : s.plan.sweeps[run[t - 1]].writes) node_writer[w.second] = t;
+  auto start_of = [&](int32_t t) { return t == 0 ? -1 : s.plan.sweeps[run[t - 1]].start; };
   pending = 0;
   for (int32_t t = 0; t < S; ++t) {
     Sweep rec{};
@@ -462,35 +532,36 @@ void emit_program(const SortedHaps& s, bool with_suffix, ProgramBuild& out) {
     if (t + 1 < S) {
       const int32_t nxt = start_of(t + 1);
       if (node_writer[nxt] < 0 || node_writer[nxt] > t) throw std::logic_error("sweep starts from an unwritten node");
-      if (node_writer[nxt] < t) rec.next_node = nxt;
+      if (node_writer[nxt] < t) rec.next_node = node_id[static_cast<size_t>(nxt)];
     }
     out.sweeps.push_back(rec);
     auto node_flags = [&](int32_t node) {
       const bool stage = t + 1 < S && start_of(t + 1) == node;
-      return EV_NODE | (stage ? EV_NSTAGE : 0u) | (static_cast<uint32_t>(node) << kPayloadShift);
+      return EV_NODE | (stage ? EV_NSTAGE : 0u) | (static_cast<uint32_t>(node_id[static_cast<size_t>(node)]) << kPayloadShift);
     };
     if (t == 0) {
       push(out.bwd, EV_SWEEP);
       pending |= node_flags(0);
       continue;
     }
-    const auto& sw = plan.sweeps[t - 1];
+    const auto& sw = s.plan.sweeps[run[t - 1]];
+    std::vector<std::pair<int32_t, int32_t>> mine;  // (depth, node) writes in use
+    for (const auto& w : sw.writes)
+      if (node_used[static_cast<size_t>(w.second)]) mine.push_back({w.first, w.second});
     const int32_t len = s.bases[sw.hap].len;
-    const int32_t right = len - sw.resume, left = len - sw.need;
+    const int32_t right = len - sw.resume, left = len - mine.back().first;
     size_t w = 0;
     for (int32_t j = right - 1; j >= left; --j) {
       // Base at column j + 1, emitted moving down-right from column j.
       push(out.bwd, s.codes[sw.hap][j] | (j == right - 1 ? EV_SWEEP : 0u));
-      if (w < sw.writes.size() && len - sw.writes[w].first == j) {
-        pending |= node_flags(sw.writes[w].second);
+      if (w < mine.size() && len - mine[w].first == j) {
+        pending |= node_flags(mine[w].second);
         ++w;
       }
     }
-    if (w != sw.writes.size()) throw std::logic_error("backward write outside its sweep");
-    out.bwd_columns += static_cast<uint64_t>(sw.need - sw.resume);
+    if (w != mine.size()) throw std::logic_error("backward write outside its sweep");
   }
   push(out.bwd, 0);
-  out.n_nodes = plan.nodes;
 }
 
 }  // namespace fgkl

@@ -98,6 +98,29 @@ struct SortedHaps {
   SharedColumns columns() const;
 };
 
+// The forward segments of a sorted set's distinct haplotypes (program.h, Segment), and what a run of all
+// of them computes.
+struct ForwardPlan {
+  struct Seg {
+    int32_t hap, start, stop, len;
+    int32_t tree_len;  // the longest haplotype of its sharing tree
+    Cut cut;
+    // A cut segment also computes its cut column.
+    int32_t last() const { return cut.column >= 0 ? cut.column : stop; }
+  };
+  std::vector<Seg> segs;
+  // Columns of the whole set's forward and backward passes, per read row.
+  uint64_t fwd_columns = 0, bwd_columns = 0;
+  bool has_backward = false;
+  // Wavefront steps of the whole set's program on the 32-lane forms.
+  uint64_t steps() const { return fwd_columns + 32 + (has_backward ? bwd_columns + 1 + 32 : 0); }
+};
+ForwardPlan forward_plan(const SortedHaps& s, bool with_suffix);
+
+// Bounds of `chunks` (at most; one segment a chunk at least) runs of consecutive segments of about equal
+// cost: chunk c holds segments bounds[c] .. bounds[c + 1] - 1.
+std::vector<int32_t> split_segments(const ForwardPlan& p, int32_t chunks);
+
 // Host copy of one program (program.h), before it is concatenated into a batch. Streams hold only
 // the entries of positions 0..n (the last carries the post events of the final column); the
 // kStreamPad zero entries around them are added when the batch is assembled.
@@ -106,18 +129,22 @@ struct ProgramBuild {
   std::vector<Segment> segs;
   std::vector<Sweep> sweeps;
   int32_t n_slots = 0, n_nodes = 0;
-  // Σ(forward columns) and Σ(backward columns) per read row, for the computed-cell count.
-  uint64_t fwd_columns = 0, bwd_columns = 0;
+  int32_t seg_first = 0;  // its first segment, among the set's
+  uint64_t steps() const { return fwd.size() + 31 + (bwd.empty() ? 0 : bwd.size() + 31); }
 };
 
-// The forward (and, with `with_suffix`, backward) column stream of a sorted haplotype set.
+// The column streams of segments lo..hi-1 of a sorted haplotype set: a program by itself, which several
+// of one set run side by side. Segment lo starts from the origin and recomputes the prefix that the
+// whole set's program would resume; the backward pass holds the sweeps whose nodes these segments join.
+// A column's arithmetic, its tree's constant and the cuts are the whole set's, so however a set is
+// split, each pair's result keeps its bits.
 //
 // Snapshot placement: a segment resuming at column q reads the value the LAST earlier segment
 // passing q wrote (the semantics of fgkl's per-column snapshot array, kernel.rs:254-259, :656-662),
 // so each snapshot is written once, by that last writer: into the staging buffer when the very next
 // segment reads it, and into a global slot when a later one does (prefetched into staging at the
 // BEGIN of the segment before its reader).
-void emit_program(const SortedHaps& s, bool with_suffix, ProgramBuild& out);
+void emit_program(const SortedHaps& s, const ForwardPlan& plan, int32_t lo, int32_t hi, ProgramBuild& out);
 
 // 256-entry byte -> prior code table of a sorted set (kNoCode for bytes no haplotype holds that
 // are not A, C, G, T or N).

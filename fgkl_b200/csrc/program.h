@@ -1,7 +1,7 @@
 // Device-program layout shared by the host planner and the sm_100a kernels.
 //
-// A region (one PairHMM call: R reads x H haplotypes) is planned on the host into a program that
-// every read of the region walks, one warp per read task. The forward stream holds one 32-bit entry
+// A region (one PairHMM call: R reads x H haplotypes) is planned on the host into one or more programs
+// that every read of the region walks, a warp per (reads, program) task. The forward stream holds one 32-bit entry
 // per DP column of each distinct sorted haplotype; the backward stream one per backward column of
 // each suffix sweep. An entry's low byte is the prior code of the haplotype base the column emits;
 // its flags name the events a lane handles when it reaches the entry: events that load or keep state
@@ -96,10 +96,16 @@ struct Program {
   int32_t seg_off, n_segs;
   int32_t sweep_off, n_sweeps;
   int32_t n_slots, n_nodes;  // global snapshot slots and backward nodes one read needs
+  int32_t seg_first;         // the region's segment that its first one is (HapInfo::seg)
+  int32_t pad_;
 };
 
 struct Region {
-  Program prog;     // the first pass: prefix (and, when enabled, suffix) sharing
+  // The first pass: prefix (and, when enabled, suffix) sharing. The segments lie in programs prog ..
+  // prog + n_progs - 1, consecutive runs that separate tasks walk.
+  int32_t prog, n_progs;
+  int32_t whole_steps;  // wavefront steps of all segments as one program
+  int32_t pad_;
   int32_t hap_off;  // into the HapInfo array
   int32_t n_haps;
   int32_t read_off; // first global read index
@@ -124,14 +130,18 @@ struct HapInfo {
   int32_t pad_[3];
 };
 
-// One warp's unit of work: one or two reads of a region, with R rows per lane (31 * R >= length).
+// Reads a task holds at most.
+constexpr int kMaxReads = 4;
+
+// One warp's unit of work: one to kMaxReads reads of a region, with R rows per lane.
 // A recomputation task (hap >= 0) runs one read against one distinct haplotype from the origin,
 // without sharing, from a stream synthesised from the haplotype's codes.
 struct Task {
   int32_t region;
-  int32_t read[2];  // global read indices; read[1] = -1 when the task holds one read
+  int32_t read[kMaxReads];  // global read indices; -1 where the task holds fewer
   int32_t rows;     // R
   int32_t hap;      // sorted haplotype of a recomputation task, else -1
+  int32_t prog;     // the program it walks (when hap is -1)
 };
 
 // Per-pass counters written by the kernels.
@@ -150,6 +160,7 @@ struct BatchView {
   const uint8_t* gcp;
   const int64_t* read_off;   // global read -> first byte
   const Region* regions;
+  const Program* progs;
   const HapInfo* haps;
   const uint32_t* stream;
   const Segment* segs;

@@ -1,0 +1,6 @@
+// The quad form at 2 to 8 rows per lane.
+#include "quad_kernel.cuh"
+
+namespace fgkl {
+template struct QuadRange<2, 8>;
+}  // namespace fgkl

@@ -1,0 +1,6 @@
+// The quad form at 12 to 14 rows per lane.
+#include "quad_kernel.cuh"
+
+namespace fgkl {
+template struct QuadRange<12, 14>;
+}  // namespace fgkl

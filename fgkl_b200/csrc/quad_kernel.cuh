@@ -1,0 +1,54 @@
+// Definitions of a range of the quad form (quad.cuh): kLo, kLo + 2, .. kHi rows per lane.
+#pragma once
+#include "plain_kernel.cuh"
+#include "quad.cuh"
+
+namespace fgkl {
+
+namespace {
+constexpr int kQuadWarps = block_warps<kQuadLanes>();
+
+// Calls f with the compile-time value of `rows`, one of R, R + 2, .. kHi.
+template <int R, int kHi, class F>
+void rows_at(int rows, F&& f) {
+  if (rows == R)
+    f(std::integral_constant<int, R>{});
+  else if constexpr (R + 2 <= kHi)
+    rows_at<R + 2, kHi>(rows, f);
+}
+
+template <int R>
+constexpr size_t quad_smem() {
+  return kQuadWarps * Layout<PackedF32, R>::kSmemPerWarp;
+}
+}  // namespace
+
+template <int kLo, int kHi>
+size_t QuadRange<kLo, kHi>::scratch(int rows, int max_slots, int max_nodes, int max_segs) {
+  size_t bytes = 0;
+  rows_at<kLo, kHi>(rows, [&](auto r) { bytes = scratch_size<PackedF32, decltype(r)::value>(max_slots, max_nodes, max_segs); });
+  return bytes;
+}
+
+template <int kLo, int kHi>
+int QuadRange<kLo, kHi>::occupancy(int rows, int* threads) {
+  int blocks = 0;
+  *threads = kQuadWarps * 32;
+  rows_at<kLo, kHi>(rows, [&](auto r) {
+    constexpr int R = decltype(r)::value;
+    static std::atomic<int> cache[kMaxDevices];
+    blocks = resident_blocks(pairhmm_kernel<PackedF32, R, kQuadLanes>, quad_smem<R>(), kQuadWarps * 32, cache);
+  });
+  return blocks;
+}
+
+template <int kLo, int kHi>
+cudaError_t QuadRange<kLo, kHi>::launch(int rows, int blocks, const LaunchArgs& a, cudaStream_t s) {
+  rows_at<kLo, kHi>(rows, [&](auto r) {
+    constexpr int R = decltype(r)::value;
+    pairhmm_kernel<PackedF32, R, kQuadLanes><<<blocks, kQuadWarps * 32, quad_smem<R>(), s>>>(a);
+  });
+  return cudaGetLastError();
+}
+
+}  // namespace fgkl
