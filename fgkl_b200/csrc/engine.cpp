@@ -647,6 +647,8 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   int64_t n_haps = 0, n_stream = kStreamPad, n_segs = 0, n_sweeps = 0, n_seq = 0, n_pd_seq = 0, n_sigs = 0;
   int max_slots = 1, max_nodes = 1, max_segs = 1;
   std::vector<int64_t> queue_cap(kQueueBins, 0);
+  int max_read_len = 1;
+  for (int64_t r = 0; r < total_reads; ++r) max_read_len = std::max(max_read_len, static_cast<int>(in.read_off[r + 1] - in.read_off[r]));
   int max_hap_len = 1;  // scratch of the strip-mined kinds: one carry column per haplotype base
   for (int g = 0; g < N; ++g) {
     const RegionPlan& rp = plans[g];
@@ -710,6 +712,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   struct BinList {
     std::vector<std::pair<uint64_t, Task>> list;
     uint64_t fwd_cells = 0, bwd_cells = 0;  // forward, backward DP cells
+    int row_blocks = 0;                     // strip-mined: the most a read has
   };
   std::vector<BinList> by_bin(static_cast<size_t>(kKinds) * kBinRows);
   auto bin_at = [&](Kind kind, int rows) -> BinList& { return by_bin[static_cast<size_t>(kind) * kBinRows + rows]; };
@@ -815,6 +818,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       if (t.task.hap >= 0) {
         // An unshared strip-mined pair: read length x haplotype length forward cells.
         bl.list.push_back({t.cost, t.task});
+        bl.row_blocks = std::max(bl.row_blocks, long_blocks(t.len, t.rows));
         bl.fwd_cells += static_cast<uint64_t>(rp.haps[t.task.hap].len) * static_cast<uint64_t>(t.len);
         continue;
       }
@@ -851,13 +855,14 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
         cost += e.first;
       }
       const bool fp32 = b.kind == Kind::kShortF32 || b.kind == Kind::kOneF32 || b.kind == Kind::kPackedF32Pd || b.kind == Kind::kOneF32Pd;
-      b.warps = fp32 ? tuning_.warps_per_block : kWarpsPerBlock;
+      const bool pipelined = b.kind == Kind::kLongF32 || b.kind == Kind::kLongF64;
+      b.warps = pipelined ? long_warps(bl.row_blocks) : (fp32 ? tuning_.warps_per_block : kWarpsPerBlock);
       int per_sm = 0, threads = 0;
       occupancy(b.kind, b.rows, &per_sm, &threads, b.warps);
       b.warps = threads / 32;
       if (per_sm <= 0) return fail(FGKL_E_CUDA, "kernel instantiation unavailable on this device");
       const int grid = std::max(sms_, per_sm * sms_ * tuning_.grid_percent / 100);
-      b.blocks = std::max(1, std::min((b.n_tasks + b.warps - 1) / b.warps, grid));
+      b.blocks = std::max(1, std::min(pipelined ? b.n_tasks : (b.n_tasks + b.warps - 1) / b.warps, grid));
       first.push_back({cost, b});
     }
   // The launch with the most work comes last: its many tasks fill the SMs that the others' last ones leave
@@ -892,11 +897,13 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       const Kind kind = q >= 2 * kRowBins ? Kind::kGenericF64Pd
                                           : (q >= kRowBins ? (pd ? Kind::kLongF64Pd : Kind::kLongF64) : (pd ? Kind::kOneF64Pd : Kind::kOneF64));
       int per_sm = 0, threads = 0;
-      occupancy(kind, r, &per_sm, &threads);
-      if (per_sm <= 0) return fail(FGKL_E_CUDA, "recomputation kernel unavailable on this device");
+      const bool pipelined = kind == Kind::kLongF64;
       Bin b{kind, r, queue_off[q], cap, 0, 0, 0};
+      if (pipelined) b.warps = long_warps(long_blocks(max_read_len, r));
+      occupancy(kind, r, &per_sm, &threads, b.warps);
+      if (per_sm <= 0) return fail(FGKL_E_CUDA, "recomputation kernel unavailable on this device");
       b.queue_bin = q;
-      b.blocks = std::max(1, std::min((cap + kWarpsPerBlock - 1) / kWarpsPerBlock, per_sm * sms_));
+      b.blocks = std::max(1, std::min(pipelined ? cap : (cap + kWarpsPerBlock - 1) / kWarpsPerBlock, per_sm * sms_));
       rescue_bins_.push_back(b);
     }
   }

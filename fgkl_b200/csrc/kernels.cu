@@ -76,12 +76,16 @@ __global__ void __launch_bounds__(256) collect_kernel(CollectArgs a) {
 // Strip-mined reads (longer than 620 bases; fgkl sizes its row tables by the batch's longest read,
 // kernel.rs:485-577, so any length is accepted): one read against one distinct haplotype, unshared,
 // from a stream synthesised from the haplotype's codes (the recomputation form above), with the read's
-// rows cut into B = ceil(len / 32R) blocks of 32R rows that the warp runs one after another. The
-// padding rows sit at the top of the first block. Lane 0's row above comes from a carry row instead of
-// its own bottom row: GATK's row 0 (M = X = 0, Y = INITIAL / hap_len) in the first block, the previous
-// block's bottom row after that, which lane 31 writes to the warp's scratch column by column. Lane 0
-// reads column j at step j, and lane 31 of the same block overwrites it at step j + 31 with a value
-// computed from it through the wavefront, so one carry row serves every block in place.
+// rows cut into B = ceil(len / 32R) blocks of 32R rows, the padding rows at the top of the first.
+//
+// A block of W warps runs W consecutive row blocks of a pair as a pipeline: warp w takes what its top row
+// needs from the bottom row of warp w - 1's, column by column, from a ring in shared memory, kDelay
+// supersteps of kChunk columns behind it; a barrier ends each superstep, so nothing waits on a flag. A
+// pair's latency is then n + 64 (W - 1) + 32 steps instead of W (n + 32). More row blocks than warps run
+// as several rounds, the last warp's bottom row going through the block's scratch to the first warp of
+// the next round. (One warp a pair, its row blocks one after another, left 288 reads of about 1,000 bases
+// against 6 haplotypes at 2.6 ms in FP32 and 5.8 ms for the 72 pairs recomputed in FP64, most of the GPU
+// idle.)
 // ---------------------------------------------------------------------------------------------
 
 // What a block's bottom row hands to the next block's top row, per column (FwdState::xs and ts): 8 or
@@ -93,73 +97,68 @@ struct __align__(2 * sizeof(typename P::S)) Carry {
 
 template <class P>
 __host__ __device__ constexpr size_t long_scratch_size(int max_hap_len) {
-  return 16 + static_cast<size_t>(max_hap_len) * sizeof(Carry<P>);
+  return static_cast<size_t>(max_hap_len) * sizeof(Carry<P>);
 }
 
-// One block of a strip-mined pair: rd's pad is relative to the block (negative below the first).
-template <class P, int R>
-__device__ void long_block(const LaunchArgs& a, const ReadRef* rd, int lane, const FwdRows<P, R, 32>& fr, typename P::V an,
-                           Scratch<P, R>& sc, const uint8_t* seq, int n, Carry<P>* carry, const Carry<P>& row0, bool first,
-                           bool last) {
-  FwdState<P, R> st;
-  st.clear();
-  st.cX = row0.x;
-  st.cT = row0.t;
-  const Program prog{};  // unused: the stream is synthesised
-  // Lane 0's carry values for the next iteration's two steps, loaded an iteration ahead.
-  Carry<P> c0 = row0, c1 = row0;
-  auto fetch = [&](Carry<P>& c, int p) {
-    if (!first && lane == 0 && p < n) c = carry[p];
-  };
-  auto step = [&](const Carry<P>& c, uint32_t e, int t) {
-    st.cX = c.x;
-    st.cT = c.t;
-    forward_step<P, R, 32, true, true>(a, prog, rd, lane, fr, an, sc, st, n, e);
-    const int p = t - 31;  // lane 31's position
-    if (!last && lane == 31 && p >= 0 && p < n) carry[p] = Carry<P>{st.xs, st.ts};
-  };
-  fetch(c0, 0);
-  fetch(c1, 1);
-  for (int t = 0; t < n + 32; t += 2) {
-    const uint32_t e0 = synth_entry(seq, n, t - lane), e1 = synth_entry(seq, n, t + 1 - lane);
-    const Carry<P> d0 = c0, d1 = c1;
-    fetch(c0, t + 2);
-    fetch(c1, t + 3);
-    step(d0, e0, t);
-    step(d1, e1, t + 1);
-  }
-}
-
-template <class P, int R>
-struct LongMinBlocks {
-  static constexpr int value = P::kDouble ? 1 : 2;
-};
+// Columns a superstep, and the supersteps a warp starts behind the one above it: at superstep s a warp
+// reads columns up to (s - w kDelay) kChunk - 1 - (kDelay - 1) kChunk + ... of its ring, of which the warp
+// above has written (s - w kDelay + kDelay) kChunk - 32 by the barrier before, so
+// kDelay * kChunk >= kChunk + 31. What that warp writes meanwhile lies behind those columns and at most
+// kDelay * kChunk + kChunk - 32 ahead of the oldest one, so a ring of kRing entries holds both.
+constexpr int kChunk = 32, kDelay = 2, kRing = 128;
+static_assert(kDelay * kChunk >= kChunk + 31 && kRing >= (kDelay + 1) * kChunk, "ring");
 
 template <class P, int R>
 constexpr size_t long_smem_per_warp() {
   using L = Layout<P, R>;
-  return static_cast<size_t>(L::kPriorCodes) * L::kRp * 32 * sizeof(typename P::V);
+  return static_cast<size_t>(L::kPriorCodes) * L::kRp * 32 * sizeof(typename P::V) + kRing * sizeof(Carry<P>);
+}
+
+// One superstep of a warp: columns' steps t0 .. t0 + kChunk - 1. kInner: every lane is strictly inside the
+// haplotype throughout, so no events and no bounds.
+template <class P, int R, bool kInner>
+__device__ __forceinline__ void long_superstep(const LaunchArgs& a, const ReadRef* rd, int lane, const FwdRows<P, R, 32>& fr,
+                                               typename P::V an, Scratch<P, R>& sc, FwdState<P, R>& st, const uint8_t* seq, int n,
+                                               int t0, const Carry<P>* in, Carry<P>* out, int out_mask) {
+  const Program prog{};  // unused: the stream is synthesised
+#pragma unroll 4
+  for (int i = 0; i < kChunk; ++i) {
+    const int t = t0 + i;
+    const uint32_t e = kInner ? __ldg(seq + t - lane) : synth_entry(seq, n, t - lane);
+    const Carry<P> c = in[t & (kRing - 1)];
+    st.cX = c.x;
+    st.cT = c.t;
+    forward_step<P, R, 32, !kInner, true>(a, prog, rd, lane, fr, an, sc, st, n, e);
+    const int p = t - 31;  // lane 31's column
+    if (lane == 31 && out && (kInner || (p >= 0 && p < n))) out[p & out_mask] = Carry<P>{st.xs, st.ts};
+  }
 }
 
 template <class P, int R>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, (LongMinBlocks<P, R>::value)) long_kernel(LaunchArgs a) {
+__global__ void __launch_bounds__(kLongWarps * 32, (P::kDouble || R > 12 ? 1 : 2)) long_kernel(LaunchArgs a) {
   using V = typename P::V;
   using S = typename P::S;
   using C = Consts<P::kDouble>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31;
-  const int warp_in_block = threadIdx.x >> 5;
-  const int warp = blockIdx.x * kWarpsPerBlock + warp_in_block;
-  V* priors = reinterpret_cast<V*>(smem_raw + warp_in_block * long_smem_per_warp<P, R>());
+  __shared__ int s_task;
+  __shared__ double s_raw[kLongWarps][kMaxReads];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  Carry<P>* const rings = reinterpret_cast<Carry<P>*>(smem_raw);  // [warp][kRing]: what the warp's top row takes
+  V* const priors = reinterpret_cast<V*>(rings + warps * kRing) +
+                    static_cast<size_t>(w) * ((long_smem_per_warp<P, R>() - kRing * sizeof(Carry<P>)) / sizeof(V));
+  Carry<P>* const ring = rings + w * kRing;
   const int count = a.count ? min(*a.count, a.n_tasks) : a.n_tasks;
-  char* scratch = a.scratch + static_cast<size_t>(warp) * a.scratch_stride;
-  Carry<P>* carry = reinterpret_cast<Carry<P>*>(scratch + 16);
+  // The block's scratch: one carry entry a column, from the last warp of a round to the first of the next.
+  Carry<P>* const carry = reinterpret_cast<Carry<P>*>(a.scratch + static_cast<size_t>(blockIdx.x) * a.scratch_stride);
+  Scratch<P, R> sc(nullptr, priors, 0, 0, 0);
+  sc.priors = priors;
+  sc.seg_raw = s_raw[w];
   for (;;) {
-    int t = 0;
-    if (lane == 0) t = atomicAdd(a.task_counter, 1);
-    t = __shfl_sync(kFull, t, 0);
-    if (t >= count) break;
-    const Task task = a.tasks[t];
+    if (threadIdx.x == 0) s_task = atomicAdd(a.task_counter, 1);
+    __syncthreads();
+    const int task_i = s_task;
+    if (task_i >= count) break;
+    const Task task = a.tasks[task_i];
     const Region region = a.v.regions[task.region];
     const HapInfo info = a.v.haps[region.hap_off + task.hap];
     const uint8_t* seq = a.v.hap_codes + region.seq_off + info.seq;
@@ -170,41 +169,70 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (LongMinBlocks<P, R>::val
     const int blocks = long_blocks(rd[0].len, R);
     const int pad0 = 32 * R * blocks - rd[0].len;
     const uint8_t* codes = a.v.code_of_byte + region.code_off;
-    Scratch<P, R> sc(scratch, priors, 0, 0, 0);
-    sc.priors = priors;
     // X factor of the read's last row: the accumulated result is the sum of M + mi_n * X^.
     const V an = static_cast<S>(P::kTransformed ? err_prob(a.v, a.v.ins[rd[0].off + rd[0].len - 1]) : 1.0);
-    for (int b = 0; b < blocks; ++b) {
-      rd[0].pad = pad0 - 32 * R * b;
+    for (int b0 = 0; b0 < blocks; b0 += warps) {
+      const int in_round = min(warps, blocks - b0), b = b0 + w;
+      const bool on = w < in_round;
       FwdRows<P, R, 32> fr;
-      fr.load(a.v, rd, lane, codes, priors);
-      // GATK's row 0 above the first block: M = X = 0, Y = INITIAL / hap_len. Below a padding row nothing
-      // reads it.
-      Carry<P> row0{S(0), S(0)};
-      if (b == 0 && pad0 == 0 && lane == 0) {
-        const BracketFactors<P> k(row_model(a.v, rd[0], 0, codes));
-        row0.t = cell_match<P>(S(0), S(0), static_cast<S>(C::kInitial / n), k.k0, k.k1, k.k2);
+      FwdState<P, R> st;
+      st.clear();
+      Carry<P> next{S(0), S(0)};  // the first warp's input for column t0 + kChunk + lane
+      if (on) {
+        rd[0].pad = pad0 - 32 * R * b;
+        fr.load(a.v, rd, lane, codes, priors);
+        if (b == 0) {
+          // GATK's row 0 above the first block: M = X = 0, Y = INITIAL / hap_len. Below a padding row
+          // nothing reads it.
+          if (pad0 == 0) {
+            const BracketFactors<P> k(row_model(a.v, rd[0], 0, codes));
+            next.t = cell_match<P>(S(0), S(0), static_cast<S>(C::kInitial / n), k.k0, k.k1, k.k2);
+          }
+        } else if (w == 0 && lane < n) {
+          next = carry[lane];
+        }
+        __syncwarp();
       }
-      __syncwarp();
-      long_block<P, R>(a, rd, lane, fr, an, sc, seq, n, carry, row0, b == 0, b == blocks - 1);
-      __syncwarp();
+      // The last row block hands nothing on; a round's last warp hands on through the scratch.
+      const bool through_ring = w + 1 < in_round;
+      Carry<P>* const out = !on || b == blocks - 1 ? nullptr : (through_ring ? ring + kRing : carry);
+      const int out_mask = through_ring ? kRing - 1 : -1;
+      const int supersteps = (n + 32 + kChunk - 1) / kChunk + (in_round - 1) * kDelay;
+      for (int s = 0; s < supersteps; ++s) {
+        const int t0 = (s - w * kDelay) * kChunk;
+        if (on && t0 >= 0 && t0 < n + 32) {
+          if (w == 0) {
+            ring[(t0 + lane) & (kRing - 1)] = next;
+            const int col = t0 + kChunk + lane;
+            if (b > 0 && col < n) next = carry[col];
+            __syncwarp();
+          }
+          if (t0 >= 32 && t0 + kChunk <= n)
+            long_superstep<P, R, true>(a, rd, lane, fr, an, sc, st, seq, n, t0, ring, out, out_mask);
+          else
+            long_superstep<P, R, false>(a, rd, lane, fr, an, sc, st, seq, n, t0, ring, out, out_mask);
+        }
+        __syncthreads();
+      }
     }
-    // Thresholds of an unshared pair (fgkl kernel.rs:897-914): FP32 results below 1e-28 or not finite
-    // go to the FP64 recomputation.
-    const double raw = sc.raw(0, 0);
-    bool lost = a.min_accept_plain ? !(raw >= C::kMinAccepted) : (raw != raw);
-    if (!P::kDouble) lost |= isinf(raw);
-    const double result = lost ? __longlong_as_double(0x7ff8000000000000ll) : log10(raw) - C::kLog10Initial;
-    const int read_local = task.read[0] - region.read_off;
-    unsigned long long lost_count = 0;
-    for (int k = lane; k < region.n_haps; k += 32) {
-      const HapInfo h = a.v.haps[region.hap_off + k];
-      if (h.src != task.hap) continue;
-      a.v.out[region.out_off + static_cast<int64_t>(read_local) * region.n_haps + h.order] = result;
-      lost_count += lost;
+    if (w == 0) {
+      // Thresholds of an unshared pair (fgkl kernel.rs:897-914): FP32 results below 1e-28 or not finite
+      // go to the FP64 recomputation.
+      const double raw = s_raw[(blocks - 1) % warps][0];
+      bool lost = a.min_accept_plain ? !(raw >= C::kMinAccepted) : (raw != raw);
+      if (!P::kDouble) lost |= isinf(raw);
+      const double result = lost ? __longlong_as_double(0x7ff8000000000000ll) : log10(raw) - C::kLog10Initial;
+      const int read_local = task.read[0] - region.read_off;
+      unsigned long long lost_count = 0;
+      for (int k = lane; k < region.n_haps; k += 32) {
+        const HapInfo h = a.v.haps[region.hap_off + k];
+        if (h.src != task.hap) continue;
+        a.v.out[region.out_off + static_cast<int64_t>(read_local) * region.n_haps + h.order] = result;
+        lost_count += lost;
+      }
+      if (lost_count) atomicAdd(&a.v.counters->lost_pairs, lost_count);
     }
-    if (lost_count) atomicAdd(&a.v.counters->lost_pairs, lost_count);
-    __syncwarp();
+    __syncthreads();
   }
 }
 
@@ -349,14 +377,15 @@ auto long_rows_wide(int rows, F&& f) {
 }
 
 template <class P, int R>
-void long_occ(int* blocks) {
-  static std::atomic<int> cache[kMaxDevices];
-  *blocks = resident_blocks(long_kernel<P, R>, kWarpsPerBlock * long_smem_per_warp<P, R>(), kWarpsPerBlock * 32, cache);
+void long_occ(int* blocks, int warps) {
+  static std::atomic<int> cache[kLongWarps + 1][kMaxDevices];
+  *blocks = resident_blocks(long_kernel<P, R>, warps * long_smem_per_warp<P, R>(), warps * 32, cache[warps],
+                            kLongWarps * long_smem_per_warp<P, R>());
 }
 
 template <class P, int R>
-cudaError_t long_go(int blocks, const LaunchArgs& a, cudaStream_t s) {
-  long_kernel<P, R><<<blocks, kWarpsPerBlock * 32, kWarpsPerBlock * long_smem_per_warp<P, R>(), s>>>(a);
+cudaError_t long_go(int blocks, const LaunchArgs& a, cudaStream_t s, int warps) {
+  long_kernel<P, R><<<blocks, warps * 32, warps * long_smem_per_warp<P, R>(), s>>>(a);
   return cudaGetLastError();
 }
 
@@ -370,29 +399,32 @@ size_t long_scratch_bytes(Kind k, int rows, int max_hap_len) {
   return k == Kind::kLongF64 ? long_scratch_size<OneF64>(max_hap_len) : long_scratch_size<OneF32>(max_hap_len);
 }
 
-void long_occupancy(Kind k, int rows, int* blocks, int* threads) {
+void long_occupancy(Kind k, int rows, int* blocks, int* threads, int warps) {
   *blocks = 0;
   *threads = kWarpsPerBlock * 32;
   if (!is_long(k) || !valid_long_rows(k, rows)) return;
   if (is_pd(k)) return pd_long_occupancy(k, rows, blocks, threads);
+  *threads = warps * 32;
+  if (warps < 1 || warps > kLongWarps) return;
   if (k == Kind::kLongF64)
     long_rows_narrow(rows, [&](auto r) {
-      long_occ<OneF64, decltype(r)::value>(blocks);
+      long_occ<OneF64, decltype(r)::value>(blocks, warps);
       return 0;
     });
   else
     long_rows_wide(rows, [&](auto r) {
-      long_occ<OneF32, decltype(r)::value>(blocks);
+      long_occ<OneF32, decltype(r)::value>(blocks, warps);
       return 0;
     });
 }
 
-cudaError_t long_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream) {
+cudaError_t long_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream, int warps) {
   if (!is_long(k) || !valid_long_rows(k, rows)) return cudaErrorInvalidValue;
   if (is_pd(k)) return pd_long_launch(k, rows, blocks, args, stream);
+  if (warps < 1 || warps > kLongWarps) return cudaErrorInvalidValue;
   if (k == Kind::kLongF64)
-    return long_rows_narrow(rows, [&](auto r) { return long_go<OneF64, decltype(r)::value>(blocks, args, stream); });
-  return long_rows_wide(rows, [&](auto r) { return long_go<OneF32, decltype(r)::value>(blocks, args, stream); });
+    return long_rows_narrow(rows, [&](auto r) { return long_go<OneF64, decltype(r)::value>(blocks, args, stream, warps); });
+  return long_rows_wide(rows, [&](auto r) { return long_go<OneF32, decltype(r)::value>(blocks, args, stream, warps); });
 }
 
 size_t scratch_bytes(Kind k, int rows, int max_slots, int max_nodes, int max_segs) {
@@ -405,8 +437,8 @@ size_t scratch_bytes(Kind k, int rows, int max_slots, int max_nodes, int max_seg
 void occupancy(Kind k, int rows, int* blocks, int* threads, int warps) {
   *blocks = 0;
   *threads = kWarpsPerBlock * 32;
+  if (is_long(k)) return long_occupancy(k, rows, blocks, threads, warps);
   if (!valid_rows(k, rows) || (warps != 1 && warps != 2 && warps != 4)) return;
-  if (is_long(k)) return long_occupancy(k, rows, blocks, threads);
   if (is_pd(k)) return pd_occupancy(pd_form(k), rows, blocks, threads, warps);
   if (k == Kind::kQuadF32) return quad_occupancy(rows, blocks, threads);
   dispatch<OccF>(k, rows, blocks, threads, warps);
@@ -419,8 +451,8 @@ cudaError_t launch_collect(const CollectArgs& args, int n_regions, cudaStream_t 
 }
 
 cudaError_t launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream, int warps) {
+  if (is_long(k)) return long_launch(k, rows, blocks, args, stream, warps);
   if (!valid_rows(k, rows) || (warps != 1 && warps != 2 && warps != 4)) return cudaErrorInvalidValue;
-  if (is_long(k)) return long_launch(k, rows, blocks, args, stream);
   if (is_pd(k)) return pd_launch(pd_form(k), rows, blocks, args, stream, warps);
   if (k == Kind::kQuadF32) return quad_launch(rows, blocks, args, stream);
   return dispatch<GoF>(k, rows, blocks, args, stream, warps);

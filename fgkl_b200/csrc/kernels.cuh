@@ -61,6 +61,13 @@ __host__ __device__ inline int long_rows(int len, bool wide) {
   return best;
 }
 __host__ __device__ inline int long_blocks(int len, int rows) { return (len + 32 * rows - 1) / (32 * rows); }
+// Warps a block of the plain strip-mined kernels: one a row block up to kLongWarps; more row blocks run in
+// rounds of about equal size.
+constexpr int kLongWarps = 8;
+inline int long_warps(int row_blocks) {
+  const int rounds = (row_blocks + kLongWarps - 1) / kLongWarps;
+  return rounds > 0 ? (row_blocks + rounds - 1) / rounds : 1;
+}
 
 // Recomputation queue bins: rows-per-lane 1..20 of single-block reads, then kRowBins + R for
 // strip-mined reads and 2 * kRowBins + R for the pairs of byte-compared PD regions.
@@ -129,8 +136,8 @@ cudaError_t pd_launch(PdForm form, int rows, int blocks, const LaunchArgs& args,
 // bottom row a block hands to the next, plus the pair's result), occupancy and launch. The plain
 // ones live in kernels.cu, the PD ones in pd_kernels.cu.
 size_t long_scratch_bytes(Kind k, int rows, int max_hap_len);
-void long_occupancy(Kind k, int rows, int* blocks_per_sm, int* threads_per_block);
-cudaError_t long_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream);
+void long_occupancy(Kind k, int rows, int* blocks_per_sm, int* threads_per_block, int warps_per_block);
+cudaError_t long_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream, int warps_per_block);
 size_t pd_long_scratch_bytes(Kind k, int rows, int max_hap_len);
 void pd_long_occupancy(Kind k, int rows, int* blocks_per_sm, int* threads_per_block);
 cudaError_t pd_long_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream);
