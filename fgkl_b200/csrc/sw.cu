@@ -1,25 +1,32 @@
 // sm_100a Smith-Waterman: GATK's SmithWatermanJavaAligner (fgkl crates/smithwaterman/src/reference.rs,
 // lib.rs) over a batch of (reference, alternate) pairs, one warp per pair.
 //
-// Rows are reference positions, on lanes: lane l holds rows l*8+1 .. l*8+8 of a 256-row block, and a
-// longer reference runs as consecutive blocks. Columns are alternate positions, walked as an
-// anti-diagonal wavefront: at step t lane l is at column t - l + 1, and the row above arrives from
-// lane l - 1 by shuffle (lane 0 takes GATK's row 0, or, below the first block, the bottom row the
-// block above stored per column). Per cell (reference.rs:69-110), in integers:
+// Rows are reference positions, on lanes: lane l holds rows l*R+1 .. l*R+R of a 32*R-row block (R = 4, 8 or
+// 16 by the batch's lengths), and a longer reference runs as consecutive blocks. Columns are alternate
+// positions, walked as an anti-diagonal wavefront: at step t lane l is at column t - l + 1, and the row
+// above arrives from lane l - 1 by shuffle (lane 0 takes GATK's row 0, or, below the first block, the bottom
+// row the block above stored per column). Per cell (reference.rs:69-110), in integers:
 //   diag  = H(i-1, j-1) + (ref[i] == alt[j] ? match : mismatch)
 //   F(i, j) = max over the vertical gap: F(i-1, j) + extend, or H(i-1, j) + open when that is larger
 //   E(i, j) = the same along the row from (i, j-1)
 //   H = diag when diag >= F and diag >= E, else E when E >= F, else F; never below -1e8.
 // Each cell keeps one traceback byte: the direction (diagonal, horizontal, vertical) and whether its
 // vertical and its horizontal gap extend the neighbour's (not opened here), from which the traceback
-// recovers GATK's gap lengths. The bytes are stored anti-diagonal-major ([block][step][lane][8
-// rows]), so each step's stores are one contiguous 256-byte run. After the fill, lane 0 picks the
-// end cell from the last column and last row with GATK's tie rules and walks back (reference.rs:
-// 113-203). For the SoftClip and Ignore strategies an alternate that occurs exactly in the
-// reference short-circuits to one match (lib.rs:602-607, the last occurrence), found first by the
-// warp testing 32 start positions at a time.
+// recovers GATK's gap lengths. The bytes are stored anti-diagonal-major ([block][step][lane][R rows]), so
+// each step's stores are one contiguous run. After the fill, the warp picks the end cell from the last
+// column and last row with GATK's tie rules and walks back (reference.rs:113-203). For the SoftClip and
+// Ignore strategies an alternate that occurs exactly in the reference short-circuits to one match
+// (lib.rs:602-607, the last occurrence), found first by the warp testing 32 start positions at a time.
+//
+// The integer ALU pipe bounds the fill (80% active). Measured on 16,384 pairs of 500 x 500 bases: 25 ALU
+// operations a cell, 8 rows a lane 6.31 ms; tagged cells (below) and the traceback by the warp 5.14 ms;
+// steps inside the matrix without edge cases, the end cell's row and column kept only where a strategy
+// looks there 4.43 ms; 16 rows a lane, so that 500 rows are one block and a step's overhead is shared by
+// twice the cells, 3.67 ms (1,112 G cells/s).
+#include <algorithm>
 #include <climits>
 #include <cstdint>
+#include <type_traits>
 
 #include "dp_common.cuh"
 #include "sw.cuh"
@@ -28,16 +35,33 @@ namespace fgkl {
 
 namespace {
 
-constexpr int kBlockRows = 32 * kSwRows;
 constexpr int kCutoff = -100000000;  // GATK's MATRIX_MIN_CUTOFF
 constexpr int kLowInit = INT_MIN / 2;  // GATK's lowInitValue
-constexpr uint32_t kExtV = 4, kExtH = 8;
+
+// The two cell forms. Plain: GATK's scores as they are, floored at -1e8. Tagged (scores small enough, see
+// sw_tagged): a score s is held as 16 s, and the low bits say how it came about, so that the maximum
+// that takes the better score also takes GATK's choice among equal ones and its traceback bits:
+//   F (vertical gap)   bit 0 set: extends the gap above        (a tie extends)
+//   E (horizontal gap) bit 1 set: extends the gap to the left  (a tie extends)
+//   H                  8 + .. diagonal, 4 + .. horizontal, else vertical (ties in that order)
+// A cell is then five add-and-maximum operations, a base comparison with its select and six bit
+// operations instead of 25 compares, selects and adds on the integer ALU pipe, which bounds the kernel.
+constexpr int kTagLow = -1200000000;  // below any tagged score, and so that adding a penalty does not overflow
+template <bool kTagged>
+struct Cell {
+  static constexpr int kLow = kTagged ? kTagLow : kLowInit;
+  static constexpr uint32_t kExtV = kTagged ? 1 : 4, kExtH = kTagged ? 2 : 8;
+  // A traceback byte's direction: 0 diagonal, 1 horizontal, 2 vertical.
+  __device__ static uint32_t dir(uint32_t byte) { return kTagged ? 2u - ((byte >> 2) & 3u) : byte & 3u; }
+};
 
 __host__ __device__ inline size_t sw_align256(size_t x) { return (x + 255) / 256 * 256; }
 
-// A pair's per-warp scratch.
+// A pair's per-warp scratch, at kRows reference rows a lane.
+template <int kRows>
 struct SwScratch {
-  uint8_t* tb;         // [block][step][lane][8 rows]
+  static constexpr int kBlockRows = 32 * kRows;
+  uint8_t* tb;         // [block][step][lane][kRows]
   int32_t* last_col;   // H(i, m), i = 1..n
   int32_t* last_row;   // H(n, j), j = 1..m
   int2* carry;         // bottom row of a block: (H, F) per column
@@ -59,20 +83,41 @@ struct SwScratch {
   }
   // Traceback byte of cell (i, j), 1 <= i <= n, 1 <= j <= m.
   __device__ uint32_t at(int i, int j) const {
-    const int b = (i - 1) / kBlockRows, rl = (i - 1) - b * kBlockRows, ln = rl / kSwRows, r = rl % kSwRows;
+    const int b = (i - 1) / kBlockRows, rl = (i - 1) - b * kBlockRows, ln = rl / kRows, r = rl % kRows;
     const size_t t = static_cast<size_t>(j - 1) + ln;
-    return tb[((static_cast<size_t>(b) * (m + 31) + t) * 32 + ln) * kSwRows + r];
+    return tb[((static_cast<size_t>(b) * (m + 31) + t) * 32 + ln) * kRows + r];
   }
 };
 
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, 8) sw_kernel(SwArgs a) {
+// A lane's traceback bytes of a step, one store.
+__device__ __forceinline__ void store_words(uint8_t* dst, const uint32_t (&w)[1]) { *reinterpret_cast<uint32_t*>(dst) = w[0]; }
+__device__ __forceinline__ void store_words(uint8_t* dst, const uint32_t (&w)[2]) {
+  *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+}
+__device__ __forceinline__ void store_words(uint8_t* dst, const uint32_t (&w)[4]) {
+  *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Resident blocks of four warps per SM: what the registers of kRows rows leave room for.
+constexpr int sw_min_blocks(int rows) { return rows <= 8 ? 8 : 5; }
+
+template <bool kTagged, int kRows>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, sw_min_blocks(kRows)) sw_kernel(SwArgs a) {
+  using C = Cell<kTagged>;
+  constexpr int kBlockRows = 32 * kRows;
+  constexpr int kScale = kTagged ? 16 : 1;
   const int lane = threadIdx.x & 31;
   const int warp = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   char* const base = a.scratch + static_cast<size_t>(warp) * a.stride;
   const bool edge = a.strategy == kSwIndel || a.strategy == kSwLeadingIndel;
-  const int open = a.open, extend = a.extend;
+  const int open = kScale * a.open, extend = kScale * a.extend;
+  // Tagged scores are held with the penalty of opening a gap from them already added, which both gaps take.
+  const int bias = kTagged ? open : 0;
+  const int match = kScale * a.match - bias + (kTagged ? 8 : 0), mismatch = kScale * a.mismatch - bias + (kTagged ? 8 : 0);
   // H of row 0 at column x, and of column 0 at row x (reference.rs:50-62).
-  auto edge_val = [&](int x) { return (edge && x >= 1) ? open + (x - 1) * extend : 0; };
+  auto edge_val = [&](int x) { return bias + ((edge && x >= 1) ? open + (x - 1) * extend : 0); };
+  // The end cell is looked for in the last column (not for Indel) and the last row (SoftClip and Ignore).
+  const bool keep_col = a.strategy != kSwIndel, keep_row = a.strategy == kSwSoftClip || a.strategy == kSwIgnore;
   for (;;) {
     int task = 0;
     if (lane == 0) task = atomicAdd(a.counter, 1);
@@ -110,94 +155,124 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 8) sw_kernel(SwArgs a) {
     }
 
     // The fill, one row block after another.
-    SwScratch sc(base, n, m);
+    SwScratch<kRows> sc(base, n, m);
     const int blocks = (n + kBlockRows - 1) / kBlockRows;
+    const int last_r = (n - 1) % kRows;  // row n among its lane's rows
     for (int b = 0; b < blocks; ++b) {
-      const int top = b * kBlockRows + lane * kSwRows + 1;  // the lane's first row (1-based)
-      int rb[kSwRows], H[kSwRows], E[kSwRows];
+      const int top = b * kBlockRows + lane * kRows + 1;  // the lane's first row (1-based)
+      int rb[kRows], H[kRows], E[kRows];
 #pragma unroll
-      for (int r = 0; r < kSwRows; ++r) {
+      for (int r = 0; r < kRows; ++r) {
         rb[r] = top + r <= n ? static_cast<int>(__ldg(ref + top + r - 1)) : -1;
         H[r] = 0;
-        E[r] = kLowInit;
+        E[r] = C::kLow;
       }
-      const int last_r = (n - top >= 0 && n - top < kSwRows) ? n - top : -1;  // row n among the lane's rows
+      const bool row_here = keep_row && n >= top && n < top + kRows;
       int dH = 0;                  // H of the row above at the previous column (the top row's diagonal)
-      int bH = 0, bF = kLowInit;   // this lane's bottom row at its last column, for the lane below
-      uint8_t* tbb = sc.tb + static_cast<size_t>(b) * (m + 31) * kBlockRows;
-      for (int t = 0; t < m + 31; ++t) {
+      int bH = 0, bF = C::kLow;    // this lane's bottom row at its last column, for the lane below
+      uint8_t* tbb = sc.tb + (static_cast<size_t>(b) * (m + 31) * 32 + lane) * kRows;
+      // Lane 0's row above and every lane's base, loaded a step ahead.
+      int2 above = make_int2(edge_val(1), C::kLow);
+      if (b > 0 && lane == 0) above = sc.carry[0];
+      int base_next = lane == 0 ? static_cast<int>(__ldg(alt)) : 0;
+      // One step. kInner: every lane is past column 1 and before column m.
+      auto step = [&](auto inner, int t) {
+        constexpr bool kInner = decltype(inner)::value;
         const int j = t - lane + 1;
         int uH = __shfl_up_sync(kFull, bH, 1), uF = __shfl_up_sync(kFull, bF, 1);
-        const bool active = j >= 1 && j <= m;
+        const bool active = kInner || (j >= 1 && j <= m);
+        const int ab = base_next;
+        if (kInner || (j >= 0 && j < m)) base_next = static_cast<int>(__ldg(alt + j));
         if (lane == 0) {
-          if (b == 0) {
-            uH = edge_val(j);
-            uF = kLowInit;
-          } else if (active) {
-            const int2 c = sc.carry[j - 1];
-            uH = c.x;
-            uF = c.y;
-          }
+          uH = above.x;
+          uF = above.y;
+          if (b == 0)
+            above.x = edge_val(j + 1);
+          else if (j < m)
+            above = sc.carry[j];
         }
-        if (j == 1) {
+        if (!kInner && j == 1) {
           // Column 0: GATK's edge values, no horizontal gap yet.
 #pragma unroll
-          for (int r = 0; r < kSwRows; ++r) {
+          for (int r = 0; r < kRows; ++r) {
             H[r] = edge_val(top + r);
-            E[r] = kLowInit;
+            E[r] = C::kLow;
           }
           dH = edge_val(top - 1);
         }
-        uint32_t lo = 0, hi = 0;
+        uint32_t words[kRows / 4] = {};
         if (active) {
-          const int ab = __ldg(alt + j - 1);
           int upH = uH, upF = uF, dg = dH;
+          uint32_t bytes[kRows];
 #pragma unroll
-          for (int r = 0; r < kSwRows; ++r) {
-            const int sd = dg + (rb[r] == ab ? a.match : a.mismatch);
-            // A gap extends the neighbour's unless opening here scores strictly more. H is the largest
-            // of the three: the diagonal when it is at least both gaps, else the horizontal gap when it
-            // is at least the vertical one (so max(sd, max(E, F)) and one compare decide it).
-            const int fe = upF + extend, fo = upH + open;
-            const int F = max(fe, fo);
-            const int ee = E[r] + extend, eo = H[r] + open;
-            E[r] = max(ee, eo);
-            const int gap = max(E[r], F);
-            const uint32_t dir = sd >= gap ? 0u : (E[r] >= F ? 1u : 2u);
-            int h = max(sd, gap);
-            h = h > kCutoff ? h : kCutoff;
-            const uint32_t byte = dir | (fe >= fo ? kExtV : 0u) | (ee >= eo ? kExtH : 0u);
-            if (r < 4)
-              lo |= byte << (8 * r);
-            else
-              hi |= byte << (8 * (r - 4));
-            dg = H[r];
-            H[r] = h;
-            upH = h;
-            upF = F;
+          for (int r = 0; r < kRows; ++r) {
+            if constexpr (kTagged) {
+              const int F = __viaddmax_s32(upF | 1, extend, upH);
+              E[r] = __viaddmax_s32(E[r] | 2, extend, H[r]);
+              const int h = __viaddmax_s32(dg, rb[r] == ab ? match : mismatch, __viaddmax_s32(E[r], 4, F));
+              // The direction from H, the horizontal flag from E, the vertical one from F; the bits above
+              // are not read.
+              bytes[r] = (static_cast<uint32_t>(h) & 12u) | (static_cast<uint32_t>(E[r]) & ~12u);
+              bytes[r] = (bytes[r] & ~1u) | (static_cast<uint32_t>(F) & 1u);
+              dg = H[r];
+              H[r] = (h & ~15) + open;
+              upH = H[r];
+              upF = F;
+            } else {
+              const int sd = dg + (rb[r] == ab ? match : mismatch);
+              // A gap extends the neighbour's unless opening here scores strictly more. H is the largest
+              // of the three: the diagonal when it is at least both gaps, else the horizontal gap when it
+              // is at least the vertical one (so max(sd, max(E, F)) and one compare decide it).
+              const int fe = upF + extend, fo = upH + open;
+              const int F = max(fe, fo);
+              const int ee = E[r] + extend, eo = H[r] + open;
+              E[r] = max(ee, eo);
+              const int gap = max(E[r], F);
+              const uint32_t dir = sd >= gap ? 0u : (E[r] >= F ? 1u : 2u);
+              int h = max(sd, gap);
+              h = h > kCutoff ? h : kCutoff;
+              bytes[r] = dir | (fe >= fo ? C::kExtV : 0u) | (ee >= eo ? C::kExtH : 0u);
+              dg = H[r];
+              H[r] = h;
+              upH = h;
+              upF = F;
+            }
           }
+#pragma unroll
+          for (int q = 0; q < kRows / 4; ++q)
+            words[q] = __byte_perm(__byte_perm(bytes[4 * q], bytes[4 * q + 1], 0x0040),
+                                   __byte_perm(bytes[4 * q + 2], bytes[4 * q + 3], 0x0040), 0x5410);
           bH = upH;
           bF = upF;
           // The last row and the last column, for the end cell: the lane holding the reference's last
           // row stores its H at every column, and each lane stores its rows once, at the last column.
-          // Kept out of the row loop, where they were a compare and a predicated store per cell.
-          if (last_r >= 0) {
-            int v = H[0];
+          if (row_here) {
+            // H[last_r], halving the candidates by a bit of last_r at a time (the same in every lane).
+            int v[kRows];
 #pragma unroll
-            for (int r = 1; r < kSwRows; ++r)
-              if (r == last_r) v = H[r];
-            sc.last_row[j - 1] = v;
+            for (int r = 0; r < kRows; ++r) v[r] = H[r];
+#pragma unroll
+            for (int half = kRows / 2; half > 0; half /= 2)
+#pragma unroll
+              for (int r = 0; r < half; ++r) v[r] = (last_r & half) ? v[r + half] : v[r];
+            sc.last_row[j - 1] = v[0];
           }
-          if (j == m) {
+          if (!kInner && keep_col && j == m) {
 #pragma unroll
-            for (int r = 0; r < kSwRows; ++r)
+            for (int r = 0; r < kRows; ++r)
               if (top + r <= n) sc.last_col[top + r - 1] = H[r];
           }
           if (lane == 31 && b + 1 < blocks) sc.carry[j - 1] = make_int2(bH, bF);
         }
         dH = uH;
-        *reinterpret_cast<uint2*>(tbb + (static_cast<size_t>(t) * 32 + lane) * kSwRows) = make_uint2(lo, hi);
-      }
+        store_words(tbb + static_cast<size_t>(t) * kBlockRows, words);
+      };
+      // Steps 32 .. m - 2 are inside in every lane.
+      int t = 0;
+      for (; t < min(32, m + 31); ++t) step(std::false_type{}, t);
+#pragma unroll 2
+      for (; t <= m - 2; ++t) step(std::true_type{}, t);
+      for (; t < m + 31; ++t) step(std::false_type{}, t);
       __syncwarp();
     }
     __threadfence_block();
@@ -256,57 +331,76 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 8) sw_kernel(SwArgs a) {
       }
     }
 
-    // Traceback (reference.rs:144-203), lane 0.
-    if (lane == 0) {
-      // Elements last to first, reversed at the end.
-      int e = 0;
-      if (seg > 0 && a.strategy == kSwSoftClip) {
-        cig[e++] = (static_cast<uint32_t>(seg) << 4) | kSwOpS;
-        seg = 0;
-      }
-      uint32_t state = kSwOpM;
-      do {
-        const uint32_t byte = sc.at(p1, p2);
-        const uint32_t dir = byte & 3u;
-        uint32_t next;
-        int step = 1;
-        if (dir == 2) {
-          next = kSwOpD;
-          // GATK's gap length: one more than the run of extending cells above (row 1 always opens).
-          for (int q = p1; q > 1 && (sc.at(q, p2) & kExtV); --q) ++step;
-          p1 -= step;
-        } else if (dir == 1) {
-          next = kSwOpI;
-          for (int q = p2; q > 1 && (sc.at(p1, q) & kExtH); --q) ++step;
-          p2 -= step;
-        } else {
-          next = kSwOpM;
-          p1 -= 1;
-          p2 -= 1;
-        }
-        if (next == state) {
-          seg += step;
-        } else {
-          if (seg > 0) cig[e++] = (static_cast<uint32_t>(seg) << 4) | state;
-          seg = step;
-          state = next;
-        }
-      } while (p1 > 0 && p2 > 0);
-      int off = 0;
-      if (a.strategy == kSwSoftClip) {
-        cig[e++] = (static_cast<uint32_t>(seg) << 4) | state;
-        if (p2 > 0) cig[e++] = (static_cast<uint32_t>(p2) << 4) | kSwOpS;
-        off = p1;
-      } else if (a.strategy == kSwIgnore) {
-        cig[e++] = (static_cast<uint32_t>(seg + p2) << 4) | state;
-        off = p1 - p2;
+    // Traceback (reference.rs:144-203), by the warp: 32 cells of a diagonal run, or of a gap, at a time (one
+    // lane following one cell after another waited on a load for each). Elements last to first, reversed at
+    // the end; lane 0 writes them.
+    int e = 0;
+    auto put = [&](int len, uint32_t op) {
+      if (lane == 0) cig[e] = (static_cast<uint32_t>(len) << 4) | op;
+      ++e;
+    };
+    if (seg > 0 && a.strategy == kSwSoftClip) {
+      put(seg, kSwOpS);
+      seg = 0;
+    }
+    uint32_t state = kSwOpM;
+    do {
+      // The diagonal from (p1, p2): lane l looks at the l-th cell up it.
+      const int i = p1 - lane, j = p2 - lane;
+      const bool in = i > 0 && j > 0;
+      const uint32_t dir = in ? C::dir(sc.at(i, j)) : 3u;
+      const uint32_t here = __shfl_sync(kFull, dir, 0);
+      uint32_t next;
+      int step = 0;
+      if (here == 0) {
+        next = kSwOpM;
+        const unsigned off_diagonal = __ballot_sync(kFull, dir != 0);
+        step = off_diagonal ? __ffs(off_diagonal) - 1 : 32;
+        p1 -= step;
+        p2 -= step;
       } else {
-        cig[e++] = (static_cast<uint32_t>(seg) << 4) | state;
-        if (p1 > 0)
-          cig[e++] = (static_cast<uint32_t>(p1) << 4) | kSwOpD;
-        else if (p2 > 0)
-          cig[e++] = (static_cast<uint32_t>(p2) << 4) | kSwOpI;
+        // GATK's gap length: one more than the run of extending cells before this one (the first row or
+        // column always opens).
+        const bool vertical = here == 2;
+        next = vertical ? kSwOpD : kSwOpI;
+        const int from = vertical ? p1 : p2;
+        unsigned opens = 0;
+        while (!opens) {
+          const int q = from - step - lane;
+          const bool extends = q > 1 && (sc.at(vertical ? q : p1, vertical ? p2 : q) & (vertical ? C::kExtV : C::kExtH)) != 0;
+          opens = __ballot_sync(kFull, !extends);
+          step += opens ? __ffs(opens) - 1 : 32;
+        }
+        ++step;
+        if (vertical)
+          p1 -= step;
+        else
+          p2 -= step;
       }
+      if (next == state) {
+        seg += step;
+      } else {
+        if (seg > 0) put(seg, state);
+        seg = step;
+        state = next;
+      }
+    } while (p1 > 0 && p2 > 0);
+    int off = 0;
+    if (a.strategy == kSwSoftClip) {
+      put(seg, state);
+      if (p2 > 0) put(p2, kSwOpS);
+      off = p1;
+    } else if (a.strategy == kSwIgnore) {
+      put(seg + p2, state);
+      off = p1 - p2;
+    } else {
+      put(seg, state);
+      if (p1 > 0)
+        put(p1, kSwOpD);
+      else if (p2 > 0)
+        put(p2, kSwOpI);
+    }
+    if (lane == 0) {
       for (int x = 0, y = e - 1; x < y; ++x, --y) {
         const uint32_t tmp = cig[x];
         cig[x] = cig[y];
@@ -361,7 +455,28 @@ __global__ void __launch_bounds__(kCompactThreads) sw_compact_kernel(const uint3
 
 }  // namespace
 
-size_t sw_scratch_bytes(int64_t ref_len, int64_t alt_len) { return SwScratch::bytes(ref_len, alt_len); }
+bool sw_tagged(int64_t longest, int match, int mismatch, int open, int extend) {
+  int64_t most = 0;
+  for (const int64_t v : {int64_t{match}, int64_t{mismatch}, int64_t{open}, int64_t{extend}}) most = std::max(most, v < 0 ? -v : v);
+  // No score or gap is further from zero than `most` a row and column; 16 times that and a further penalty
+  // must stay above kTagLow, and above the plain form's floor, so that the floor is never met.
+  return most * (longest + 2) <= 50000000;
+}
+
+namespace {
+template <class F>
+auto sw_at(int rows, F&& f) {
+  switch (rows) {
+    case 4: return f(std::integral_constant<int, 4>{});
+    case 8: return f(std::integral_constant<int, 8>{});
+    default: return f(std::integral_constant<int, 16>{});
+  }
+}
+}  // namespace
+
+size_t sw_scratch_bytes(int rows, int64_t ref_len, int64_t alt_len) {
+  return sw_at(rows, [&](auto r) { return SwScratch<decltype(r)::value>::bytes(ref_len, alt_len); });
+}
 
 cudaError_t sw_compact(const uint32_t* cigar, const int64_t* slot, const int32_t* count, int n_pairs, uint32_t* packed,
                        cudaStream_t stream) {
@@ -370,14 +485,26 @@ cudaError_t sw_compact(const uint32_t* cigar, const int64_t* slot, const int32_t
   return cudaGetLastError();
 }
 
-void sw_occupancy(int* blocks_per_sm, int* threads_per_block) {
+void sw_occupancy(int rows, bool tagged, int* blocks_per_sm, int* threads_per_block) {
   *threads_per_block = kWarpsPerBlock * 32;
-  static std::atomic<int> cache[kMaxDevices];
-  *blocks_per_sm = resident_blocks(sw_kernel, 0, kWarpsPerBlock * 32, cache);
+  sw_at(rows, [&](auto r) {
+    constexpr int R = decltype(r)::value;
+    static std::atomic<int> cache[2][kMaxDevices];
+    *blocks_per_sm = tagged ? resident_blocks(sw_kernel<true, R>, 0, kWarpsPerBlock * 32, cache[1])
+                            : resident_blocks(sw_kernel<false, R>, 0, kWarpsPerBlock * 32, cache[0]);
+    return 0;
+  });
 }
 
-cudaError_t sw_launch(int blocks, const SwArgs& a, cudaStream_t stream) {
-  sw_kernel<<<blocks, kWarpsPerBlock * 32, 0, stream>>>(a);
+cudaError_t sw_launch(int rows, int blocks, const SwArgs& a, cudaStream_t stream) {
+  sw_at(rows, [&](auto r) {
+    constexpr int R = decltype(r)::value;
+    if (a.tagged)
+      sw_kernel<true, R><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(a);
+    else
+      sw_kernel<false, R><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(a);
+    return 0;
+  });
   return cudaGetLastError();
 }
 
