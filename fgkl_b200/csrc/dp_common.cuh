@@ -22,7 +22,7 @@ constexpr int kWarpsPerBlock = 4;
 __host__ __device__ constexpr int warps_index(int warps) { return warps <= 1 ? 0 : (warps == 2 ? 1 : 2); }
 
 // ---------------------------------------------------------------------------------------------
-// Arithmetic policies. up and down move a value one lane within groups of G lanes (the first, respectively
+// Arithmetic policies. kTable: priors come from a table by haplotype code. up and down move a value one lane within groups of G lanes (the first, respectively
 // last, lane of a group receives its own).
 // ---------------------------------------------------------------------------------------------
 
@@ -32,6 +32,7 @@ struct PackedF32 {
   static constexpr int NC = 2;
   static constexpr bool kTransformed = true;
   static constexpr bool kDouble = false;
+  static constexpr bool kTable = true;
   __device__ __forceinline__ static V fma(V a, V b, V c) { return __ffma2_rn(a, b, c); }
   __device__ __forceinline__ static V mul(V a, V b) { return __fmul2_rn(a, b); }
   __device__ __forceinline__ static V add(V a, V b) { return __fadd2_rn(a, b); }
@@ -64,6 +65,7 @@ struct OneF32 {
   static constexpr int NC = 1;
   static constexpr bool kTransformed = true;
   static constexpr bool kDouble = false;
+  static constexpr bool kTable = true;
   __device__ __forceinline__ static V fma(V a, V b, V c) { return __fmaf_rn(a, b, c); }
   __device__ __forceinline__ static V mul(V a, V b) { return __fmul_rn(a, b); }
   __device__ __forceinline__ static V add(V a, V b) { return __fadd_rn(a, b); }
@@ -89,6 +91,7 @@ struct OneF64 {
   static constexpr int NC = 1;
   static constexpr bool kTransformed = false;
   static constexpr bool kDouble = true;
+  static constexpr bool kTable = false;
   __device__ __forceinline__ static V fma(V a, V b, V c) { return __fma_rn(a, b, c); }
   __device__ __forceinline__ static V mul(V a, V b) { return __dmul_rn(a, b); }
   __device__ __forceinline__ static V add(V a, V b) { return __dadd_rn(a, b); }
@@ -106,6 +109,12 @@ struct OneF64 {
   }
   __device__ __forceinline__ static V sel(bool m0, bool, V a, V b) { return m0 ? a : b; }
   __device__ __forceinline__ static V max(V a, V b) { return fmax(a, b); }
+};
+
+// FP64 for regions whose haplotypes hold A, C, G, T and N only: priors from a table in shared memory, as in
+// FP32 (a comparison and two selects a cell less than comparing codes).
+struct OneF64Table : OneF64 {
+  static constexpr bool kTable = true;
 };
 
 // Precision constants (fgkl simd.rs:102-154).

@@ -735,6 +735,10 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
     Task task;
     uint64_t cost;  // strip-mined pairs: steps x rows; 0 for the region's program tasks
   };
+  // One FP64 form a batch: the one that compares codes when a region needs it (the bits are the same).
+  bool extra_codes = false;
+  for (const RegionPlan& rp : plans) extra_codes |= rp.extra_codes;
+  const Kind f64 = extra_codes ? Kind::kOneF64Codes : Kind::kOneF64;
   std::vector<std::vector<RegionTask>> region_tasks(static_cast<size_t>(N));
   parallel_for(N, std::min(host_threads(), (N + 63) / 64), [&](int64_t gi) {
     const int g = static_cast<int>(gi);
@@ -792,7 +796,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
         one(Kind::kOneF32Pd, single_rows(len_of(order[i])), i);
       for (; i < order.size(); i += 2) two(Kind::kPackedF32Pd, packed_rows(len_of(order[i])), i);
     } else if (cfg.double_precision || plans[g].extra_codes) {
-      for (; i < order.size(); ++i) one(Kind::kOneF64, single_rows(len_of(order[i])), i);
+      for (; i < order.size(); ++i) one(f64, single_rows(len_of(order[i])), i);
     } else {
       // The tile-shape axis: rows_extra moves each read to the next instantiated rows-per-lane
       // (more padding rows, other registers and occupancy; the same bits).
@@ -895,7 +899,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       // Queue bin -> the FP64 form of the pairs it holds (queue_bin).
       const int r = queue_bin_rows(q);
       const Kind kind = q >= 2 * kRowBins ? Kind::kGenericF64Pd
-                                          : (q >= kRowBins ? (pd ? Kind::kLongF64Pd : Kind::kLongF64) : (pd ? Kind::kOneF64Pd : Kind::kOneF64));
+                                          : (q >= kRowBins ? (pd ? Kind::kLongF64Pd : Kind::kLongF64) : (pd ? Kind::kOneF64Pd : f64));
       int per_sm = 0, threads = 0;
       const bool pipelined = kind == Kind::kLongF64;
       Bin b{kind, r, queue_off[q], cap, 0, 0, 0};

@@ -304,6 +304,26 @@ auto dispatch(Kind k, int rows, Args&&... args) -> decltype(F<OneF32, 1>::run(ar
       break;
     case Kind::kOneF64:
       switch (rows) {
+        FGKL_CASE(OneF64Table, 1)
+        FGKL_CASE(OneF64Table, 2)
+        FGKL_CASE(OneF64Table, 3)
+        FGKL_CASE(OneF64Table, 4)
+        FGKL_CASE(OneF64Table, 5)
+        FGKL_CASE(OneF64Table, 6)
+        FGKL_CASE(OneF64Table, 7)
+        FGKL_CASE(OneF64Table, 8)
+        FGKL_CASE(OneF64Table, 10)
+        FGKL_CASE(OneF64Table, 12)
+        FGKL_CASE(OneF64Table, 14)
+        FGKL_CASE(OneF64Table, 16)
+        FGKL_CASE(OneF64Table, 18)
+        FGKL_CASE(OneF64Table, 20)
+        default:
+          break;
+      }
+      break;
+    case Kind::kOneF64Codes:
+      switch (rows) {
         FGKL_CASE(OneF64, 1)
         FGKL_CASE(OneF64, 2)
         FGKL_CASE(OneF64, 3)
@@ -346,6 +366,7 @@ bool valid_rows(Kind k, int rows) {
     case Kind::kOneF32:
       return rows >= 10 && rows <= 20 && rows % 2 == 0;
     case Kind::kOneF64:
+    case Kind::kOneF64Codes:
     case Kind::kOneF32Pd:
     case Kind::kOneF64Pd:
       return (rows >= 1 && rows <= 8) || (rows >= 10 && rows <= 20 && rows % 2 == 0);
@@ -510,15 +531,19 @@ __device__ void forward_unshared(const LaunchArgs& a, const ReadRef* rd, int lan
   FwdState<P, R> st;
   st.clear();
   const Program prog{};  // unused: the stream is synthesised from the haplotype bytes
-  for (int t = 0; t < n + 32; t += 2) {
-    const uint32_t e0 = byte_entry(hap, n, t - lane), e1 = byte_entry(hap, n, t + 1 - lane);
-    forward_step<P, R, 32>(a, prog, rd, lane, fr, an, sc, st, n, e0);
-    forward_step<P, R, 32>(a, prog, rd, lane, fr, an, sc, st, n, e1);
+  int t = 0;
+  for (; t < 32; ++t) forward_step<P, R, 32>(a, prog, rd, lane, fr, an, sc, st, n, byte_entry(hap, n, t - lane));
+  // Every lane strictly inside the haplotype: no events.
+  const uint8_t* seq = hap - lane;
+  for (; t + 4 <= n; t += 4) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) forward_step<P, R, 32, false>(a, prog, rd, lane, fr, an, sc, st, n, byte_code(__ldg(seq + t + i)));
   }
+  for (; t < n + 32; ++t) forward_step<P, R, 32>(a, prog, rd, lane, fr, an, sc, st, n, byte_entry(hap, n, t - lane));
 }
 
 template <int R>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, 1) noalloc_kernel(NoAllocArgs na) {
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, f64_min_blocks(R, false)) noalloc_kernel(NoAllocArgs na) {
   using P = OneF64;
   extern __shared__ __align__(16) unsigned char smem_raw[];  // none requested: nothing is staged
   const int lane = threadIdx.x & 31;

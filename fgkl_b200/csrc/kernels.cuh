@@ -25,8 +25,9 @@ enum class Kind : int {
   kGenericF32Pd = 10,
   kGenericF64Pd = 11,
   kQuadF32 = 12,   // up to four reads, two on each half of the lanes in FP32x2, rows-per-lane 2..14 (even)
+  kOneF64Codes = 13,  // as kOneF64, priors by comparing haplotype codes (bytes other than A, C, G, T and N)
 };
-constexpr int kNumKinds = 13;
+constexpr int kNumKinds = 14;
 // Lanes that hold two reads in the quad form, reads a warp, its largest rows-per-lane and its longest
 // read (the first row of the first lane is padding).
 constexpr int kQuadLanes = 16, kQuadReads = 4;

@@ -65,9 +65,9 @@ struct Layout {
   static constexpr int kNode = up(2 * R + 1);  // BM, BY rows; below-row BM
   static constexpr int kJoin = up(2 * R);      // cut column M and Y rows
   static constexpr int kStage = kSnap > kNode ? kSnap : kNode;
-  // FP32 kernels look priors up in a per-lane table indexed by haplotype code (A, C, G, T, N);
-  // regions holding other haplotype bytes run on the FP64 kernel, which compares codes instead.
-  static constexpr int kPriorCodes = P::kDouble ? 0 : 5;
+  // Priors are looked up in a per-lane table indexed by haplotype code (A, C, G, T, N); regions holding
+  // other haplotype bytes run on the FP64 form that compares codes instead.
+  static constexpr int kPriorCodes = P::kTable ? 5 : 0;
   // A lane's priors for one code: its rows padded to whole 16-byte chunks, kPer16 rows a chunk.
   static constexpr int kPer16 = kRound;
   static constexpr int kRp = up(R);
@@ -272,6 +272,10 @@ constexpr int block_warps() {
 // Resident blocks per SM each instantiation is compiled for: in the quad form what registers (seven values
 // a row and component, and about 42 for the rest) and shared memory leave room for; one read a warp at 16
 // warps an SM up to 8 rows.
+// FP64: three blocks of four warps while their registers hold the rows (128 regions in FP64, 5 rows: 7.8 ms,
+// against 8.3 at the 8 warps an SM of one block's full budget; four blocks 7.9); priors from the table
+// instead of by comparison 6.4 ms, and at 6 rows three blocks fit then.
+constexpr int f64_min_blocks(int rows, bool table) { return rows <= (table ? 6 : 5) ? 3 : 1; }
 template <class P, int R, int G>
 struct MinBlocks {
   static constexpr int kRegs = (7 * R * P::NC + 42) > 255 ? 255 : 7 * R * P::NC + 42;
@@ -279,7 +283,7 @@ struct MinBlocks {
   // A quarter of the SM's registers serves a quarter of its warps.
   static constexpr int kByRegs = 2 * (512 / ((kRegs + 7) / 8 * 8));
   static constexpr int kQuad = kByRegs < kBySmem ? kByRegs : kBySmem;
-  static constexpr int value = G < 32 ? (kQuad > 12 ? 12 : kQuad) : (P::kDouble ? 1 : (R <= 8 ? 4 : 2));
+  static constexpr int value = G < 32 ? (kQuad > 12 ? 12 : kQuad) : (P::kDouble ? f64_min_blocks(R, P::kTable) : (R <= 8 ? 4 : 2));
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -568,11 +572,15 @@ __device__ __forceinline__ void forward_pass(const LaunchArgs& a, const Program&
   st.load_next(a.v, prog, synth_len > 0 ? prog.n_segs : 0);
   if (P::kDouble && synth_len > 0) {
     const int n = synth_len;
-    for (int t = 0; t < n + G; t += 2) {
-      const uint32_t e0 = synth_entry(synth_seq, n, t - gl), e1 = synth_entry(synth_seq, n, t + 1 - gl);
-      forward_step<P, R, G>(a, prog, rd, lane, fr, an, sc, st, synth_len, e0);
-      forward_step<P, R, G>(a, prog, rd, lane, fr, an, sc, st, synth_len, e1);
+    int t = 0;
+    for (; t < G; ++t) forward_step<P, R, G>(a, prog, rd, lane, fr, an, sc, st, n, synth_entry(synth_seq, n, t - gl));
+    // Every lane strictly inside the haplotype: no events.
+    const uint8_t* seq = synth_seq - gl;
+    for (; t + 4 <= n; t += 4) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) forward_step<P, R, G, false>(a, prog, rd, lane, fr, an, sc, st, n, __ldg(seq + t + i));
     }
+    for (; t < n + G; ++t) forward_step<P, R, G>(a, prog, rd, lane, fr, an, sc, st, n, synth_entry(synth_seq, n, t - gl));
   } else {
     const int n = prog.fwd_len;
     const uint32_t* stream = a.v.stream + prog.fwd_off - gl;

@@ -67,3 +67,19 @@ def test_split_regions_keep_their_bits(gpu, pd, precision, haps):
         ref = O.compute_matrix(reads[:3] + reads[-3:], hs).reshape(6, -1)
         assert np.max(np.abs(alone - ref)) < TOL[precision]
     assert not pd or isinstance(parts[0][1][0], PdHaplotype)
+
+
+def test_other_haplotype_bytes_take_the_comparing_form(gpu):
+    """Priors come from a table for A, C, G, T and N haplotypes and by comparing codes for any others, a whole
+    FP64 batch at a time; a region's bits are the same beside either."""
+    parts = regions((1, 30, 155, 156), 3, 5, 4, 220)
+    reads, haps = parts[1]
+    odd = (reads, [haps[0].replace(b"A", b"R", 3), *haps[1:]])
+    cfg = Config(precision=Precision.DOUBLE)
+    table, _ = BatchContext().compute(synthetic.from_regions(parts), cfg)
+    w = synthetic.from_regions([parts[0], odd, parts[2]])
+    compared, _ = BatchContext().compute(w, cfg)
+    offs = w.output_offsets()
+    for g in (0, 2):
+        assert table[offs[g]:offs[g + 1]].tobytes() == compared[offs[g]:offs[g + 1]].tobytes()
+    assert np.max(np.abs(compared[offs[1]:offs[2]] - O.compute_matrix(*odd))) < TOL[Precision.DOUBLE]
