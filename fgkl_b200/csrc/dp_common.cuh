@@ -229,6 +229,43 @@ __device__ __forceinline__ typename P::V cell_match(const typename P::V& dM, con
   return P::fma(dY, k1, P::fma(dX, k1, P::mul(dM, k0)));
 }
 
+// Factors of a row's match bracket (cell_match). X^ = X / mi and Y^ = Y / md (FP32 form):
+// S = mm*M + (im*mi')*X^ + (im*md')*Y^ is taken as mm * (M + (im*mi'/mm)*X^ + (im*md'/mm)*Y^) with mm in
+// the prior table.
+template <class P>
+struct BracketFactors {
+  using S = typename P::S;
+  S k0, k1, k2;
+  __device__ explicit BracketFactors(const RowModel& m)
+      : k0(static_cast<S>(m.mm)),
+        k1(static_cast<S>(!P::kTransformed ? m.im : (m.read ? m.im * m.mi_prev / m.mm : 0.0))),
+        k2(!P::kTransformed ? k1 : static_cast<S>(m.read ? m.im * m.md_prev / m.mm : 0.0)) {}
+};
+
+// ---------------------------------------------------------------------------------------------
+// Strip-mined reads: row blocks as a pipeline of warps (kernels.cu, pd_kernels.cu).
+// ---------------------------------------------------------------------------------------------
+
+// What a block's bottom row hands to the next block's top row, per column (FwdState::xs and ts, PdState::xs and ts): 8 or
+// 16 bytes.
+template <class P>
+struct __align__(2 * sizeof(typename P::S)) Carry {
+  typename P::S x, t;
+};
+
+template <class P>
+__host__ __device__ constexpr size_t long_scratch_size(int max_hap_len) {
+  return static_cast<size_t>(max_hap_len) * sizeof(Carry<P>);
+}
+
+// Columns a superstep, and the supersteps a warp starts behind the one above it: at superstep s a warp
+// reads columns up to (s - w kDelay) kChunk - 1 - (kDelay - 1) kChunk + ... of its ring, of which the warp
+// above has written (s - w kDelay + kDelay) kChunk - 32 by the barrier before, so
+// kDelay * kChunk >= kChunk + 31. What that warp writes meanwhile lies behind those columns and at most
+// kDelay * kChunk + kChunk - 32 ahead of the oldest one, so a ring of kRing entries holds both.
+constexpr int kChunk = 32, kDelay = 2, kRing = 128;
+static_assert(kDelay * kChunk >= kChunk + 31 && kRing >= (kDelay + 1) * kChunk, "ring");
+
 }  // namespace
 
 // Resident blocks per SM of a kernel taking `smem` bytes of dynamic shared memory, resolved once per

@@ -697,8 +697,12 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
     planned_.prefix_only_cells += rp.read_bases * rp.cols.prefix_only;
     for (const HapInfo& h : rp.haps) max_hap_len = std::max(max_hap_len, static_cast<int>(h.len));
     if (rp.n_distinct > 0)
-      for (int64_t r = first_read[g]; r < first_read[g + 1]; ++r)
-        queue_cap[queue_bin(static_cast<int>(in.read_off[r + 1] - in.read_off[r]), rp.generic)] += rp.n_distinct;
+      for (int64_t r = first_read[g]; r < first_read[g + 1]; ++r) {
+        const int len = static_cast<int>(in.read_off[r + 1] - in.read_off[r]);
+        const int bin = queue_bin(len, rp.generic), pair_bin = queue_pair_bin(len, rp.generic);
+        queue_cap[bin] += rp.n_distinct;
+        if (pair_bin != bin) queue_cap[pair_bin] += rp.n_distinct;
+      }
   }
   if (n_stream > INT32_MAX || n_seq > INT32_MAX || n_pd_seq > INT32_MAX || n_haps > INT32_MAX)
     return fail(FGKL_E_INVALID_ARGUMENT, "batch too large for 32-bit plan offsets; split it");
@@ -859,7 +863,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
         cost += e.first;
       }
       const bool fp32 = b.kind == Kind::kShortF32 || b.kind == Kind::kOneF32 || b.kind == Kind::kPackedF32Pd || b.kind == Kind::kOneF32Pd;
-      const bool pipelined = b.kind == Kind::kLongF32 || b.kind == Kind::kLongF64;
+      const bool pipelined = is_long(b.kind);
       b.warps = pipelined ? long_warps(bl.row_blocks) : (fp32 ? tuning_.warps_per_block : kWarpsPerBlock);
       int per_sm = 0, threads = 0;
       occupancy(b.kind, b.rows, &per_sm, &threads, b.warps);
@@ -901,7 +905,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       const Kind kind = q >= 2 * kRowBins ? Kind::kGenericF64Pd
                                           : (q >= kRowBins ? (pd ? Kind::kLongF64Pd : Kind::kLongF64) : (pd ? Kind::kOneF64Pd : f64));
       int per_sm = 0, threads = 0;
-      const bool pipelined = kind == Kind::kLongF64;
+      const bool pipelined = is_long(kind);
       Bin b{kind, r, queue_off[q], cap, 0, 0, 0};
       if (pipelined) b.warps = long_warps(long_blocks(max_read_len, r));
       occupancy(kind, r, &per_sm, &threads, b.warps);

@@ -60,12 +60,15 @@ __global__ void __launch_bounds__(256) collect_kernel(CollectArgs a) {
       if (lane == 0) atomicAdd(&a.v.counters->rescue_reads, static_cast<unsigned long long>(lost_distinct));
       continue;
     }
+    const int pair_bin = queue_pair_bin(len, generic);
+    const int pair_cap = a.queue_off[pair_bin + 1] - a.queue_off[pair_bin];
     for (int k = lane; k < region.n_haps; k += 32) {
       const HapInfo info = a.v.haps[region.hap_off + k];
       if (info.src != k || !isnan(row[info.order])) continue;
-      const int slot = atomicAdd(a.queue_tail + bin, 1);
-      if (slot < cap) {
-        a.queue[a.queue_off[bin] + slot] = Task{static_cast<int32_t>(blockIdx.x), {read, -1, -1, -1}, rows, k, region.prog};
+      const int slot = atomicAdd(a.queue_tail + pair_bin, 1);
+      if (slot < pair_cap) {
+        a.queue[a.queue_off[pair_bin] + slot] =
+            Task{static_cast<int32_t>(blockIdx.x), {read, -1, -1, -1}, queue_bin_rows(pair_bin), k, region.prog};
         atomicAdd(&a.v.counters->rescue_reads, 1ull);
       }
     }
@@ -87,26 +90,6 @@ __global__ void __launch_bounds__(256) collect_kernel(CollectArgs a) {
 // against 6 haplotypes at 2.6 ms in FP32 and 5.8 ms for the 72 pairs recomputed in FP64, most of the GPU
 // idle.)
 // ---------------------------------------------------------------------------------------------
-
-// What a block's bottom row hands to the next block's top row, per column (FwdState::xs and ts): 8 or
-// 16 bytes.
-template <class P>
-struct __align__(2 * sizeof(typename P::S)) Carry {
-  typename P::S x, t;
-};
-
-template <class P>
-__host__ __device__ constexpr size_t long_scratch_size(int max_hap_len) {
-  return static_cast<size_t>(max_hap_len) * sizeof(Carry<P>);
-}
-
-// Columns a superstep, and the supersteps a warp starts behind the one above it: at superstep s a warp
-// reads columns up to (s - w kDelay) kChunk - 1 - (kDelay - 1) kChunk + ... of its ring, of which the warp
-// above has written (s - w kDelay + kDelay) kChunk - 32 by the barrier before, so
-// kDelay * kChunk >= kChunk + 31. What that warp writes meanwhile lies behind those columns and at most
-// kDelay * kChunk + kChunk - 32 ahead of the oldest one, so a ring of kRing entries holds both.
-constexpr int kChunk = 32, kDelay = 2, kRing = 128;
-static_assert(kDelay * kChunk >= kChunk + 31 && kRing >= (kDelay + 1) * kChunk, "ring");
 
 template <class P, int R>
 constexpr size_t long_smem_per_warp() {
@@ -422,11 +405,9 @@ size_t long_scratch_bytes(Kind k, int rows, int max_hap_len) {
 
 void long_occupancy(Kind k, int rows, int* blocks, int* threads, int warps) {
   *blocks = 0;
-  *threads = kWarpsPerBlock * 32;
-  if (!is_long(k) || !valid_long_rows(k, rows)) return;
-  if (is_pd(k)) return pd_long_occupancy(k, rows, blocks, threads);
   *threads = warps * 32;
-  if (warps < 1 || warps > kLongWarps) return;
+  if (!is_long(k) || !valid_long_rows(k, rows) || warps < 1 || warps > kLongWarps) return;
+  if (is_pd(k)) return pd_long_occupancy(k, rows, blocks, threads, warps);
   if (k == Kind::kLongF64)
     long_rows_narrow(rows, [&](auto r) {
       long_occ<OneF64, decltype(r)::value>(blocks, warps);
@@ -440,9 +421,8 @@ void long_occupancy(Kind k, int rows, int* blocks, int* threads, int warps) {
 }
 
 cudaError_t long_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream, int warps) {
-  if (!is_long(k) || !valid_long_rows(k, rows)) return cudaErrorInvalidValue;
-  if (is_pd(k)) return pd_long_launch(k, rows, blocks, args, stream);
-  if (warps < 1 || warps > kLongWarps) return cudaErrorInvalidValue;
+  if (!is_long(k) || !valid_long_rows(k, rows) || warps < 1 || warps > kLongWarps) return cudaErrorInvalidValue;
+  if (is_pd(k)) return pd_long_launch(k, rows, blocks, args, stream, warps);
   if (k == Kind::kLongF64)
     return long_rows_narrow(rows, [&](auto r) { return long_go<OneF64, decltype(r)::value>(blocks, args, stream, warps); });
   return long_rows_wide(rows, [&](auto r) { return long_go<OneF32, decltype(r)::value>(blocks, args, stream, warps); });

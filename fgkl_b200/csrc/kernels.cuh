@@ -82,6 +82,13 @@ __host__ __device__ inline int queue_bin(int len, bool generic) {
   return rows;
 }
 __host__ __device__ inline int queue_bin_rows(int bin) { return bin % kRowBins; }
+// The bin of a single lost pair of a read: as queue_bin up to 248 bases; above, the strip-mined form's, whose
+// row blocks run side by side on a few warps (one block of 10 to 20 rows a lane in FP64 spills registers and
+// is one warp's work). A read's whole-program tasks stay in queue_bin's.
+__host__ __device__ inline int queue_pair_bin(int len, bool generic) {
+  const int bin = queue_bin(len, generic);
+  return bin < kRowBins && bin > 8 ? kRowBins + long_rows(len, false) : bin;
+}
 
 inline bool is_long(Kind k) { return k >= Kind::kLongF32 && k <= Kind::kGenericF64Pd; }
 inline bool is_pd(Kind k) {
@@ -140,8 +147,8 @@ size_t long_scratch_bytes(Kind k, int rows, int max_hap_len);
 void long_occupancy(Kind k, int rows, int* blocks_per_sm, int* threads_per_block, int warps_per_block);
 cudaError_t long_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream, int warps_per_block);
 size_t pd_long_scratch_bytes(Kind k, int rows, int max_hap_len);
-void pd_long_occupancy(Kind k, int rows, int* blocks_per_sm, int* threads_per_block);
-cudaError_t pd_long_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream);
+void pd_long_occupancy(Kind k, int rows, int* blocks_per_sm, int* threads_per_block, int warps_per_block);
+cudaError_t pd_long_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream, int warps_per_block);
 
 // Launches the lost-pair collection over `n_regions` regions.
 cudaError_t launch_collect(const CollectArgs& args, int n_regions, cudaStream_t stream);

@@ -43,8 +43,8 @@ struct PdLayout {
   using V = typename P::V;
   static constexpr int kRound = 16 / static_cast<int>(sizeof(V)) > 1 ? 16 / static_cast<int>(sizeof(V)) : 1;
   static constexpr int up(int x) { return (x + kRound - 1) / kRound * kRound; }
-  // M, X, Y rows; branch M, X, Y rows; above-row M, X, Y; accumulated result.
-  static constexpr int kSnap = up(6 * R + 4);
+  // M, X, Y rows; branch M, X, Y rows; accumulated result.
+  static constexpr int kSnap = up(6 * R + 1);
   static constexpr size_t kStageBytes = 32ull * kSnap * sizeof(V);
   static constexpr size_t kSmemPerWarp = kStageBytes;
 };
@@ -54,7 +54,7 @@ struct PdScratch {
   using V = typename P::V;
   using L = PdLayout<P, R>;
   V* slots;         // [slot][lane][kSnap]
-  double* seg_raw;  // [seg][c]
+  double* seg_raw;  // [seg][read slot]
   V* stage;         // shared: [buf][lane][kSnap]
 
   __device__ PdScratch(char* base, V* smem, int n_slots) {
@@ -63,6 +63,8 @@ struct PdScratch {
     stage = smem;
   }
   __device__ V* slot(int s, int lane) { return slots + (static_cast<size_t>(s) * 32 + lane) * L::kSnap; }
+  // The result of a segment for one of the warp's reads, before its factor.
+  __device__ double& raw(int seg, int slot) { return seg_raw[seg * kMaxReads + slot]; }
   // One staging record per lane serves every segment: a lane writes or prefetches the next
   // segment's start into it only after loading the current one at its BEGIN.
   __device__ V* staged(int, int lane) { return stage + static_cast<size_t>(lane) * L::kSnap; }
@@ -71,19 +73,30 @@ struct PdScratch {
 template <class P, int R>
 constexpr size_t pd_scratch_size(int n_slots, int n_segs) {
   return static_cast<size_t>(n_slots) * 32 * PdLayout<P, R>::kSnap * sizeof(typename P::V) +
-         static_cast<size_t>(n_segs) * P::NC * sizeof(double);
+         static_cast<size_t>(n_segs) * kMaxReads * sizeof(double);
 }
 
-// Forward coefficients of the lane's rows (the plain kernels' FwdRows) and each row's read class.
-template <class P, int R>
+// Forward coefficients of the lane's rows and each row's read class. As in the plain kernel, what row r + 1
+// takes from row r is held with row r (k0..k3, k5), because the lane computes both values that its bottom
+// row hands to the lane below.
+template <class P, int R, int G>
 struct PdRows {
   using V = typename P::V;
   using S = typename P::S;
-  V c0[R], c1[R], c2[R], c3[R], c4[R], pm[R], px[R];
+  V k0[R], k1[R], k2[R], k3[R], k4[R], k5[R], k6[R], pm[R], px[R];
   uint32_t cls[P::NC][R];  // bit of the row's read class; 0 for a padding row (no code accepts it)
 
   __device__ V prior(uint32_t sig, int r) const {
     return P::sel((sig & cls[0][r]) != 0u, (sig & cls[P::NC - 1][r]) != 0u, pm[r], px[r]);
+  }
+  // What row r + 1's match value is, before its prior, from row r.
+  __device__ V bracket(const V& M, const V& X, const V& Y, int r) const { return cell_match<P>(M, X, Y, k0[r], k1[r], k2[r]); }
+  // Row r + 1's insertion value from row r's.
+  __device__ V insertion(const V& M, const V& X, int r) const {
+    return P::kTransformed ? P::fma(X, k3[r], M) : P::fma(X, k3[r], P::mul(M, k5[r]));
+  }
+  __device__ V deletion(const V& M, const V& Y, int r) const {
+    return P::kTransformed ? P::fma(Y, k4[r], M) : P::fma(Y, k4[r], P::mul(M, k6[r]));
   }
 
   // Regions whose reads hold more distinct bytes than the class bits cover compare bytes instead:
@@ -98,45 +111,29 @@ struct PdRows {
   }
 
   __device__ void load(const BatchView& v, const ReadRef* rd, int lane, const uint8_t* classes) {
+    const int top = (lane % G) * R;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+    for (int r = 0; r <= R; ++r) {
 #pragma unroll
       for (int c = 0; c < P::NC; ++c) {
-        const RowModel m = row_model(v, rd[c], lane * R + r - rd[c].pad, classes);
-        double k0, k1, k2, k3, k4;
-        if (P::kTransformed) {
-          // The match-to-match factor moves into the priors (cell_match).
-          if (m.read) {
-            k0 = m.mm;
-            k1 = m.im * m.mi_prev / m.mm;
-            k2 = m.im * m.md_prev / m.mm;
-            k3 = m.gc * m.mi_prev / m.mi;
-            k4 = m.gc;
-          } else {
-            k0 = k1 = k2 = k3 = 0.0;
-            k4 = 1.0;
-          }
-        } else {
-          if (m.read) {
-            k0 = m.mm;
-            k1 = m.im;
-            k2 = m.mi;
-            k3 = m.gc;
-            k4 = m.md;
-          } else {
-            k0 = k1 = k2 = k4 = 0.0;
-            k3 = 1.0;
-          }
+        const RowModel m = row_model(v, rd[c], top + r - rd[c].pad, classes);
+        if (r > 0) {
+          const BracketFactors<P> b(m);
+          P::put(k0[r - 1], c, b.k0);
+          P::put(k1[r - 1], c, b.k1);
+          P::put(k2[r - 1], c, b.k2);
+          P::put(k3[r - 1], c, static_cast<S>(!P::kTransformed ? (m.read ? m.gc : 1.0) : (m.read ? m.gc * m.mi_prev / m.mi : 0.0)));
+          P::put(k5[r - 1], c, static_cast<S>(m.mi));
         }
-        const double fold = (P::kTransformed && m.read) ? m.mm : 1.0;
-        P::put(c0[r], c, static_cast<S>(k0));
-        P::put(c1[r], c, static_cast<S>(k1));
-        P::put(c2[r], c, static_cast<S>(k2));
-        P::put(c3[r], c, static_cast<S>(k3));
-        P::put(c4[r], c, static_cast<S>(k4));
-        P::put(pm[r], c, static_cast<S>(m.pm * fold));
-        P::put(px[r], c, static_cast<S>(m.px * fold));
-        cls[c][r] = m.read ? (1u << (m.oc & 31)) : 0u;
+        if (r < R) {
+          // The match-to-match factor moves into the priors in the FP32 form (cell_match).
+          const double fold = (P::kTransformed && m.read) ? m.mm : 1.0;
+          P::put(k4[r], c, static_cast<S>(m.read ? m.gc : 1.0));
+          P::put(k6[r], c, static_cast<S>(m.md));
+          P::put(pm[r], c, static_cast<S>(m.pm * fold));
+          P::put(px[r], c, static_cast<S>(m.px * fold));
+          cls[c][r] = m.read ? (1u << (m.oc & 31)) : 0u;
+        }
       }
     }
   }
@@ -146,7 +143,7 @@ struct PdRows {
     load(v, rd, lane, classes);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int q = lane * R + r - rd[0].pad;
+      const int q = (lane % G) * R + r - rd[0].pad;
       uint32_t d = 0;
       if (rd[0].len > 0 && q >= 0 && q < rd[0].len) {
         const uint32_t b = v.bases[rd[0].off + q];
@@ -163,44 +160,71 @@ struct PdState {
   using V = typename P::V;
   V M[R], X[R], Y[R];
   V BM[R], BX[R], BY[R];
+  // For the lane below's top row, at the column the lane has just computed: its new insertion value (from
+  // the merged bottom row on a DEL_END column), and the bracket of its match value (from the column before).
+  V xs, ts;
   V acc;
   int seg_i;
-  // Strip-mined reads: the row above lane 0's top row for this step's column (read only by
+  // Strip-mined reads: what lane 0's top row takes from the row above for this step's column (read only by
   // pd_step<..., kCarry = true>).
-  V cM, cX, cY;
+  V cX, cT;
+
+  __device__ void clear() {
+#pragma unroll
+    for (int r = 0; r < R; ++r) M[r] = X[r] = Y[r] = BM[r] = BX[r] = BY[r] = P::zero();
+    xs = ts = acc = P::zero();
+    seg_i = -1;
+  }
 };
 
-// The lane above's bottom row.
-template <class P>
-struct PdEdge {
+// The rows of one column. kSlow: some lane's column carries DEL_START or DEL_END; the branch-value path is
+// exact for every column, so the whole warp takes it. keep(r): what to do with the branch values of row r
+// before its column; de: the lane's column carries DEL_END, and each row's values take the max with its
+// branch values once its X is computed, so that the next row's X reads U = max(B(up), V(up)).
+template <class P, int R, int G, bool kSlow, class Prior, class Keep>
+__device__ __forceinline__ void pd_rows_down(const PdRows<P, R, G>& pr, PdState<P, R>& st, const typename P::V& an, typename P::V qX,
+                                             typename P::V T, bool de, Prior&& prior, Keep&& keep) {
   using V = typename P::V;
-  V M, X, Y;
-};
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const V below = pr.bracket(st.M[r], st.X[r], st.Y[r], r);
+    if (kSlow) keep(r);
+    st.Y[r] = pr.deletion(st.M[r], st.Y[r], r);
+    st.M[r] = P::mul(prior(r), T);
+    T = below;
+    st.X[r] = qX;
+    if (r == R - 1) st.acc = P::fma(qX, an, P::add(st.acc, st.M[r]));  // the result takes the unmerged values
+    if (kSlow && de) {
+      st.M[r] = P::max(st.BM[r], st.M[r]);
+      st.X[r] = P::max(st.BX[r], st.X[r]);
+      st.Y[r] = P::max(st.BY[r], st.Y[r]);
+    }
+    qX = pr.insertion(st.M[r], st.X[r], r);
+  }
+  st.xs = qX;
+  st.ts = T;
+}
 
-// One PD forward step: events, then the column. `u` receives the lane above's bottom row for this
-// column, `d` holds it for the previous column (the top row's diagonal); the two alternate. kEv = false
-// compiles the event code out, for steps where no lane of the warp has an event. kCarry = true gives
-// lane 0 the row above from the state's carry values (strip-mined reads); kGeneric = true decides
-// priors by comparing bytes (PdRows::prior_generic) instead of by class bits.
-template <class P, int R, bool kEv = true, bool kCarry = false, bool kGeneric = false>
+// One PD forward step: events, then the column. kEv = false compiles the event code out, for steps where no
+// lane of the warp has an event. kCarry = true gives lane 0 the row above from the state's carry values
+// (strip-mined reads); otherwise a group's first lane starts with a padding row, for which the row above is
+// zero. kGeneric = true decides priors by comparing bytes (PdRows::prior_generic) instead of by class bits.
+template <class P, int R, int G, bool kEv = true, bool kCarry = false, bool kGeneric = false>
 __device__ __forceinline__ void pd_step(const LaunchArgs& a, const Program& prog, const ReadRef* rd, int lane,
-                                        const PdRows<P, R>& pr, const typename P::V& an, int pad_hi, PdScratch<P, R>& sc,
-                                        PdState<P, R>& st, int synth_len, uint32_t ev, uint32_t sig, PdEdge<P>& u,
-                                        PdEdge<P>& d) {
+                                        const PdRows<P, R, G>& pr, const typename P::V& an, PdScratch<P, R>& sc,
+                                        PdState<P, R>& st, int synth_len, uint32_t ev, uint32_t sig) {
   using V = typename P::V;
   using S = typename P::S;
   using L = PdLayout<P, R>;
-  u.M = P::up(st.M[R - 1]);
-  u.X = P::up(st.X[R - 1]);
-  u.Y = P::up(st.Y[R - 1]);
-  if (kCarry && lane == 0) {
-    u.M = st.cM;
-    u.X = st.cX;
-    u.Y = st.cY;
+  const int gl = lane % G;
+  V qX = P::template up<G>(st.xs), T = P::template up<G>(st.ts);
+  if (gl == 0) {
+    qX = kCarry ? st.cX : P::zero();
+    T = kCarry ? st.cT : P::zero();
   }
-  // END and ACC act in lane 31 alone (the read's last row); the other lanes pass them by without
-  // entering the event code, which every lane otherwise reaches at its own step.
-  if (kEv && (ev & (lane == 31 ? kEvMask : (kEvMask & ~(EV_END | EV_ACC))))) {
+  // END and ACC act in the group's last lane alone (the read's last row); the other lanes pass them by
+  // without entering the event code, which every lane otherwise reaches at its own step.
+  if (kEv && (ev & (gl == G - 1 ? kEvMask : (kEvMask & ~(EV_END | EV_ACC))))) {
     if (ev & EV_SNAP) {
       const uint32_t slot = ev >> kPdPayloadShift;
       V* dst[2] = {slot != kPdPayloadNone ? sc.slot(static_cast<int>(slot), lane) : nullptr,
@@ -218,15 +242,12 @@ __device__ __forceinline__ void pd_step(const LaunchArgs& a, const Program& prog
           o[4 * R + r] = st.BX[r];
           o[5 * R + r] = st.BY[r];
         }
-        o[6 * R] = d.M;
-        o[6 * R + 1] = d.X;
-        o[6 * R + 2] = d.Y;
-        o[6 * R + 3] = st.acc;
+        o[6 * R] = st.acc;
       }
     }
-    if ((ev & EV_END) && lane == 31) {
+    if ((ev & EV_END) && gl == G - 1) {
 #pragma unroll
-      for (int c = 0; c < P::NC; ++c) sc.seg_raw[st.seg_i * P::NC + c] = static_cast<double>(P::get(st.acc, c));
+      for (int c = 0; c < P::NC; ++c) sc.raw(st.seg_i, lane / G * P::NC + c) = static_cast<double>(P::get(st.acc, c));
     }
     if (ev & EV_BEGIN) {
       ++st.seg_i;
@@ -247,38 +268,26 @@ __device__ __forceinline__ void pd_step(const LaunchArgs& a, const Program& prog
           st.BX[r] = s[4 * R + r];
           st.BY[r] = s[5 * R + r];
         }
-        d.M = s[6 * R];
-        d.X = s[6 * R + 1];
-        d.Y = s[6 * R + 2];
-        st.acc = s[6 * R + 3];
+        st.acc = s[6 * R];
       } else {
         // The origin: the row-0 constant in the padding rows, zero branch values (GATK never writes
         // branch column zero).
         const S in_s = synth ? static_cast<S>(Consts<P::kDouble>::kInitial / synth_len)
                              : (P::kDouble ? static_cast<S>(rec->init_d) : static_cast<S>(rec->init_f));
 #pragma unroll
-        for (int r = 0; r < R; ++r) st.M[r] = st.X[r] = st.Y[r] = st.BM[r] = st.BX[r] = st.BY[r] = P::zero();
-        d.M = d.X = d.Y = st.acc = P::zero();
-        if (lane * R <= pad_hi) {
+        for (int r = 0; r < R; ++r) {
+          st.M[r] = st.X[r] = st.BM[r] = st.BX[r] = st.BY[r] = P::zero();
 #pragma unroll
-          for (int c = 0; c < P::NC; ++c) {
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-              if (lane * R + r < rd[c].pad) P::put(st.Y[r], c, in_s);
-            if (lane * R - 1 < rd[c].pad) P::put(d.Y, c, in_s);
-          }
+          for (int c = 0; c < P::NC; ++c) P::put(st.Y[r], c, gl * R + r < rd[c].pad ? in_s : S(0));
         }
+        st.acc = P::zero();
       }
       if (next_slot >= 0) prefetch(sc.staged(st.seg_i + 1, lane), sc.slot(next_slot, lane), L::kSnap);
     }
   }
-  // A slow step (some lane at a column carrying DEL_START or DEL_END) runs the branch-value path for
-  // the whole warp; it is exact for every column, so lanes do not diverge between it and the plain
-  // recurrence.
-  const bool slow = __any_sync(kFull, (ev & kPdSlowMask) != 0);
-  const bool de = slow && (ev & PD_DE) != 0;
-  if (slow) {
-    const bool mat = (ev & PD_MAT) != 0;
+  auto prior = [&](int r) { return kGeneric ? pr.prior_generic(ev, r) : pr.prior(sig, r); };
+  if (__any_sync(kFull, (ev & kPdSlowMask) != 0)) {
+    const bool de = (ev & PD_DE) != 0, mat = (ev & PD_MAT) != 0;
     const uint32_t s_first = (ev >> kPdFirstShift) & 3u, s_later = (ev >> kPdLaterShift) & 3u;
     if (__all_sync(kFull, s_first == s_later)) {
       // Every row of each lane in one deletion state (the read's first row starts NORMAL, the later
@@ -286,68 +295,28 @@ __device__ __forceinline__ void pd_step(const LaunchArgs& a, const Program& prog
       // haplotype's end): a column carrying either flag keeps V(left) as the branch values unless
       // inside a deletion, one predicate a lane.
       const bool keep = mat && s_later != kPdInsideDel;
-#pragma unroll
-      for (int r = R - 1; r >= 0; --r) {
-        const V pM = r ? st.M[r - 1] : d.M, pX = r ? st.X[r - 1] : d.X, pY = r ? st.Y[r - 1] : d.Y;
+      pd_rows_down<P, R, G, true>(pr, st, an, qX, T, de, prior, [&](int r) {
         if (keep) {
           st.BM[r] = st.M[r];
           st.BX[r] = st.X[r];
           st.BY[r] = st.Y[r];
         }
-        const V prior = kGeneric ? pr.prior_generic(ev, r) : pr.prior(sig, r);
-        st.Y[r] = P::kTransformed ? P::fma(st.Y[r], pr.c4[r], st.M[r]) : P::fma(st.Y[r], pr.c3[r], P::mul(st.M[r], pr.c4[r]));
-        st.M[r] = P::mul(prior, cell_match<P>(pM, pX, pY, pr.c0[r], pr.c1[r], pr.c2[r]));
-      }
+      });
     } else {
       // Some lane's first read row is in another state than its later rows.
-#pragma unroll
-      for (int r = R - 1; r >= 0; --r) {
+      pd_rows_down<P, R, G, true>(pr, st, an, qX, T, de, prior, [&](int r) {
         bool inside[P::NC];
 #pragma unroll
-        for (int c = 0; c < P::NC; ++c) inside[c] = ((lane * R + r == rd[c].pad) ? s_first : s_later) == kPdInsideDel;
-        const V pM = r ? st.M[r - 1] : d.M, pX = r ? st.X[r - 1] : d.X, pY = r ? st.Y[r - 1] : d.Y;
+        for (int c = 0; c < P::NC; ++c) inside[c] = ((gl * R + r == rd[c].pad) ? s_first : s_later) == kPdInsideDel;
         if (mat) {
           st.BM[r] = P::sel(inside[0], inside[P::NC - 1], st.BM[r], st.M[r]);
           st.BX[r] = P::sel(inside[0], inside[P::NC - 1], st.BX[r], st.X[r]);
           st.BY[r] = P::sel(inside[0], inside[P::NC - 1], st.BY[r], st.Y[r]);
         }
-        const V prior = kGeneric ? pr.prior_generic(ev, r) : pr.prior(sig, r);
-        st.Y[r] = P::kTransformed ? P::fma(st.Y[r], pr.c4[r], st.M[r]) : P::fma(st.Y[r], pr.c3[r], P::mul(st.M[r], pr.c4[r]));
-        st.M[r] = P::mul(prior, cell_match<P>(pM, pX, pY, pr.c0[r], pr.c1[r], pr.c2[r]));
-      }
-    }
-    // Insertion values from the top row down. On a DEL_END column each row's values take the max
-    // with its branch values once its X is computed (the last row's after the result below), so
-    // the next row's X reads U = max(B(up), V(up)); the lane above's bottom row arrives merged.
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const V qM = r ? st.M[r - 1] : u.M, qX = r ? st.X[r - 1] : u.X;
-      st.X[r] = P::kTransformed ? P::fma(qX, pr.c3[r], qM) : P::fma(qX, pr.c3[r], P::mul(qM, pr.c2[r]));
-      if (de && r + 1 < R) {
-        st.M[r] = P::max(st.BM[r], st.M[r]);
-        st.X[r] = P::max(st.BX[r], st.X[r]);
-        st.Y[r] = P::max(st.BY[r], st.Y[r]);
-      }
+      });
     }
   } else {
-#pragma unroll
-    for (int r = R - 1; r >= 0; --r) {
-      const V pM = r ? st.M[r - 1] : d.M, pX = r ? st.X[r - 1] : d.X, pY = r ? st.Y[r - 1] : d.Y;
-      const V prior = kGeneric ? pr.prior_generic(ev, r) : pr.prior(sig, r);
-      st.Y[r] = P::kTransformed ? P::fma(st.Y[r], pr.c4[r], st.M[r]) : P::fma(st.Y[r], pr.c3[r], P::mul(st.M[r], pr.c4[r]));
-      st.M[r] = P::mul(prior, cell_match<P>(pM, pX, pY, pr.c0[r], pr.c1[r], pr.c2[r]));
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const V qM = r ? st.M[r - 1] : u.M, qX = r ? st.X[r - 1] : u.X;
-      st.X[r] = P::kTransformed ? P::fma(qX, pr.c3[r], qM) : P::fma(qX, pr.c3[r], P::mul(qM, pr.c2[r]));
-    }
-  }
-  st.acc = P::fma(st.X[R - 1], an, P::add(st.acc, st.M[R - 1]));
-  if (de) {
-    st.M[R - 1] = P::max(st.BM[R - 1], st.M[R - 1]);
-    st.X[R - 1] = P::max(st.BX[R - 1], st.X[R - 1]);
-    st.Y[R - 1] = P::max(st.BY[R - 1], st.Y[R - 1]);
+    pd_rows_down<P, R, G, false>(pr, st, an, qX, T, false, prior, [](int) {});
   }
 }
 
@@ -361,55 +330,63 @@ __device__ __forceinline__ uint32_t pd_synth_entry(const uint32_t* seq, int len,
   return e;
 }
 
-template <class P, int R>
-__device__ void pd_forward_pass(const LaunchArgs& a, const Program& prog, const ReadRef* rd, const uint8_t* classes,
-                                const uint32_t* sigs, int lane, PdScratch<P, R>& sc, const uint32_t* synth_seq, int synth_len) {
+template <class P, int R, int G>
+__device__ __forceinline__ void pd_forward_pass(const LaunchArgs& a, const Program& prog, const ReadRef* rd, const uint8_t* classes,
+                                                const uint32_t* sigs, int lane, PdScratch<P, R>& sc, const uint32_t* synth_seq,
+                                                int synth_len) {
   using V = typename P::V;
   using S = typename P::S;
-  PdRows<P, R> pr;
+  const int gl = lane % G;
+  PdRows<P, R, G> pr;
   pr.load(a.v, rd, lane, classes);
   V an;
 #pragma unroll
   for (int c = 0; c < P::NC; ++c)
     P::put(an, c, static_cast<S>((P::kTransformed && rd[c].len > 0) ? err_prob(a.v, a.v.ins[rd[c].off + rd[c].len - 1]) : 1.0));
-  int pad_hi = 0;
-#pragma unroll
-  for (int c = 0; c < P::NC; ++c) pad_hi = rd[c].pad > pad_hi ? rd[c].pad : pad_hi;
 
   PdState<P, R> st;
-#pragma unroll
-  for (int r = 0; r < R; ++r) st.M[r] = st.X[r] = st.Y[r] = st.BM[r] = st.BX[r] = st.BY[r] = P::zero();
-  st.acc = P::zero();
-  st.seg_i = -1;
-  PdEdge<P> ea, eb;
-  ea.M = ea.X = ea.Y = P::zero();
-  eb = ea;
+  st.clear();
   if (P::kDouble && synth_len > 0) {
     const int n = synth_len;
-    for (int t = 0; t < n + 32; t += 2) {
-      const uint32_t e0 = pd_synth_entry(synth_seq, n, t - lane), e1 = pd_synth_entry(synth_seq, n, t + 1 - lane);
-      pd_step<P, R>(a, prog, rd, lane, pr, an, pad_hi, sc, st, synth_len, e0, __ldg(sigs + (e0 & kCodeMask)), ea, eb);
-      pd_step<P, R>(a, prog, rd, lane, pr, an, pad_hi, sc, st, synth_len, e1, __ldg(sigs + (e1 & kCodeMask)), eb, ea);
+    auto at = [&](int t) {
+      const uint32_t e = pd_synth_entry(synth_seq, n, t - gl);
+      pd_step<P, R, G>(a, prog, rd, lane, pr, an, sc, st, synth_len, e, __ldg(sigs + (e & kCodeMask)));
+    };
+    int t = 0;
+    for (; t < G; ++t) at(t);
+    // Every lane strictly inside the haplotype: no events. The next entry and its signature are loaded a
+    // step ahead.
+    const uint32_t* seq = synth_seq - gl;
+    if (t < n) {
+      uint32_t e = __ldg(seq + t), g = __ldg(sigs + (e & kCodeMask));
+#pragma unroll 2
+      for (; t < n; ++t) {
+        const uint32_t e1 = t + 1 < n ? __ldg(seq + t + 1) : 0u, g1 = __ldg(sigs + (e1 & kCodeMask));
+        pd_step<P, R, G, false>(a, prog, rd, lane, pr, an, sc, st, synth_len, e, g);
+        e = e1;
+        g = g1;
+      }
     }
+    for (; t < n + G; ++t) at(t);
   } else {
     const int n = prog.fwd_len;
-    const uint32_t* stream = a.v.stream + prog.fwd_off - lane;
+    const uint32_t* stream = a.v.stream + prog.fwd_off - gl;
     // Two steps an iteration; one where no lane has an event runs a body without event code.
-    const uint32_t keep = lane == 31 ? kEvMask : (kEvMask & ~(EV_END | EV_ACC));
+    const uint32_t keep = gl == G - 1 ? kEvMask : (kEvMask & ~(EV_END | EV_ACC));
     uint32_t n0 = __ldg(stream), n1 = __ldg(stream + 1);
     uint32_t g0 = __ldg(sigs + (n0 & kCodeMask)), g1 = __ldg(sigs + (n1 & kCodeMask));
-    for (int t = 0; t < n + 32; t += 2) {
+    for (int t = 0; t < n + G; t += 2) {
       const uint32_t e0 = n0, e1 = n1, s0 = g0, s1 = g1;
       n0 = __ldg(stream + t + 2);
       n1 = __ldg(stream + t + 3);
       g0 = __ldg(sigs + (n0 & kCodeMask));
       g1 = __ldg(sigs + (n1 & kCodeMask));
       if (__any_sync(kFull, (e0 | e1) & keep)) {
-        pd_step<P, R>(a, prog, rd, lane, pr, an, pad_hi, sc, st, 0, e0, s0, ea, eb);
-        pd_step<P, R>(a, prog, rd, lane, pr, an, pad_hi, sc, st, 0, e1, s1, eb, ea);
+        pd_step<P, R, G>(a, prog, rd, lane, pr, an, sc, st, 0, e0, s0);
+        pd_step<P, R, G>(a, prog, rd, lane, pr, an, sc, st, 0, e1, s1);
       } else {
-        pd_step<P, R, false>(a, prog, rd, lane, pr, an, pad_hi, sc, st, 0, e0, s0, ea, eb);
-        pd_step<P, R, false>(a, prog, rd, lane, pr, an, pad_hi, sc, st, 0, e1, s1, eb, ea);
+        pd_step<P, R, G, false>(a, prog, rd, lane, pr, an, sc, st, 0, e0, s0);
+        pd_step<P, R, G, false>(a, prog, rd, lane, pr, an, sc, st, 0, e1, s1);
       }
     }
   }
@@ -417,13 +394,13 @@ __device__ void pd_forward_pass(const LaunchArgs& a, const Program& prog, const 
 }
 
 // Thresholds, log10 and the caller's layout (fgkl kernel.rs:897-914 via pd_kernel.rs:262-270).
-template <class P, int R>
-__device__ void pd_finalize(const LaunchArgs& a, const Task& task, const Region& region, const Program& prog, int lane,
+template <class P, int R, int G>
+__device__ __forceinline__ void pd_finalize(const LaunchArgs& a, const Task& task, const Region& region, const Program& prog, int lane,
                             PdScratch<P, R>& sc) {
   using C = Consts<P::kDouble>;
   __syncwarp();
   if (P::kDouble && task.hap >= 0) {
-    const double raw = sc.seg_raw[0];
+    const double raw = sc.raw(0, 0);
     const double result = raw != raw ? __longlong_as_double(0x7ff8000000000000ll) : log10(raw) - C::kLog10Initial;
     const int read_local = task.read[0] - region.read_off;
     for (int k = lane; k < region.n_haps; k += 32) {
@@ -442,12 +419,12 @@ __device__ void pd_finalize(const LaunchArgs& a, const Task& task, const Region&
     if (own < 0 || own >= prog.n_segs) continue;
     const double factor = a.v.segs[prog.seg_off + own].factor;
 #pragma unroll
-    for (int c = 0; c < P::NC; ++c) {
+    for (int c = 0; c < 32 / G * P::NC; ++c) {
       if (task.read[c] < 0) continue;
       const int read_local = task.read[c] - region.read_off;
       double* dst = a.v.out + region.out_off + static_cast<int64_t>(read_local) * region.n_haps + info.order;
       if (dense && !isnan(*dst)) continue;
-      const double raw = __dmul_rn(sc.seg_raw[own * P::NC + c], factor);
+      const double raw = __dmul_rn(sc.raw(own, c), factor);
       bool lost = a.min_accept_plain ? !(raw >= C::kMinAccepted) : (raw != raw);
       if (!P::kDouble) lost |= isinf(raw);
       const double result = lost ? __longlong_as_double(0x7ff8000000000000ll) : log10(raw) - C::kLog10Initial;
@@ -458,15 +435,17 @@ __device__ void pd_finalize(const LaunchArgs& a, const Task& task, const Region&
   if (lost_count && !dense) atomicAdd(&a.v.counters->lost_pairs, lost_count);
 }
 
-// Resident blocks of 4 warps the register budget is cut for (measured on c3): one-read FP32 at 4
-// (128 registers, no spill), the FP32x2 form at 2 (up to 255), FP64 at 3 for R <= 5 (168 registers,
-// a few spilled values: the recomputation sweeps run faster at 12 warps per SM than at 8), else 1.
+// Resident blocks of 4 warps the register budget is cut for. Two reads a warp at 5 rows: three (168
+// registers, a few spilled values; 256 regions of 64 reads x 16 haplotypes 8.8 ms, 9.8 at two); one read
+// a warp: four up to 6 rows and fewer above, where four spill (41 reads of 342 bases, 12 rows: 2.75 ms at
+// two, 6.3 at four); FP64 three up to 5 rows. Two reads on 16 lanes each in scalar FP32 at 10 rows measured
+// the same as two on 32 lanes in FP32x2 (8.8 ms).
 template <class P, int R>
 struct PdMinBlocks {
-  static constexpr int value = P::kDouble ? (R <= 5 ? 3 : 1) : (P::NC == 2 ? 2 : 4);
+  static constexpr int value = P::kDouble ? (R <= 5 ? 3 : 1) : (P::NC == 2 ? (R <= 5 ? 3 : 2) : (R <= 6 ? 4 : R <= 9 ? 3 : 2));
 };
 
-template <class P, int R>
+template <class P, int R, int G>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, (PdMinBlocks<P, R>::value)) pd_kernel(LaunchArgs a) {
   using V = typename P::V;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -486,7 +465,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (PdMinBlocks<P, R>::value
     ReadRef rd[P::NC];
 #pragma unroll
     for (int c = 0; c < P::NC; ++c) {
-      const int id = task.read[c];
+      const int id = task.read[lane / G * P::NC + c];
       if (id >= 0) {
         rd[c].off = a.v.read_off[id];
         rd[c].len = static_cast<int>(a.v.read_off[id + 1] - rd[c].off);
@@ -494,7 +473,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (PdMinBlocks<P, R>::value
         rd[c].off = 0;
         rd[c].len = 0;
       }
-      rd[c].pad = 32 * R - rd[c].len;
+      rd[c].pad = G * R - rd[c].len;
     }
     const uint8_t* classes = a.v.code_of_byte + region.code_off;
     const uint32_t* sigs = a.v.pd_sigs + region.sig_off;
@@ -502,117 +481,81 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (PdMinBlocks<P, R>::value
     if (P::kDouble && task.hap >= 0) {
       const HapInfo info = a.v.haps[region.hap_off + task.hap];
       PdScratch<P, R> sc(scratch, smem, 0);
-      pd_forward_pass<P, R>(a, prog, rd, classes, sigs, lane, sc, a.v.pd_entries + region.seq_off + info.seq, info.len);
-      pd_finalize<P, R>(a, task, region, prog, lane, sc);
+      pd_forward_pass<P, R, G>(a, prog, rd, classes, sigs, lane, sc, a.v.pd_entries + region.seq_off + info.seq, info.len);
+      pd_finalize<P, R, G>(a, task, region, prog, lane, sc);
     } else {
       PdScratch<P, R> sc(scratch, smem, prog.n_slots);
-      pd_forward_pass<P, R>(a, prog, rd, classes, sigs, lane, sc, nullptr, 0);
-      pd_finalize<P, R>(a, task, region, prog, lane, sc);
+      pd_forward_pass<P, R, G>(a, prog, rd, classes, sigs, lane, sc, nullptr, 0);
+      pd_finalize<P, R, G>(a, task, region, prog, lane, sc);
     }
     __syncwarp();
   }
 }
 
 // ---------------------------------------------------------------------------------------------
-// Strip-mined PD pairs (reads longer than 620 bases), and every pair of a region whose reads hold
-// more distinct bytes than the class bits cover (kGeneric): one read against one distinct
-// haplotype, unshared, over the haplotype's forward entries, the rows cut into blocks of 32 R rows
-// run one after another. Lane 0's row above comes from a carry row (merged on DEL_END columns like
-// every row): GATK's row 0 in the first block (M = X = 0, Y = INITIAL / hap_len), after that
-// the previous block's bottom row, written by lane 31 column by column and read by lane 0 31 steps
-// before lane 31 of the next block overwrites it (the plain strip-mined kernel's scheme). The
-// state a block's top row starts in is the previous row's, which the entries' later-row state
-// carries; only the read's first row (in the first block) takes the first-row state.
+// Strip-mined PD pairs (reads longer than 620 bases), every pair of a region whose reads hold more distinct
+// bytes than the class bits cover (kGeneric), and the FP64 recomputation of reads above 248 bases, whose
+// rows in one block would not fit the registers: one read against one distinct haplotype, unshared, over
+// the haplotype's forward entries, the rows cut into blocks of 32 R rows that the warps of a block run as a
+// pipeline (the plain strip-mined kernel's scheme, kernels.cu). The first block's row above is GATK's row 0
+// (M = X = 0, Y = INITIAL / hap_len). The state a block's top row starts in is the previous row's, which
+// the entries' later-row state carries; only the read's first row (in the first block) takes the first-row
+// state.
 // ---------------------------------------------------------------------------------------------
-
-constexpr int kPdCarryVals = 4;  // M, X, Y, padded to 16 bytes
 
 template <class P>
 constexpr size_t pd_long_scratch_size(int max_hap_len) {
-  return 16 + static_cast<size_t>(max_hap_len) * kPdCarryVals * sizeof(typename P::V);
-}
-
-template <class P, int R>
-__device__ __forceinline__ void pd_long_store(typename P::V* carry, const PdState<P, R>& st, int lane, int t, int n, bool last) {
-  const int p = t - 31;
-  if (!last && lane == 31 && p >= 0 && p < n) {
-    typename P::V rec[kPdCarryVals] = {st.M[R - 1], st.X[R - 1], st.Y[R - 1], P::zero()};
-    store_record(carry + static_cast<size_t>(p) * kPdCarryVals, rec);
-  }
+  return static_cast<size_t>(max_hap_len) * sizeof(Carry<P>);
 }
 
 template <class P>
-__device__ __forceinline__ void pd_long_fetch(const typename P::V* carry, typename P::V (&rec)[kPdCarryVals], int lane, int p, int n,
-                                              bool first) {
-  if (!first && lane == 0 && p < n) load_record(rec, carry + static_cast<size_t>(p) * kPdCarryVals);
+constexpr size_t pd_long_smem_per_warp() {
+  return kRing * sizeof(Carry<P>);
 }
 
-template <class P, int R>
-__device__ __forceinline__ void pd_set_carry(PdState<P, R>& st, const typename P::V (&c)[kPdCarryVals]) {
-  st.cM = c[0];
-  st.cX = c[1];
-  st.cY = c[2];
-}
-
-template <class P, int R, bool kGeneric>
-__device__ void pd_long_block(const LaunchArgs& a, const ReadRef* rd, int lane, const PdRows<P, R>& pr, typename P::V an,
-                              PdScratch<P, R>& sc, const uint32_t* seq, const uint32_t* sigs, int n, typename P::V* carry,
-                              bool first, bool last) {
-  using V = typename P::V;
-  using S = typename P::S;
-  const int pad_hi = rd[0].pad;
-  PdState<P, R> st;
-#pragma unroll
-  for (int r = 0; r < R; ++r) st.M[r] = st.X[r] = st.Y[r] = st.BM[r] = st.BX[r] = st.BY[r] = P::zero();
-  st.acc = P::zero();
-  st.seg_i = -1;
-  st.cM = st.cX = P::zero();
-  st.cY = first ? static_cast<S>(Consts<P::kDouble>::kInitial / n) : P::zero();
+// One superstep of a warp: steps t0 .. t0 + kChunk - 1. kInner: every lane is strictly inside the haplotype
+// throughout, so no events and no bounds.
+template <class P, int R, bool kGeneric, bool kInner>
+__device__ __forceinline__ void pd_long_superstep(const LaunchArgs& a, const ReadRef* rd, int lane, const PdRows<P, R, 32>& pr,
+                                                  typename P::V an, PdScratch<P, R>& sc, PdState<P, R>& st, const uint32_t* seq,
+                                                  const uint32_t* sigs, int n, int t0, const Carry<P>* in, Carry<P>* out,
+                                                  int out_mask) {
   const Program prog{};
-  PdEdge<P> ea, eb;
-  ea.M = ea.X = ea.Y = P::zero();
-  eb = ea;
-  V n0[kPdCarryVals], n1[kPdCarryVals];
-#pragma unroll
-  for (int i = 0; i < kPdCarryVals; ++i) n0[i] = n1[i] = P::zero();
-  pd_long_fetch<P>(carry, n0, lane, 0, n, first);
-  pd_long_fetch<P>(carry, n1, lane, 1, n, first);
-  for (int t = 0; t < n + 32; t += 2) {
-    const uint32_t e0 = pd_synth_entry(seq, n, t - lane), e1 = pd_synth_entry(seq, n, t + 1 - lane);
-    const uint32_t s0 = kGeneric ? 0u : __ldg(sigs + (e0 & kCodeMask)), s1 = kGeneric ? 0u : __ldg(sigs + (e1 & kCodeMask));
-    V c0[kPdCarryVals], c1[kPdCarryVals];
-#pragma unroll
-    for (int i = 0; i < kPdCarryVals; ++i) {
-      c0[i] = n0[i];
-      c1[i] = n1[i];
-    }
-    pd_long_fetch<P>(carry, n0, lane, t + 2, n, first);
-    pd_long_fetch<P>(carry, n1, lane, t + 3, n, first);
-    if (!first) pd_set_carry<P, R>(st, c0);
-    pd_step<P, R, true, true, kGeneric>(a, prog, rd, lane, pr, an, pad_hi, sc, st, n, e0, s0, ea, eb);
-    pd_long_store<P, R>(carry, st, lane, t, n, last);
-    if (!first) pd_set_carry<P, R>(st, c1);
-    pd_step<P, R, true, true, kGeneric>(a, prog, rd, lane, pr, an, pad_hi, sc, st, n, e1, s1, eb, ea);
-    pd_long_store<P, R>(carry, st, lane, t + 1, n, last);
+#pragma unroll 2
+  for (int i = 0; i < kChunk; ++i) {
+    const int t = t0 + i;
+    const uint32_t e = kInner ? __ldg(seq + t - lane) : pd_synth_entry(seq, n, t - lane);
+    const uint32_t sig = kGeneric ? 0u : __ldg(sigs + (e & kCodeMask));
+    const Carry<P> c = in[t & (kRing - 1)];
+    st.cX = c.x;
+    st.cT = c.t;
+    pd_step<P, R, 32, !kInner, true, kGeneric>(a, prog, rd, lane, pr, an, sc, st, n, e, sig);
+    const int p = t - 31;  // lane 31's column
+    if (lane == 31 && out && (kInner || (p >= 0 && p < n))) out[p & out_mask] = Carry<P>{st.xs, st.ts};
   }
 }
 
 template <class P, int R, bool kGeneric>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, (P::kDouble ? 1 : 2)) pd_long_kernel(LaunchArgs a) {
+__global__ void __launch_bounds__(kLongWarps * 32, 1) pd_long_kernel(LaunchArgs a) {
   using V = typename P::V;
   using S = typename P::S;
   using C = Consts<P::kDouble>;
-  const int lane = threadIdx.x & 31;
-  const int warp = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int s_task;
+  __shared__ double s_raw[kLongWarps][kMaxReads];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  Carry<P>* const ring = reinterpret_cast<Carry<P>*>(smem_raw) + w * kRing;  // what the warp's top row takes
   const int count = a.count ? min(*a.count, a.n_tasks) : a.n_tasks;
-  char* scratch = a.scratch + static_cast<size_t>(warp) * a.scratch_stride;
-  V* carry = reinterpret_cast<V*>(scratch + 16);
+  // The block's scratch: one carry entry a column, from the last warp of a round to the first of the next.
+  Carry<P>* const carry = reinterpret_cast<Carry<P>*>(a.scratch + static_cast<size_t>(blockIdx.x) * a.scratch_stride);
+  PdScratch<P, R> sc(nullptr, nullptr, 0);
+  sc.seg_raw = s_raw[w];
   for (;;) {
-    int t = 0;
-    if (lane == 0) t = atomicAdd(a.task_counter, 1);
-    t = __shfl_sync(kFull, t, 0);
-    if (t >= count) break;
-    const Task task = a.tasks[t];
+    if (threadIdx.x == 0) s_task = atomicAdd(a.task_counter, 1);
+    __syncthreads();
+    const int task_i = s_task;
+    if (task_i >= count) break;
+    const Task task = a.tasks[task_i];
     const Region region = a.v.regions[task.region];
     const HapInfo info = a.v.haps[region.hap_off + task.hap];
     const uint32_t* seq = a.v.pd_entries + region.seq_off + info.seq;
@@ -624,46 +567,83 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (P::kDouble ? 1 : 2)) pd_
     rd[0].len = static_cast<int>(a.v.read_off[task.read[0] + 1] - rd[0].off);
     const int blocks = long_blocks(rd[0].len, R);
     const int pad0 = 32 * R * blocks - rd[0].len;
-    PdScratch<P, R> sc(scratch, nullptr, 0);
     const V an = static_cast<S>(P::kTransformed ? err_prob(a.v, a.v.ins[rd[0].off + rd[0].len - 1]) : 1.0);
-    for (int b = 0; b < blocks; ++b) {
-      rd[0].pad = pad0 - 32 * R * b;
-      PdRows<P, R> pr;
-      if (kGeneric)
-        pr.load_generic(a.v, rd, lane, classes);
-      else
-        pr.load(a.v, rd, lane, classes);
-      pd_long_block<P, R, kGeneric>(a, rd, lane, pr, an, sc, seq, sigs, n, carry, b == 0, b == blocks - 1);
-      __syncwarp();
+    for (int b0 = 0; b0 < blocks; b0 += warps) {
+      const int in_round = min(warps, blocks - b0), b = b0 + w;
+      const bool on = w < in_round;
+      PdRows<P, R, 32> pr;
+      PdState<P, R> st;
+      st.clear();
+      Carry<P> next{S(0), S(0)};  // the first warp's input for column t0 + kChunk + lane
+      if (on) {
+        rd[0].pad = pad0 - 32 * R * b;
+        if (kGeneric)
+          pr.load_generic(a.v, rd, lane, classes);
+        else
+          pr.load(a.v, rd, lane, classes);
+        if (b == 0) {
+          // GATK's row 0 above the first block. Below a padding row nothing reads it.
+          if (pad0 == 0) {
+            const BracketFactors<P> k(row_model(a.v, rd[0], 0, classes));
+            next.t = cell_match<P>(S(0), S(0), static_cast<S>(C::kInitial / n), k.k0, k.k1, k.k2);
+          }
+        } else if (w == 0 && lane < n) {
+          next = carry[lane];
+        }
+        __syncwarp();
+      }
+      // The last row block hands nothing on; a round's last warp hands on through the scratch.
+      const bool through_ring = w + 1 < in_round;
+      Carry<P>* const out = !on || b == blocks - 1 ? nullptr : (through_ring ? ring + kRing : carry);
+      const int out_mask = through_ring ? kRing - 1 : -1;
+      const int supersteps = (n + 32 + kChunk - 1) / kChunk + (in_round - 1) * kDelay;
+      for (int s = 0; s < supersteps; ++s) {
+        const int t0 = (s - w * kDelay) * kChunk;
+        if (on && t0 >= 0 && t0 < n + 32) {
+          if (w == 0) {
+            ring[(t0 + lane) & (kRing - 1)] = next;
+            const int col = t0 + kChunk + lane;
+            if (b > 0 && col < n) next = carry[col];
+            __syncwarp();
+          }
+          if (t0 >= 32 && t0 + kChunk <= n)
+            pd_long_superstep<P, R, kGeneric, true>(a, rd, lane, pr, an, sc, st, seq, sigs, n, t0, ring, out, out_mask);
+          else
+            pd_long_superstep<P, R, kGeneric, false>(a, rd, lane, pr, an, sc, st, seq, sigs, n, t0, ring, out, out_mask);
+        }
+        __syncthreads();
+      }
     }
-    const double raw = sc.seg_raw[0];
-    bool lost = a.min_accept_plain ? !(raw >= C::kMinAccepted) : (raw != raw);
-    if (!P::kDouble) lost |= isinf(raw);
-    const double result = lost ? __longlong_as_double(0x7ff8000000000000ll) : log10(raw) - C::kLog10Initial;
-    const int read_local = task.read[0] - region.read_off;
-    unsigned long long lost_count = 0;
-    for (int k = lane; k < region.n_haps; k += 32) {
-      const HapInfo h = a.v.haps[region.hap_off + k];
-      if (h.src != task.hap) continue;
-      a.v.out[region.out_off + static_cast<int64_t>(read_local) * region.n_haps + h.order] = result;
-      lost_count += lost;
+    if (w == 0) {
+      const double raw = s_raw[(blocks - 1) % warps][0];
+      bool lost = a.min_accept_plain ? !(raw >= C::kMinAccepted) : (raw != raw);
+      if (!P::kDouble) lost |= isinf(raw);
+      const double result = lost ? __longlong_as_double(0x7ff8000000000000ll) : log10(raw) - C::kLog10Initial;
+      const int read_local = task.read[0] - region.read_off;
+      unsigned long long lost_count = 0;
+      for (int k = lane; k < region.n_haps; k += 32) {
+        const HapInfo h = a.v.haps[region.hap_off + k];
+        if (h.src != task.hap) continue;
+        a.v.out[region.out_off + static_cast<int64_t>(read_local) * region.n_haps + h.order] = result;
+        lost_count += lost;
+      }
+      if (lost_count) atomicAdd(&a.v.counters->lost_pairs, lost_count);
     }
-    if (lost_count) atomicAdd(&a.v.counters->lost_pairs, lost_count);
-    __syncwarp();
+    __syncthreads();
   }
 }
 
 template <class P, int R>
 void pd_occ(int* blocks, int warps) {
   static std::atomic<int> cache[3][kMaxDevices];
-  *blocks = resident_blocks(pd_kernel<P, R>, warps * PdLayout<P, R>::kSmemPerWarp, warps * 32, cache[warps_index(warps)],
+  *blocks = resident_blocks(pd_kernel<P, R, 32>, warps * PdLayout<P, R>::kSmemPerWarp, warps * 32, cache[warps_index(warps)],
                             kWarpsPerBlock * PdLayout<P, R>::kSmemPerWarp);
 }
 
 template <class P, int R>
 cudaError_t pd_go(int blocks, const LaunchArgs& a, cudaStream_t s, int warps) {
   const size_t smem = warps * PdLayout<P, R>::kSmemPerWarp;
-  pd_kernel<P, R><<<blocks, warps * 32, smem, s>>>(a);
+  pd_kernel<P, R, 32><<<blocks, warps * 32, smem, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -714,9 +694,15 @@ auto pd_long_rows(int rows, F&& f) {
 }
 
 template <class P, int R, bool kGeneric>
-void pd_long_occ(int* blocks) {
-  static std::atomic<int> cache[kMaxDevices];
-  *blocks = resident_blocks(pd_long_kernel<P, R, kGeneric>, 0, kWarpsPerBlock * 32, cache);
+void pd_long_occ(int* blocks, int warps) {
+  static std::atomic<int> cache[kLongWarps + 1][kMaxDevices];
+  *blocks = resident_blocks(pd_long_kernel<P, R, kGeneric>, warps * pd_long_smem_per_warp<P>(), warps * 32, cache[warps],
+                            kLongWarps * pd_long_smem_per_warp<P>());
+}
+
+template <class P, int R, bool kGeneric>
+void pd_long_go(int blocks, const LaunchArgs& a, cudaStream_t s, int warps) {
+  pd_long_kernel<P, R, kGeneric><<<blocks, warps * 32, warps * pd_long_smem_per_warp<P>(), s>>>(a);
 }
 
 }  // namespace
@@ -726,30 +712,30 @@ size_t pd_long_scratch_bytes(Kind k, int, int max_hap_len) {
   return dbl ? pd_long_scratch_size<OneF64>(max_hap_len) : pd_long_scratch_size<OneF32>(max_hap_len);
 }
 
-void pd_long_occupancy(Kind k, int rows, int* blocks, int* threads) {
-  *threads = kWarpsPerBlock * 32;
+void pd_long_occupancy(Kind k, int rows, int* blocks, int* threads, int warps) {
+  *threads = warps * 32;
   *blocks = 0;
   pd_long_rows(rows, [&](auto r) {
     constexpr int R = decltype(r)::value;
     switch (k) {
-      case Kind::kLongF32Pd: pd_long_occ<OneF32, R, false>(blocks); break;
-      case Kind::kLongF64Pd: pd_long_occ<OneF64, R, false>(blocks); break;
-      case Kind::kGenericF32Pd: pd_long_occ<OneF32, R, true>(blocks); break;
-      case Kind::kGenericF64Pd: pd_long_occ<OneF64, R, true>(blocks); break;
+      case Kind::kLongF32Pd: pd_long_occ<OneF32, R, false>(blocks, warps); break;
+      case Kind::kLongF64Pd: pd_long_occ<OneF64, R, false>(blocks, warps); break;
+      case Kind::kGenericF32Pd: pd_long_occ<OneF32, R, true>(blocks, warps); break;
+      case Kind::kGenericF64Pd: pd_long_occ<OneF64, R, true>(blocks, warps); break;
       default: break;
     }
     return 0;
   });
 }
 
-cudaError_t pd_long_launch(Kind k, int rows, int blocks, const LaunchArgs& a, cudaStream_t s) {
+cudaError_t pd_long_launch(Kind k, int rows, int blocks, const LaunchArgs& a, cudaStream_t s, int warps) {
   return pd_long_rows(rows, [&](auto r) -> cudaError_t {
     constexpr int R = decltype(r)::value;
     switch (k) {
-      case Kind::kLongF32Pd: pd_long_kernel<OneF32, R, false><<<blocks, kWarpsPerBlock * 32, 0, s>>>(a); break;
-      case Kind::kLongF64Pd: pd_long_kernel<OneF64, R, false><<<blocks, kWarpsPerBlock * 32, 0, s>>>(a); break;
-      case Kind::kGenericF32Pd: pd_long_kernel<OneF32, R, true><<<blocks, kWarpsPerBlock * 32, 0, s>>>(a); break;
-      case Kind::kGenericF64Pd: pd_long_kernel<OneF64, R, true><<<blocks, kWarpsPerBlock * 32, 0, s>>>(a); break;
+      case Kind::kLongF32Pd: pd_long_go<OneF32, R, false>(blocks, a, s, warps); break;
+      case Kind::kLongF64Pd: pd_long_go<OneF64, R, false>(blocks, a, s, warps); break;
+      case Kind::kGenericF32Pd: pd_long_go<OneF32, R, true>(blocks, a, s, warps); break;
+      case Kind::kGenericF64Pd: pd_long_go<OneF64, R, true>(blocks, a, s, warps); break;
       default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

@@ -106,19 +106,6 @@ __device__ __forceinline__ void load_priors(const typename P::V* table, int code
 // Forward coefficients of the lane's rows. What row r + 1 takes from row r is held with row r (k0..k3
 // at index r are row r + 1's), because the lane computes both values that its bottom row hands to the
 // lane below: the bracket of that lane's top match value and its new insertion value.
-// Factors of a row's match bracket (cell_match). X^ = X / mi and Y^ = Y / md (FP32 form):
-// S = mm*M + (im*mi')*X^ + (im*md')*Y^ is taken as mm * (M + (im*mi'/mm)*X^ + (im*md'/mm)*Y^) with mm in
-// the prior table.
-template <class P>
-struct BracketFactors {
-  using S = typename P::S;
-  S k0, k1, k2;
-  __device__ explicit BracketFactors(const RowModel& m)
-      : k0(static_cast<S>(m.mm)),
-        k1(static_cast<S>(!P::kTransformed ? m.im : (m.read ? m.im * m.mi_prev / m.mm : 0.0))),
-        k2(!P::kTransformed ? k1 : static_cast<S>(m.read ? m.im * m.md_prev / m.mm : 0.0)) {}
-};
-
 template <class P, int R, int G>
 struct FwdRows {
   using V = typename P::V;
