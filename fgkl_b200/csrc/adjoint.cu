@@ -1,7 +1,11 @@
 // sm_100a adjoint kernels: gradients of the summed log10 likelihood with respect to every read
 // position's gap-open (insertion, deletion), gap-continuation and base-error probabilities.
 //
-// One warp per read: for each haplotype of the read's region, in caller order,
+// One warp per read, or, where the reads are fewer than the warps that fit the GPU, several per read, each for
+// a share of the haplotypes with gradient arrays of its own, added up part by part at the end (16 regions
+// of 2 reads of 89-445 bases x 8 haplotypes: 17.7 ms at one warp a read, 3.1 at eight, 1.4 with the launches of
+// different rows per lane side by side). A warp, for
+// each of its haplotypes, in caller order,
 //   1. a backward sweep (the reverse wavefront of the suffix-sharing backward pass, right to left
 //      over the haplotype) computes B = d(raw)/d(cell state) for M, X and Y, scaled by 2^120 in FP32
 //      at the read's last row. It keeps nothing per cell: it saves its state every K steps, and the
@@ -41,6 +45,7 @@
 // Most steps of a one-block read are interior: every lane lies strictly inside the haplotype in both
 // sweeps (steps 32 .. m - 1). Those steps, block by block, run without the column-0 resets, the
 // masks of lanes outside the haplotype and the row-block exchanges.
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 
@@ -675,16 +680,45 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (AdjMinBlocks<P, R>::valu
     if (lane == 0) t = atomicAdd(a.task_counter, 1);
     t = __shfl_sync(kFull, t, 0);
     if (t >= count) break;
-    const int read = a.tasks[t];
+    const int read = a.tasks[t] / a.split, part = a.tasks[t] % a.split;
     const int g = a.v.read_region[read];
+    AdjView v = a.v;
+    if (part > 0) {
+      v.g_ins = a.part + static_cast<size_t>(part - 1) * 4 * a.part_len;
+      v.g_del = v.g_ins + a.part_len;
+      v.g_eps = v.g_del + a.part_len;
+      v.g_err = v.g_eps + a.part_len;
+    }
     const int64_t off = a.v.read_off[read];
     const int len = static_cast<int>(a.v.read_off[read + 1] - off);
     const int blocks = adj_row_blocks(len, R);
     const int pad0 = 32 * R * blocks - len;
     const int h0 = a.v.region_hap[g], nh = a.v.region_nhap[g];
     const int read_local = read - a.v.region_read[g];
+    if (a.count) {
+      // The FP64 recomputation sums this part's gradients afresh: clear what the FP32 pass added, each
+      // position by the lane that adds to it (atomics of one thread to one address keep their order).
+      for (int blk = 0; blk < blocks; ++blk)
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int q = lane * R + r - (pad0 - 32 * R * blk);
+          if (q < 0 || q >= len) continue;
+          atomicExch(reinterpret_cast<unsigned long long*>(v.g_ins + off + q), 0ull);
+          atomicExch(reinterpret_cast<unsigned long long*>(v.g_del + off + q), 0ull);
+          atomicExch(reinterpret_cast<unsigned long long*>(v.g_eps + off + q), 0ull);
+          atomicExch(reinterpret_cast<unsigned long long*>(v.g_err + off + q), 0ull);
+        }
+      __syncwarp();
+    }
     bool lost = false;
-    for (int h = 0; h < nh && !lost; ++h) {
+    const int h_end = static_cast<int>(static_cast<int64_t>(nh) * (part + 1) / a.split);
+    for (int h = static_cast<int>(static_cast<int64_t>(nh) * part / a.split); h < h_end; ++h) {
+      // A part of a read that another part has lost already need not go on.
+      if (!P::kDouble && a.split > 1) {
+        int gone = 0;
+        if (lane == 0) gone = *static_cast<volatile int*>(a.lost_flag + read);
+        if (__shfl_sync(kFull, gone, 0)) break;
+      }
       const int64_t hlo = a.v.hap_off[h0 + h];
       const int m = static_cast<int>(a.v.hap_off[h0 + h + 1] - hlo);
       const uint8_t* hap = a.v.hap_bases + hlo;
@@ -721,7 +755,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (AdjMinBlocks<P, R>::valu
         AdjCoef<P, R> c;
         const int pad = pad0 - 32 * R * blk;
         c.load(a.v, off, len, pad, lane);
-        fwd = adj_forward<P, R>(a.v, c, off, pad, hap, m, lane, sc, blk, smem, c_fac, init_a);
+        fwd = adj_forward<P, R>(v, c, off, pad, hap, m, lane, sc, blk, smem, c_fac, init_a);
         __syncwarp();
       }
       const double fwd_raw = ldexp(static_cast<double>(fwd), shift);
@@ -732,30 +766,24 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (AdjMinBlocks<P, R>::valu
       if (lane == 0) a.v.out[a.v.region_out[g] + static_cast<int64_t>(read_local) * nh + h] = log10(fwd_raw) - C::kLog10Initial;
       __syncwarp();
     }
-    if (lost) {
-      // The FP64 recomputation sums this read's gradients afresh: clear what earlier haplotypes added,
-      // each position by the lane that added to it (atomics of one thread to one address keep their
-      // order).
-      for (int blk = 0; blk < blocks; ++blk)
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int q = lane * R + r - (pad0 - 32 * R * blk);
-          if (q < 0 || q >= len) continue;
-          atomicExch(reinterpret_cast<unsigned long long*>(a.v.g_ins + off + q), 0ull);
-          atomicExch(reinterpret_cast<unsigned long long*>(a.v.g_del + off + q), 0ull);
-          atomicExch(reinterpret_cast<unsigned long long*>(a.v.g_eps + off + q), 0ull);
-          atomicExch(reinterpret_cast<unsigned long long*>(a.v.g_err + off + q), 0ull);
-        }
-      __syncwarp();
-      if (lane == 0) {
-        atomicAdd(a.v.lost, 1ull);
-        if (a.queue) {
-          const int bin = adj_rows(len);
-          const int slot = atomicAdd(a.queue_tail + bin, 1);
-          if (slot < a.queue_off[bin + 1] - a.queue_off[bin]) a.queue[a.queue_off[bin] + slot] = read;
-        }
+    if (lost && lane == 0 && atomicExch(a.lost_flag + read, 1) == 0) {
+      atomicAdd(a.v.lost, 1ull);
+      if (a.queue) {
+        const int bin = adj_rows(len);
+        const int slot = atomicAdd(a.queue_tail + bin, a.split);
+        if (slot + a.split <= a.queue_off[bin + 1] - a.queue_off[bin])
+          for (int k = 0; k < a.split; ++k) a.queue[a.queue_off[bin] + slot + k] = read * a.split + k;
       }
     }
+    __syncwarp();
+  }
+}
+
+__global__ void adj_reduce_kernel(double* grad, const double* part, size_t n, int parts) {
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    double g = grad[i];
+    for (int k = 0; k < parts; ++k) g = __dadd_rn(g, part[static_cast<size_t>(k) * n + i]);
+    grad[i] = g;
   }
 }
 
@@ -815,6 +843,13 @@ void adj_occupancy(bool dbl, int rows, int* blocks, int* threads) {
       adj_occ<OneF32, R>(blocks);
     return 0;
   });
+}
+
+cudaError_t adj_reduce(const AdjLaunch& a, cudaStream_t s) {
+  const size_t n = 4 * a.part_len;
+  if (a.split < 2 || n == 0) return cudaSuccess;
+  adj_reduce_kernel<<<static_cast<int>(std::min<size_t>((n + 255) / 256, 2048)), 256, 0, s>>>(a.v.g_ins, a.part, n, a.split - 1);
+  return cudaGetLastError();
 }
 
 cudaError_t adj_launch(bool dbl, int rows, int blocks, const AdjLaunch& a, cudaStream_t s) {

@@ -39,13 +39,17 @@ struct AdjView {
 
 struct AdjLaunch {
   AdjView v;
-  const int32_t* tasks;  // global read indices
+  const int32_t* tasks;  // read * split + part: a part's haplotypes (an even share, in order) of a read
   int n_tasks;           // count, or the capacity when `count` is set
   const int* count;      // device-side count (FP64 recomputation queue), or nullptr
   int* task_counter;     // zeroed before the launch
   char* scratch;
   size_t scratch_stride; // bytes per warp (adj_scratch_bytes of the launch's largest pair)
-  int32_t* queue;        // FP32 launches: reads lost in FP32, for FP64 (per-bin slices), or nullptr
+  int split;             // parts that a read's haplotypes are shared among
+  double* part;          // gradients of parts 1 .. split - 1, four arrays each (part 0 adds into the view's)
+  size_t part_len;       // read positions: the length of one array
+  int* lost_flag;        // per read: set by the first part that loses it in FP32; zeroed before the launch
+  int32_t* queue;        // FP32 launches: tasks of reads lost in FP32, for FP64 (per-bin slices), or nullptr
   const int* queue_off;  // per rows-per-lane bin: first queue slot (kAdjRowBins + 1 entries)
   int* queue_tail;       // per bin
 };
@@ -71,6 +75,8 @@ __host__ __device__ inline int adj_row_blocks(int len, int rows) { return (len +
 // pass between row blocks.
 size_t adj_scratch_bytes(bool dbl, int rows, int read_len, int hap_len);
 void adj_occupancy(bool dbl, int rows, int* blocks_per_sm, int* threads_per_block);
+// Adds the parts' gradients into the view's, part by part, so the order is fixed.
+cudaError_t adj_reduce(const AdjLaunch& a, cudaStream_t stream);
 cudaError_t adj_launch(bool dbl, int rows, int blocks, const AdjLaunch& a, cudaStream_t stream);
 
 }  // namespace fgkl

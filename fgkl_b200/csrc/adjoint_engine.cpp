@@ -13,6 +13,8 @@ namespace {
 
 constexpr int kWarps = 4;                             // warps per block of the adjoint kernels
 constexpr size_t kScratchBudget = size_t{8} << 30;    // per-warp checkpoints of one launch, at most 8 GiB
+constexpr size_t kSideBudget = size_t{1} << 30;       // scratch of bins that run side by side
+constexpr size_t kPartBudget = size_t{256} << 20;     // gradient arrays of the parts beyond the first
 
 size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
@@ -22,6 +24,11 @@ AdjointEngine::AdjointEngine(int device, cudaStream_t stream) : device_(device),
   DeviceGuard device_guard(device_);
   cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_);
   cudaMalloc(&d_lost_, sizeof(unsigned long long));
+  for (int i = 0; i < kAux; ++i) {
+    cudaStreamCreateWithFlags(&aux_[i], cudaStreamNonBlocking);
+    cudaEventCreateWithFlags(&join_[i], cudaEventDisableTiming);
+  }
+  cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming);
 }
 
 AdjointEngine::~AdjointEngine() {
@@ -34,7 +41,14 @@ AdjointEngine::~AdjointEngine() {
   cudaFree(d_out_);
   cudaFree(d_small_);
   cudaFree(d_lost_);
+  cudaFree(d_part_);
   cudaFree(d_scratch_);
+  for (int i = 0; i < kAux; ++i) {
+    if (aux_[i]) cudaStreamSynchronize(aux_[i]);
+    if (aux_[i]) cudaStreamDestroy(aux_[i]);
+    if (join_[i]) cudaEventDestroy(join_[i]);
+  }
+  if (fork_) cudaEventDestroy(fork_);
 }
 
 int AdjointEngine::fail(int code, const std::string& msg) {
@@ -131,22 +145,33 @@ int AdjointEngine::prepare(const AdjointInput& in, bool double_precision) {
       need[rows] = std::max(need[rows], std::max(adj_scratch_bytes(dbl_, rows, len, longest), adj_scratch_bytes(true, rows, len, longest)));
     }
   }
+  // Parts a read's haplotypes are shared among: enough for twice the warps that fit the GPU (12 an SM), no
+  // more than the largest region's haplotypes, or than kPartBudget of gradient arrays holds.
+  int most_haps = 1;
+  for (int g = 0; g < N; ++g) most_haps = std::max(most_haps, static_cast<int>(in.region_haps[g]));
+  int64_t split = total_reads > 0 ? (2 * 12 * static_cast<int64_t>(sms_)) / total_reads : 1;
+  split = std::min<int64_t>(split, most_haps);
+  if (grad_len_ > 0) split = std::min<int64_t>(split, 1 + static_cast<int64_t>(kPartBudget / (4 * sizeof(double) * static_cast<size_t>(grad_len_))));
+  split_ = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(split, INT32_MAX / std::max<int64_t>(1, total_reads))));
   std::vector<int32_t> tasks;
   for (auto& [rows, list] : by_rows) {
     std::stable_sort(list.begin(), list.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-    Bin b{dbl_, rows, static_cast<int>(tasks.size()), static_cast<int>(list.size()), 0, 0};
-    for (auto& e : list) tasks.push_back(e.second);
+    Bin b{dbl_, rows, static_cast<int>(tasks.size()), static_cast<int>(list.size()) * split_, 0, 0};
+    for (auto& e : list)
+      for (int k = 0; k < split_; ++k) tasks.push_back(e.second * split_ + k);
     bins_.push_back(b);
   }
   std::vector<int> queue_off(kAdjRowBins + 1, 0);
-  for (int r = 0; r < kAdjRowBins; ++r) queue_off[r + 1] = queue_off[r] + (dbl_ ? 0 : per_rows[r]);
+  for (int r = 0; r < kAdjRowBins; ++r) queue_off[r + 1] = queue_off[r] + (dbl_ ? 0 : per_rows[r] * split_);
   if (!dbl_)
     for (int r = 1; r < kAdjRowBins; ++r)
-      if (per_rows[r]) rescue_.push_back(Bin{true, r, queue_off[r], per_rows[r], 0, 0});
-  // Bins run one after another, so they share the scratch; a bin's grid shrinks only when its warps'
-  // scratch would exceed the budget (very long pairs).
-  size_t scratch = 256;
-  for (auto* list : {&bins_, &rescue_})
+      if (per_rows[r]) rescue_.push_back(Bin{true, r, queue_off[r], per_rows[r] * split_, 0, 0});
+  // The bins of a pass run side by side where a scratch of its own for each fits kSideBudget (a bin of a few
+  // reads leaves most of the GPU idle), else one after another on one scratch. A bin's grid shrinks only
+  // when its warps' scratch would exceed the budget (very long pairs).
+  size_t scratch = 256, side = 0;
+  for (auto* list : {&bins_, &rescue_}) {
+    size_t sum = 0;
     for (Bin& b : *list) {
       int per_sm = 0, threads = 0;
       adj_occupancy(b.dbl, b.rows, &per_sm, &threads);
@@ -156,7 +181,13 @@ int AdjointEngine::prepare(const AdjointInput& in, bool double_precision) {
       const int64_t by_budget = static_cast<int64_t>(kScratchBudget / (kWarps * b.stride));
       b.blocks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, by_budget)));
       scratch = std::max(scratch, static_cast<size_t>(b.blocks) * kWarps * b.stride);
+      b.scratch_off = sum;
+      sum += static_cast<size_t>(b.blocks) * kWarps * b.stride;
     }
+    side = std::max(side, sum);
+  }
+  side_by_side_ = side <= kSideBudget;
+  if (side_by_side_) scratch = std::max(scratch, side);
 
   // Device buffers.
   const size_t n_bytes = static_cast<size_t>(grad_len_) + static_cast<size_t>(hap_bytes) + 16;
@@ -166,7 +197,8 @@ int AdjointEngine::prepare(const AdjointInput& in, bool double_precision) {
   if (!grow(d_bytes_, cap_bytes_, n_bytes) || !grow(d_params_, cap_params_, 4 * static_cast<size_t>(grad_len_) + 1) ||
       !grow(d_off_, cap_off_, n_off + 1) || !grow(d_idx_, cap_idx_, n_idx + 1) ||
       !grow(d_out_, cap_out_, static_cast<size_t>(out_len_) + 4 * static_cast<size_t>(grad_len_) + 1) ||
-      !grow(d_small_, cap_small_, static_cast<size_t>(n_small_)) || !grow(d_scratch_, cap_scratch_, scratch))
+      !grow(d_part_, cap_part_, static_cast<size_t>(split_ - 1) * 4 * static_cast<size_t>(grad_len_)) ||
+      !grow(d_small_, cap_small_, static_cast<size_t>(n_small_) + static_cast<size_t>(total_reads)) || !grow(d_scratch_, cap_scratch_, scratch))
     return fail(FGKL_E_OUT_OF_MEMORY, "device allocation failed");
 
   std::vector<int32_t> region_hap(N), region_nhap(N), region_read(N);
@@ -232,6 +264,7 @@ int AdjointEngine::prepare(const AdjointInput& in, bool double_precision) {
   view_.g_eps = view_.g_del + G;
   view_.g_err = view_.g_eps + G;
   view_.lost = d_lost_;
+  n_reads_ = total_reads;
   return FGKL_OK;
 }
 
@@ -249,25 +282,46 @@ int AdjointEngine::run() {
   if (grad_len_ > 0 &&
       (rc = check(cudaMemsetAsync(view_.g_ins, 0, 4 * static_cast<size_t>(grad_len_) * sizeof(double), stream_), "reset gradients")))
     return rc;
+  const size_t part_bytes = static_cast<size_t>(split_ - 1) * 4 * static_cast<size_t>(grad_len_) * sizeof(double);
+  if (part_bytes > 0 && (rc = check(cudaMemsetAsync(d_part_, 0, part_bytes, stream_), "reset gradients"))) return rc;
+  int* lost_flag = d_small_ + n_small_;
+  if (n_reads_ > 0 && (rc = check(cudaMemsetAsync(lost_flag, 0, static_cast<size_t>(n_reads_) * sizeof(int), stream_), "reset flags"))) return rc;
   launches_ = 0;
   int i = 0;
+  AdjLaunch parts{};
+  parts.v = view_;
+  parts.split = split_;
+  parts.part = d_part_;
+  parts.part_len = static_cast<size_t>(grad_len_);
+  parts.lost_flag = lost_flag;
   for (int pass = 0; pass < 2; ++pass) {
     const auto& list = pass == 0 ? bins_ : rescue_;
-    for (const Bin& b : list) {
-      AdjLaunch a{};
-      a.v = view_;
+    const bool fork = side_by_side_ && list.size() > 1;
+    if (fork && (rc = check(cudaEventRecord(fork_, stream_), "fork"))) return rc;
+    for (size_t k = 0; k < list.size(); ++k) {
+      const Bin& b = list[k];
+      const cudaStream_t s = fork ? aux_[k % kAux] : stream_;
+      if (fork && (rc = check(cudaStreamWaitEvent(s, fork_, 0), "fork wait"))) return rc;
+      AdjLaunch a = parts;
       a.tasks = (pass == 0 ? tasks_ : queue_) + b.task_off;
       a.n_tasks = b.n_tasks;
       a.count = pass == 0 ? nullptr : queue_tail + b.rows;
       a.task_counter = counters + i++;
-      a.scratch = d_scratch_;
+      a.scratch = d_scratch_ + (fork ? b.scratch_off : 0);
       a.scratch_stride = b.stride;
       a.queue = (pass == 0 && !dbl_) ? queue_ : nullptr;
       a.queue_off = queue_off;
       a.queue_tail = queue_tail;
-      if ((rc = check(adj_launch(b.dbl, b.rows, b.blocks, a, stream_), "adjoint launch"))) return rc;
+      if ((rc = check(adj_launch(b.dbl, b.rows, b.blocks, a, s), "adjoint launch"))) return rc;
       ++launches_;
+      if (fork && (rc = check(cudaEventRecord(join_[k % kAux], s), "join"))) return rc;
     }
+    for (size_t k = 0; fork && k < std::min<size_t>(list.size(), kAux); ++k)
+      if ((rc = check(cudaStreamWaitEvent(stream_, join_[k], 0), "join wait"))) return rc;
+  }
+  if (split_ > 1 && grad_len_ > 0) {
+    if ((rc = check(adj_reduce(parts, stream_), "gradient sum"))) return rc;
+    ++launches_;
   }
   return FGKL_OK;
 }

@@ -51,6 +51,7 @@ class AdjointEngine {
     int n_tasks;
     int blocks;
     size_t stride;
+    size_t scratch_off = 0;  // side by side: this bin's slice of the scratch
   };
   int fail(int code, const std::string& msg);
   int check(cudaError_t e, const char* what);
@@ -83,7 +84,15 @@ class AdjointEngine {
   size_t cap_scratch_ = 0;
   int32_t* tasks_ = nullptr;  // per bin, inside d_idx_
   int32_t* queue_ = nullptr;  // FP64 recomputation queue, inside d_idx_
-  int n_small_ = 0;
+  int n_small_ = 0;  // followed in d_small_ by a flag a read
+  static constexpr int kAux = 4;
+  cudaStream_t aux_[kAux] = {};  // side by side: the bins of a pass
+  cudaEvent_t fork_ = nullptr, join_[kAux] = {};
+  bool side_by_side_ = false;
+  int split_ = 1;    // parts that a read's haplotypes are shared among
+  int64_t n_reads_ = 0;
+  double* d_part_ = nullptr;  // gradients of the parts beyond the first, four arrays each
+  size_t cap_part_ = 0;
 };
 
 }  // namespace fgkl
