@@ -307,7 +307,6 @@ Engine::Engine(int device, cudaStream_t stream) : device_(device), stream_(strea
   cudaMalloc(&d_m2m_, sizeof(double) * t.m2m.size());
   cudaMemcpy(d_err_, t.error_prob.data(), sizeof(double) * t.error_prob.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(d_m2m_, t.m2m.data(), sizeof(double) * t.m2m.size(), cudaMemcpyHostToDevice);
-  cudaMalloc(&d_counters_, sizeof(Counters));
   for (int i = 0; i < kAuxStreams; ++i) {
     cudaStreamCreateWithFlags(&aux_[i], cudaStreamNonBlocking);
     cudaEventCreateWithFlags(&join_[i], cudaEventDisableTiming);
@@ -324,13 +323,9 @@ Engine::~Engine() {
   if (stream_) cudaStreamSynchronize(stream_);
   if (copy_) cudaStreamSynchronize(copy_);
   cudaFree(d_reads_);
-  cudaFree(d_read_off_);
-  cudaFree(d_plan_);
-  cudaFree(d_tasks_);
+  cudaFree(d_in_);
   cudaFree(d_queue_);
-  cudaFree(d_small_);
   cudaFree(d_out_);
-  cudaFree(d_counters_);
   cudaFree(d_scratch_);
   cudaFree(d_err_);
   cudaFree(d_m2m_);
@@ -596,10 +591,12 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   const uint8_t* const read_arrays[5] = {in.bases, in.quals, in.ins, in.del, in.gcp};
   bool direct_reads = read_bytes > 0;
   for (int a = 0; a < 5 && direct_reads; ++a) direct_reads = host_pinned(read_arrays[a], static_cast<size_t>(read_bytes));
-  if (!direct_reads && !grow_pinned(h_reads_, cap_h_reads_, static_cast<size_t>(read_bytes) * 5 + 16))
+  // A small call's reads travel with its plan, in one copy.
+  const bool reads_with_plan = !direct_reads && read_bytes <= (int64_t{1} << 18);
+  if (!direct_reads && !reads_with_plan && !grow_pinned(h_reads_, cap_h_reads_, static_cast<size_t>(read_bytes) * 5 + 16))
     return fail(FGKL_E_OUT_OF_MEMORY, "pinned host allocation failed");
-  Helper read_copy(!direct_reads && read_bytes >= (int64_t{8} << 20), [this, &read_arrays, read_bytes, direct_reads] {
-    if (direct_reads) return;
+  Helper read_copy(!direct_reads && read_bytes >= (int64_t{8} << 20), [this, &read_arrays, read_bytes, direct_reads, reads_with_plan] {
+    if (direct_reads || reads_with_plan) return;
     for (int a = 0; a < 5; ++a)
       if (read_bytes) parallel_copy(h_reads_ + static_cast<size_t>(a) * read_bytes, read_arrays[a], static_cast<size_t>(read_bytes));
   });
@@ -949,23 +946,21 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   section(static_cast<size_t>(n_pd_seq) * sizeof(uint32_t) + 16, o_pd_seq);
   section(static_cast<size_t>(n_sigs) * sizeof(uint32_t) + 16, o_sigs);
 
-  // Device buffers.
-  n_small_ = static_cast<int>(bins_.size() + rescue_bins_.size()) + 2 * kQueueBins + 1;
-  if (!grow(d_reads_, cap_reads_, static_cast<size_t>(read_bytes) * 5 + 16) ||
-      !grow(d_read_off_, cap_read_off_, static_cast<size_t>(total_reads) + 1) || !grow(d_plan_, cap_plan_, blob_bytes) ||
-      !grow(d_tasks_, cap_tasks_, tasks.size() + 1) || !grow(d_queue_, cap_queue_, static_cast<size_t>(queue_off[kQueueBins]) + 1) ||
-      !grow(d_small_, cap_small_, static_cast<size_t>(n_small_)) || !grow(d_out_, cap_out_, static_cast<size_t>(out_len_) + 1) ||
-      !grow(d_scratch_, cap_scratch_, scratch_total))
-    return fail(FGKL_E_OUT_OF_MEMORY, "device allocation failed");
-
-  // Pinned staging (the reads have their own buffer): read offsets | plan | tasks | queue offsets |
-  // results | counters.
+  // One upload: read offsets | plan | tasks | queue offsets | a small call's reads. The pinned staging holds
+  // it, and after it the results and counters that come back. On the device the results are followed by what
+  // every run zeroes: the counters, then a task counter for each launch and the queues' tails.
   const size_t s_read_off = 0;
   const size_t s_blob = s_read_off + align_up((total_reads + 1) * sizeof(int64_t));
   const size_t s_tasks = s_blob + align_up(blob_bytes);
   const size_t s_qoff = s_tasks + align_up(tasks.size() * sizeof(Task));
-  const size_t s_out = s_qoff + align_up((kQueueBins + 1) * sizeof(int));
-  const size_t stage_bytes = s_out + align_up(static_cast<size_t>(out_len_) * sizeof(double)) + align_up(sizeof(Counters));
+  const size_t s_reads = s_qoff + align_up((kQueueBins + 1) * sizeof(int));
+  const size_t s_out = s_reads + (reads_with_plan ? align_up(static_cast<size_t>(read_bytes) * 5) : 0);
+  const size_t stage_bytes = s_out + align_up(static_cast<size_t>(out_len_) * sizeof(double) + sizeof(Counters));
+  zero_bytes_ = sizeof(Counters) + (bins_.size() + rescue_bins_.size() + kQueueBins) * sizeof(int);
+  if ((!reads_with_plan && !grow(d_reads_, cap_reads_, static_cast<size_t>(read_bytes) * 5 + 16)) || !grow(d_in_, cap_in_, s_out + 16) ||
+      !grow(d_queue_, cap_queue_, static_cast<size_t>(queue_off[kQueueBins]) + 1) ||
+      !grow(d_out_, cap_out_, static_cast<size_t>(out_len_) + (zero_bytes_ + 7) / 8) || !grow(d_scratch_, cap_scratch_, scratch_total))
+    return fail(FGKL_E_OUT_OF_MEMORY, "device allocation failed");
   if (over_allocation_limit(stage_bytes)) return fail(FGKL_E_OUT_OF_MEMORY, "pinned host allocation failed");
   if (stage_bytes > cap_stage_) {
     // Grown by half again at least, as the device buffers are (cudaFreeHost waits for the device).
@@ -1024,25 +1019,18 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   }
   if (!tasks.empty()) std::memcpy(st + s_tasks, tasks.data(), tasks.size() * sizeof(Task));
   std::memcpy(st + s_qoff, queue_off.data(), (kQueueBins + 1) * sizeof(int));
+  if (reads_with_plan)
+    for (int a = 0; a < 5; ++a)
+      if (read_bytes) std::memcpy(st + s_reads + static_cast<size_t>(a) * read_bytes, read_arrays[a], static_cast<size_t>(read_bytes));
 
   read_copy.join();
   planned_.host_pack_ms = ms_since(t_pack);
   const auto t_up = std::chrono::steady_clock::now();
   int rc;
-  if (!direct_reads && (rc = check(cudaMemcpyAsync(d_reads_, h_reads_, static_cast<size_t>(read_bytes) * 5, cudaMemcpyHostToDevice, copy_),
-                                   "upload reads")))
+  if (!direct_reads && !reads_with_plan &&
+      (rc = check(cudaMemcpyAsync(d_reads_, h_reads_, static_cast<size_t>(read_bytes) * 5, cudaMemcpyHostToDevice, copy_), "upload reads")))
     return rc;
-  if ((rc = check(cudaMemcpyAsync(d_read_off_, st + s_read_off, (total_reads + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, copy_),
-                  "upload offsets")))
-    return rc;
-  if ((rc = check(cudaMemcpyAsync(d_plan_, st + s_blob, blob_bytes, cudaMemcpyHostToDevice, copy_), "upload plan"))) return rc;
-  if (!tasks.empty() &&
-      (rc = check(cudaMemcpyAsync(d_tasks_, st + s_tasks, tasks.size() * sizeof(Task), cudaMemcpyHostToDevice, copy_), "upload tasks")))
-    return rc;
-  if ((rc = check(cudaMemcpyAsync(d_small_ + (n_small_ - 2 * kQueueBins - 1), st + s_qoff, (kQueueBins + 1) * sizeof(int),
-                                  cudaMemcpyHostToDevice, copy_),
-                  "upload queue offsets")))
-    return rc;
+  if ((rc = check(cudaMemcpyAsync(d_in_, st, s_out, cudaMemcpyHostToDevice, copy_), "upload plan"))) return rc;
   if ((rc = check(cudaEventRecord(uploaded_, copy_), "upload event"))) return rc;
   // Uploaded from the caller's own memory: done before returning, so the caller may reuse it.
   if (direct_reads) {
@@ -1051,26 +1039,30 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   }
 
   planned_.host_upload_ms = ms_since(t_up);
-  view_.bases = d_reads_;
-  view_.quals = d_reads_ + read_bytes;
-  view_.ins = d_reads_ + 2 * read_bytes;
-  view_.del = d_reads_ + 3 * read_bytes;
-  view_.gcp = d_reads_ + 4 * read_bytes;
-  view_.read_off = d_read_off_;
-  view_.regions = reinterpret_cast<const Region*>(d_plan_ + o_regions);
-  view_.progs = reinterpret_cast<const Program*>(d_plan_ + o_progs);
-  view_.haps = reinterpret_cast<const HapInfo*>(d_plan_ + o_haps);
-  view_.stream = reinterpret_cast<const uint32_t*>(d_plan_ + o_stream);
-  view_.segs = reinterpret_cast<const Segment*>(d_plan_ + o_segs);
-  view_.sweeps = reinterpret_cast<const Sweep*>(d_plan_ + o_sweeps);
-  view_.code_of_byte = d_plan_ + o_codes;
-  view_.hap_codes = d_plan_ + o_seq;
-  view_.pd_entries = reinterpret_cast<const uint32_t*>(d_plan_ + o_pd_seq);
-  view_.pd_sigs = reinterpret_cast<const uint32_t*>(d_plan_ + o_sigs);
+  const uint8_t* const reads = reads_with_plan ? d_in_ + s_reads : d_reads_;
+  const uint8_t* const plan = d_in_ + s_blob;
+  tasks_ = reinterpret_cast<const Task*>(d_in_ + s_tasks);
+  queue_off_ = reinterpret_cast<const int*>(d_in_ + s_qoff);
+  view_.bases = reads;
+  view_.quals = reads + read_bytes;
+  view_.ins = reads + 2 * read_bytes;
+  view_.del = reads + 3 * read_bytes;
+  view_.gcp = reads + 4 * read_bytes;
+  view_.read_off = reinterpret_cast<const int64_t*>(d_in_ + s_read_off);
+  view_.regions = reinterpret_cast<const Region*>(plan + o_regions);
+  view_.progs = reinterpret_cast<const Program*>(plan + o_progs);
+  view_.haps = reinterpret_cast<const HapInfo*>(plan + o_haps);
+  view_.stream = reinterpret_cast<const uint32_t*>(plan + o_stream);
+  view_.segs = reinterpret_cast<const Segment*>(plan + o_segs);
+  view_.sweeps = reinterpret_cast<const Sweep*>(plan + o_sweeps);
+  view_.code_of_byte = plan + o_codes;
+  view_.hap_codes = plan + o_seq;
+  view_.pd_entries = reinterpret_cast<const uint32_t*>(plan + o_pd_seq);
+  view_.pd_sigs = reinterpret_cast<const uint32_t*>(plan + o_sigs);
   view_.err_prob = d_err_;
   view_.m2m = d_m2m_;
   view_.out = d_out_;
-  view_.counters = d_counters_;
+  view_.counters = reinterpret_cast<Counters*>(d_out_ + out_len_);
   (void)total_haps;
   return FGKL_OK;
 }
@@ -1088,13 +1080,10 @@ int Engine::end_run() {
 int Engine::run() {
   DeviceGuard device_guard(device_);
   int rc;
-  int* counters = d_small_;                                // one per launch
-  int* queue_off = d_small_ + (n_small_ - 2 * kQueueBins - 1);  // kQueueBins + 1 entries, uploaded by prepare
-  int* queue_tail = d_small_ + (n_small_ - kQueueBins);
   const size_t n_launch = bins_.size() + rescue_bins_.size();
-  if ((rc = check(cudaMemsetAsync(counters, 0, n_launch * sizeof(int), stream_), "reset task counters"))) return rc;
-  if ((rc = check(cudaMemsetAsync(queue_tail, 0, kQueueBins * sizeof(int), stream_), "reset queues"))) return rc;
-  if ((rc = check(cudaMemsetAsync(d_counters_, 0, sizeof(Counters), stream_), "reset counters"))) return rc;
+  int* counters = reinterpret_cast<int*>(view_.counters + 1);  // one per launch
+  int* queue_tail = counters + n_launch;
+  if ((rc = check(cudaMemsetAsync(view_.counters, 0, zero_bytes_, stream_), "reset counters"))) return rc;
   planned_.kernel_launches = 0;
   int i = 0;
   if (profile_) {
@@ -1108,16 +1097,18 @@ int Engine::run() {
   // Each pass forks its bins onto the auxiliary streams and joins them back.
   auto pass = [&](const std::vector<Bin>& list, bool rescue) -> int {
     if (list.empty()) return FGKL_OK;
-    if ((rc = check(cudaEventRecord(fork_, stream_), "fork"))) return rc;
+    // A pass of one launch stays on the main stream.
+    const bool fork = !profile_ && list.size() > 1;
+    if (fork && (rc = check(cudaEventRecord(fork_, stream_), "fork"))) return rc;
     for (size_t b = 0; b < list.size(); ++b) {
       const Bin& bin = list[b];
       // Profiled runs serialise the launches on the main stream so each one's events time it alone.
       const int lanes = std::max(1, std::min(tuning_.streams, kAuxStreams));
-      cudaStream_t s = profile_ ? stream_ : aux_[b % lanes];
-      if ((rc = check(cudaStreamWaitEvent(s, fork_, 0), "fork wait"))) return rc;
+      cudaStream_t s = fork ? aux_[b % lanes] : stream_;
+      if (fork && (rc = check(cudaStreamWaitEvent(s, fork_, 0), "fork wait"))) return rc;
       LaunchArgs a{};
       a.v = view_;
-      a.tasks = (rescue ? d_queue_ : d_tasks_) + bin.task_off;
+      a.tasks = (rescue ? d_queue_ : tasks_) + bin.task_off;
       a.n_tasks = bin.n_tasks;
       a.count = rescue ? queue_tail + bin.queue_bin : nullptr;
       a.task_counter = counters + i++;
@@ -1131,8 +1122,9 @@ int Engine::run() {
         return rc;
       if (profile_ && (rc = check(cudaEventRecord(ev_[2 * li + 1], s), "profiling event"))) return rc;
       planned_.kernel_launches++;
-      if ((rc = check(cudaEventRecord(join_[b % lanes], s), "join"))) return rc;
+      if (fork && (rc = check(cudaEventRecord(join_[b % lanes], s), "join"))) return rc;
     }
+    if (!fork) return FGKL_OK;
     const size_t used = std::min<size_t>(list.size(), static_cast<size_t>(std::max(1, std::min(tuning_.streams, kAuxStreams))));
     for (size_t b = 0; b < used; ++b)
       if ((rc = check(cudaStreamWaitEvent(stream_, join_[b], 0), "join wait"))) return rc;
@@ -1140,7 +1132,7 @@ int Engine::run() {
   };
   if ((rc = pass(bins_, false))) return rc;
   if (!rescue_bins_.empty()) {
-    CollectArgs c{view_, d_queue_, queue_off, queue_tail, cfg_.double_precision ? 0 : 1};
+    CollectArgs c{view_, d_queue_, queue_off_, queue_tail, cfg_.double_precision ? 0 : 1};
     if ((rc = check(launch_collect(c, n_regions_, stream_), "lost-pair collection"))) return rc;
     planned_.kernel_launches++;
   }
@@ -1207,16 +1199,19 @@ int Engine::fetch(double* out, int64_t out_len, BatchStats* stats) {
                                           std::to_string(out_len_));
   int rc;
   double* h_out = reinterpret_cast<double*>(h_stage_ + out_stage_);
-  Counters* h_cnt = reinterpret_cast<Counters*>(h_stage_ + out_stage_ + align_up(static_cast<size_t>(out_len_) * sizeof(double)));
+  Counters* h_cnt = reinterpret_cast<Counters*>(h_out + out_len_);
   if ((rc = check(cudaStreamWaitEvent(copy_, computed_, 0), "wait for the kernels"))) return rc;
   // Results go straight into a page-locked output array, else through pinned staging.
   const size_t out_bytes = static_cast<size_t>(out_len_) * sizeof(double);
   const bool direct_out = out_len_ > 0 && host_pinned(out, out_bytes);
-  if (out_len_ > 0 &&
-      (rc = check(cudaMemcpyAsync(direct_out ? out : h_out, d_out_, out_bytes, cudaMemcpyDeviceToHost, copy_), "download results")))
+  // The counters follow the results on the device and in the staging.
+  if (direct_out) {
+    if ((rc = check(cudaMemcpyAsync(out, d_out_, out_bytes, cudaMemcpyDeviceToHost, copy_), "download results")) ||
+        (rc = check(cudaMemcpyAsync(h_cnt, view_.counters, sizeof(Counters), cudaMemcpyDeviceToHost, copy_), "download counters")))
+      return rc;
+  } else if ((rc = check(cudaMemcpyAsync(h_out, d_out_, out_bytes + sizeof(Counters), cudaMemcpyDeviceToHost, copy_), "download results"))) {
     return rc;
-  if ((rc = check(cudaMemcpyAsync(h_cnt, d_counters_, sizeof(Counters), cudaMemcpyDeviceToHost, copy_), "download counters")))
-    return rc;
+  }
   if ((rc = check(cudaEventRecord(fetched_, copy_), "download event"))) return rc;
   if ((rc = check(cudaEventSynchronize(fetched_), "kernel execution"))) return rc;
   if (out_len_ > 0 && !direct_out) parallel_copy(reinterpret_cast<uint8_t*>(out), reinterpret_cast<const uint8_t*>(h_out), out_bytes);

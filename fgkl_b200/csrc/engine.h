@@ -201,19 +201,12 @@ class Engine {
   // Device buffers (grow-only).
   uint8_t* d_reads_ = nullptr;
   size_t cap_reads_ = 0;
-  int64_t* d_read_off_ = nullptr;
-  size_t cap_read_off_ = 0;
-  uint8_t* d_plan_ = nullptr;  // regions, haps, stream, segs, slot/node lists, code tables
-  size_t cap_plan_ = 0;
-  Task* d_tasks_ = nullptr;
-  size_t cap_tasks_ = 0;
+  uint8_t* d_in_ = nullptr;  // read offsets | plan | tasks | queue offsets | a small call's reads
+  size_t cap_in_ = 0;
   Task* d_queue_ = nullptr;
   size_t cap_queue_ = 0;
-  int* d_small_ = nullptr;  // task counters, queue offsets and tails
-  size_t cap_small_ = 0;
-  double* d_out_ = nullptr;
+  double* d_out_ = nullptr;  // results, then Counters, the launches' task counters and the queues' tails
   size_t cap_out_ = 0;
-  Counters* d_counters_ = nullptr;
   char* d_scratch_ = nullptr;
   size_t cap_scratch_ = 0;
   double* d_err_ = nullptr;
@@ -233,7 +226,9 @@ class Engine {
   int n_regions_ = 0;
   bool profile_ = false;
   std::vector<cudaEvent_t> ev_;  // begin/end per launch of the last profiled run
-  int n_small_ = 0;
+  const Task* tasks_ = nullptr;     // of the prepared batch, in d_in_
+  const int* queue_off_ = nullptr;  // kQueueBins + 1 entries, in d_in_
+  size_t zero_bytes_ = 0;           // what a run zeroes from the counters on
 };
 
 }  // namespace fgkl
