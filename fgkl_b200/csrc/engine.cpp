@@ -361,7 +361,8 @@ T* Engine::grow(T*& ptr, size_t& cap, size_t n) {
   if (bytes > cap) {
     // Half as much again as the old size: a caller whose batches vary in size stops reallocating
     // after a few calls (cudaFree waits for the whole device, other callers' streams included).
-    const size_t want = cap > 0 ? std::max(bytes, cap + cap / 2) : bytes;
+    // The first size gets an eighth more, so that the next batches of its kind fit.
+    const size_t want = cap > 0 ? std::max(bytes, cap + cap / 2) : bytes + bytes / 8;
     cudaFree(ptr);
     ptr = nullptr;
     if (device_alloc(reinterpret_cast<void**>(&ptr), want) == cudaSuccess) {

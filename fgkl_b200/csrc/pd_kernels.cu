@@ -354,17 +354,19 @@ __device__ __forceinline__ void pd_forward_pass(const LaunchArgs& a, const Progr
     };
     int t = 0;
     for (; t < G; ++t) at(t);
-    // Every lane strictly inside the haplotype: no events. The next entry and its signature are loaded a
-    // step ahead.
+    // Every lane strictly inside the haplotype: no events. An entry is loaded two steps ahead and its
+    // signature one, so neither load waits on the other.
     const uint32_t* seq = synth_seq - gl;
     if (t < n) {
-      uint32_t e = __ldg(seq + t), g = __ldg(sigs + (e & kCodeMask));
+      auto entry = [&](int i) { return i < n ? __ldg(seq + i) : 0u; };
+      uint32_t e0 = entry(t), e1 = entry(t + 1), g0 = __ldg(sigs + (e0 & kCodeMask));
 #pragma unroll 2
       for (; t < n; ++t) {
-        const uint32_t e1 = t + 1 < n ? __ldg(seq + t + 1) : 0u, g1 = __ldg(sigs + (e1 & kCodeMask));
-        pd_step<P, R, G, false>(a, prog, rd, lane, pr, an, sc, st, synth_len, e, g);
-        e = e1;
-        g = g1;
+        const uint32_t e2 = entry(t + 2), g1 = __ldg(sigs + (e1 & kCodeMask));
+        pd_step<P, R, G, false>(a, prog, rd, lane, pr, an, sc, st, synth_len, e0, g0);
+        e0 = e1;
+        e1 = e2;
+        g0 = g1;
       }
     }
     for (; t < n + G; ++t) at(t);
@@ -521,11 +523,17 @@ __device__ __forceinline__ void pd_long_superstep(const LaunchArgs& a, const Rea
                                                   const uint32_t* sigs, int n, int t0, const Carry<P>* in, Carry<P>* out,
                                                   int out_mask) {
   const Program prog{};
+  // An entry is loaded two steps ahead and its signature one.
+  auto entry = [&](int i) { return kInner ? (i < kChunk ? __ldg(seq + t0 + i - lane) : 0u) : pd_synth_entry(seq, n, t0 + i - lane); };
+  auto signature = [&](uint32_t e) { return kGeneric ? 0u : __ldg(sigs + (e & kCodeMask)); };
+  uint32_t e0 = entry(0), e1 = entry(1), g0 = signature(e0);
 #pragma unroll 2
   for (int i = 0; i < kChunk; ++i) {
     const int t = t0 + i;
-    const uint32_t e = kInner ? __ldg(seq + t - lane) : pd_synth_entry(seq, n, t - lane);
-    const uint32_t sig = kGeneric ? 0u : __ldg(sigs + (e & kCodeMask));
+    const uint32_t e = e0, sig = g0;
+    e0 = e1;
+    g0 = signature(e0);
+    e1 = entry(i + 2);
     const Carry<P> c = in[t & (kRing - 1)];
     st.cX = c.x;
     st.cT = c.t;
