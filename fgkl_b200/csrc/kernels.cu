@@ -476,6 +476,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratch
 static __device__ double g_noalloc_err[kMaxQualTable];
 static __device__ double g_noalloc_m2m[kM2MTable];
 static __device__ uint8_t g_noalloc_codes[256];
+static __device__ uint8_t g_noalloc_acgt[256];  // read byte -> acgtn_code, kNoCode for the others
 
 struct NoAllocArgs {
   BatchView v;  // read arrays and offsets, tables, read byte -> code table
@@ -492,40 +493,51 @@ struct NoAllocArgs {
 // same permutation, so a read base matches exactly the haplotype bytes equal to it.
 __device__ __forceinline__ uint32_t byte_code(uint32_t b) { return b == 'N' ? kCodeN : (b == kCodeN ? 'N' : b); }
 
-__device__ __forceinline__ uint32_t byte_entry(const uint8_t* hap, int len, int p) {
-  if (p < 0 || p > len) return 0u;
-  uint32_t e = p < len ? byte_code(__ldg(hap + p)) : 0u;
-  if (p == 0) e |= EV_BEGIN;
-  if (p == len) e |= EV_END;
-  return e;
-}
+// Prior codes of the bytes A, C, T, G and N for the table form: 0 to 3 by two bits of the letter, N as
+// kCodeN.
+__device__ __forceinline__ uint32_t acgtn_code(uint32_t b) { return b == 'N' ? kCodeN : (b >> 1) & 3u; }
+__device__ __forceinline__ bool is_acgtn(uint32_t b) { return b == 'A' || b == 'C' || b == 'G' || b == 'T' || b == 'N'; }
 
-template <int R>
-__device__ void forward_unshared(const LaunchArgs& a, const ReadRef* rd, int lane, Scratch<OneF64, R>& sc, const uint8_t* hap,
-                                 int n) {
-  using P = OneF64;
-  using V = typename P::V;
+// One unshared sweep: P is OneF64Table for a haplotype of A, C, G, T and N only (priors from the warp's
+// table, read codes from g_noalloc_acgt), else OneF64 (priors by comparing bytes).
+template <class P, int R>
+__device__ __forceinline__ void forward_unshared(const LaunchArgs& a, const ReadRef* rd, int lane, char* scratch, double* priors,
+                                                 const uint8_t* hap, int n) {
+  auto code = [](uint32_t b) { return P::kTable ? acgtn_code(b) : byte_code(b); };
+  auto entry = [&](int p) -> uint32_t {
+    if (p < 0 || p > n) return 0u;
+    return (p < n ? code(__ldg(hap + p)) : 0u) | (p == 0 ? EV_BEGIN : 0u) | (p == n ? EV_END : 0u);
+  };
+  Scratch<P, R> sc(scratch, nullptr, 0, 0, 0);
+  sc.priors = priors;
   FwdRows<P, R, 32> fr;
-  fr.load(a.v, rd, lane, a.v.code_of_byte, sc.priors);
-  const V an = 1.0;  // the plain recurrence: the result is the sum of the last row's M and X
+  fr.load(a.v, rd, lane, P::kTable ? g_noalloc_acgt : a.v.code_of_byte, sc.priors);
+  __syncwarp();
+  const double an = 1.0;  // the plain recurrence: the result is the sum of the last row's M and X
   FwdState<P, R> st;
   st.clear();
   const Program prog{};  // unused: the stream is synthesised from the haplotype bytes
   int t = 0;
-  for (; t < 32; ++t) forward_step<P, R, 32>(a, prog, rd, lane, fr, an, sc, st, n, byte_entry(hap, n, t - lane));
+  for (; t < 32; ++t) forward_step<P, R, 32>(a, prog, rd, lane, fr, an, sc, st, n, entry(t - lane));
   // Every lane strictly inside the haplotype: no events.
   const uint8_t* seq = hap - lane;
   for (; t + 4 <= n; t += 4) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) forward_step<P, R, 32, false>(a, prog, rd, lane, fr, an, sc, st, n, byte_code(__ldg(seq + t + i)));
+    for (int i = 0; i < 4; ++i) forward_step<P, R, 32, false>(a, prog, rd, lane, fr, an, sc, st, n, code(__ldg(seq + t + i)));
   }
-  for (; t < n + 32; ++t) forward_step<P, R, 32>(a, prog, rd, lane, fr, an, sc, st, n, byte_entry(hap, n, t - lane));
+  for (; t < n + 32; ++t) forward_step<P, R, 32>(a, prog, rd, lane, fr, an, sc, st, n, entry(t - lane));
+  __syncwarp();
+}
+
+template <int R>
+constexpr size_t noalloc_smem_per_warp() {
+  using L = Layout<OneF64Table, R>;
+  return static_cast<size_t>(L::kPriorCodes) * L::kRp * 32 * sizeof(double);
 }
 
 template <int R>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, f64_min_blocks(R, false)) noalloc_kernel(NoAllocArgs na) {
-  using P = OneF64;
-  extern __shared__ __align__(16) unsigned char smem_raw[];  // none requested: nothing is staged
+  extern __shared__ __align__(16) unsigned char smem_raw[];  // a prior table a warp
   const int lane = threadIdx.x & 31;
   const int warp = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   LaunchArgs a{};
@@ -548,24 +560,34 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, f64_min_blocks(R, false))
     }
     rd[0].len = static_cast<int>(read_len);
     rd[0].pad = 32 * R - rd[0].len;
-    Scratch<P, R> sc(na.scratch + static_cast<size_t>(warp) * kNoAllocPerWarp, reinterpret_cast<double*>(smem_raw), 0, 0, 0);
-    forward_unshared<R>(a, rd, lane, sc, na.hap_bases + hap_lo, static_cast<int>(hap_len));
-    __syncwarp();
-    if (lane == 0) na.out[t] = log10(sc.raw(0, 0)) - Consts<true>::kLog10Initial;
+    char* const scratch = na.scratch + static_cast<size_t>(warp) * kNoAllocPerWarp;
+    double* const priors = reinterpret_cast<double*>(smem_raw + (threadIdx.x >> 5) * noalloc_smem_per_warp<R>());
+    const uint8_t* const hap = na.hap_bases + hap_lo;
+    const int n = static_cast<int>(hap_len);
+    bool plain = true;
+    for (int i = lane; i < n; i += 32) plain &= is_acgtn(__ldg(hap + i));
+    if (__all_sync(kFull, plain))
+      forward_unshared<OneF64Table, R>(a, rd, lane, scratch, priors, hap, n);
+    else
+      forward_unshared<OneF64, R>(a, rd, lane, scratch, priors, hap, n);
+    if (lane == 0) na.out[t] = log10(*reinterpret_cast<const double*>(scratch)) - Consts<true>::kLog10Initial;
     __syncwarp();
   }
 }
 
 template <int R>
 cudaError_t noalloc_go(int blocks, const NoAllocArgs& na, cudaStream_t s) {
-  noalloc_kernel<R><<<blocks, kWarpsPerBlock * 32, 0, s>>>(na);
+  noalloc_kernel<R><<<blocks, kWarpsPerBlock * 32, kWarpsPerBlock * noalloc_smem_per_warp<R>(), s>>>(na);
   return cudaGetLastError();
 }
 
 template <int R>
 int noalloc_occupancy() {
   int b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, noalloc_kernel<R>, kWarpsPerBlock * 32, 0) != cudaSuccess) return 0;
+  constexpr size_t smem = kWarpsPerBlock * noalloc_smem_per_warp<R>();
+  if (cudaFuncSetAttribute(noalloc_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, noalloc_kernel<R>, kWarpsPerBlock * 32, smem) != cudaSuccess)
+    return 0;
   return b;
 }
 
@@ -612,6 +634,10 @@ cudaError_t noalloc_setup(NoAllocDevice* d, const double* err, size_t n_err, con
   if ((e = cudaMemcpyToSymbol(g_noalloc_err, err, n_err * sizeof(double))) != cudaSuccess) return e;
   if ((e = cudaMemcpyToSymbol(g_noalloc_m2m, m2m, n_m2m * sizeof(double))) != cudaSuccess) return e;
   if ((e = cudaMemcpyToSymbol(g_noalloc_codes, codes, 256)) != cudaSuccess) return e;
+  uint8_t acgt[256];
+  for (uint8_t& c : acgt) c = kNoCode;
+  for (const char b : {'A', 'C', 'T', 'G'}) acgt[static_cast<uint8_t>(b)] = static_cast<uint8_t>((b >> 1) & 3);
+  if ((e = cudaMemcpyToSymbol(g_noalloc_acgt, acgt, 256)) != cudaSuccess) return e;
   for (int rows = 1; rows <= 20; ++rows) {
     if (rows > 8 && rows % 2) continue;
     d->blocks_per_sm[rows] = noalloc_dispatch(rows, [](auto r) { return noalloc_occupancy<decltype(r)::value>(); });
