@@ -44,6 +44,12 @@ size_t sw_scratch_bytes(int rows, int64_t ref_len, int64_t alt_len);
 bool sw_tagged(int64_t longest, int match, int mismatch, int open, int extend);
 void sw_occupancy(int rows, bool tagged, int* blocks_per_sm, int* threads_per_block);
 cudaError_t sw_launch(int rows, int blocks, const SwArgs& a, cudaStream_t stream);
+// The pipelined form: a pair's row blocks on `warps` warps of a block (sw_pipe_warps of the longest
+// reference), one pair and one scratch of sw_pipe_scratch_bytes a block.
+int sw_pipe_warps(int64_t longest_ref);
+size_t sw_pipe_scratch_bytes(int64_t ref_len, int64_t alt_len);
+void sw_pipe_occupancy(bool tagged, int warps, int* blocks_per_sm);
+cudaError_t sw_pipe_launch(int warps, int blocks, const SwArgs& a, cudaStream_t stream);
 // Packs the pairs' CIGAR elements, pair after pair, into `packed` (as many elements as the counts
 // sum to), after sw_launch on the same stream.
 cudaError_t sw_compact(const uint32_t* cigar, const int64_t* slot, const int32_t* count, int n_pairs, uint32_t* packed,

@@ -12,6 +12,11 @@ namespace fgkl {
 namespace {
 constexpr int kWarps = 4;                           // warps per block of the kernel
 constexpr size_t kScratchBudget = size_t{8} << 30;  // per-warp traceback scratch of one launch
+// Warps an SM up to which a pair's row blocks run on several warps (sw_pipe_kernel) instead of one. One pair
+// of 500 x 500 bases takes 157 us against 248 so, 128 pairs 159 against 255, and 9 pairs of 1266 x 1172 0.68
+// ms against 1.62; with the SMs' schedulers filled (512 pairs of 500 bases, 14 warps an SM) the shorter rows
+// only cost: 270 against 263 us, and 470 against 347 at 1024 pairs.
+constexpr int64_t kPipeWarpsPerSm = 12;
 
 // Rows per lane of a batch: what makes its steps cheapest, a step costing its rows and kStepRows more, and a
 // pair ceil(n / 32 rows) (m + 31) steps. 16,384 pairs of 500 x 500 bases take 4.37 ms at 4 rows, 4.43 at 8
@@ -121,9 +126,16 @@ int SwEngine::align(const SwBatch& in, const SwScores& s, int strategy, uint32_t
   if (cigar_len < slot[P])
     return fail(FGKL_E_OUTPUT_LENGTH, "the CIGAR array holds " + std::to_string(cigar_len) + " elements; the batch needs " +
                                           std::to_string(slot[P]));
+  // Few pairs: several warps each (sw_pipe_kernel).
+  int64_t longest_ref = 0;
+  for (int64_t k = 0; k < P; ++k) longest_ref = std::max(longest_ref, in.ref_off[k + 1] - in.ref_off[k]);
+  const int pipe_warps = sw_pipe_warps(longest_ref);
+  const bool pipelined = pipe_warps > 1 && P * pipe_warps <= kPipeWarpsPerSm * sms_;
   const int rows = choose_rows(in);
-  for (int64_t k = 0; k < P; ++k)
-    stride = std::max(stride, sw_scratch_bytes(rows, in.ref_off[k + 1] - in.ref_off[k], in.alt_off[k + 1] - in.alt_off[k]));
+  for (int64_t k = 0; k < P; ++k) {
+    const int64_t n = in.ref_off[k + 1] - in.ref_off[k], m = in.alt_off[k + 1] - in.alt_off[k];
+    stride = std::max(stride, pipelined ? sw_pipe_scratch_bytes(n, m) : sw_scratch_bytes(rows, n, m));
+  }
   std::stable_sort(cost.begin(), cost.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
   std::vector<int32_t> order(static_cast<size_t>(P));
   for (int64_t k = 0; k < P; ++k) order[k] = cost[k].second;
@@ -131,15 +143,19 @@ int SwEngine::align(const SwBatch& in, const SwScores& s, int strategy, uint32_t
 
   const bool tagged = sw_tagged(longest, s.match, s.mismatch, s.open, s.extend);
   int per_sm = 0, threads = 0;
-  sw_occupancy(rows, tagged, &per_sm, &threads);
+  if (pipelined)
+    sw_pipe_occupancy(tagged, pipe_warps, &per_sm);
+  else
+    sw_occupancy(rows, tagged, &per_sm, &threads);
   if (per_sm <= 0) return fail(FGKL_E_CUDA, "Smith-Waterman kernel unavailable on this device");
-  int64_t blocks = std::min<int64_t>((P + kWarps - 1) / kWarps, static_cast<int64_t>(per_sm) * sms_);
-  blocks = std::max<int64_t>(1, std::min<int64_t>(blocks, static_cast<int64_t>(kScratchBudget / (kWarps * stride))));
+  const int scratches = pipelined ? 1 : kWarps;  // a block
+  int64_t blocks = std::min<int64_t>((P + scratches - 1) / scratches, static_cast<int64_t>(per_sm) * sms_);
+  blocks = std::max<int64_t>(1, std::min<int64_t>(blocks, static_cast<int64_t>(kScratchBudget / (scratches * stride))));
 
   const int64_t ref_bytes = in.ref_off[P], alt_bytes = in.alt_off[P];
   if (!grow(d_seq_, cap_seq_, static_cast<size_t>(ref_bytes + alt_bytes) + 16) || !grow(d_idx_, cap_idx_, 3 * static_cast<size_t>(P + 1)) ||
       !grow(d_small_, cap_small_, 3 * static_cast<size_t>(P) + 1) || !grow(d_cigar_, cap_cigar_, 2 * static_cast<size_t>(slot[P])) ||
-      !grow(d_scratch_, cap_scratch_, static_cast<size_t>(blocks) * kWarps * stride))
+      !grow(d_scratch_, cap_scratch_, static_cast<size_t>(blocks) * scratches * stride))
     return fail(FGKL_E_OUT_OF_MEMORY, "device allocation failed");
   int rc;
   auto up = [&](void* dst, const void* src, size_t bytes, const char* what) {
@@ -186,7 +202,8 @@ int SwEngine::align(const SwBatch& in, const SwScores& s, int strategy, uint32_t
     if (!ev_[0] || !ev_[1]) return fail(FGKL_E_CUDA, "event creation failed");
   }
   if ((rc = check(cudaEventRecord(ev_[0], stream_), "event")) ||
-      (rc = check(sw_launch(rows, static_cast<int>(blocks), a, stream_), "Smith-Waterman launch")) ||
+      (rc = check(pipelined ? sw_pipe_launch(pipe_warps, static_cast<int>(blocks), a, stream_) : sw_launch(rows, static_cast<int>(blocks), a, stream_),
+                  "Smith-Waterman launch")) ||
       (rc = check(cudaEventRecord(ev_[1], stream_), "event")))
     return rc;
   // Only the elements produced cross to the host: packed pair after pair on the device, then
