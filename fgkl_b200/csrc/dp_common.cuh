@@ -259,10 +259,10 @@ __host__ __device__ constexpr size_t long_scratch_size(int max_hap_len) {
 }
 
 // Columns a superstep, and the supersteps a warp starts behind the one above it: at superstep s a warp
-// reads columns up to (s - w kDelay) kChunk - 1 - (kDelay - 1) kChunk + ... of its ring, of which the warp
-// above has written (s - w kDelay + kDelay) kChunk - 32 by the barrier before, so
-// kDelay * kChunk >= kChunk + 31. What that warp writes meanwhile lies behind those columns and at most
-// kDelay * kChunk + kChunk - 32 ahead of the oldest one, so a ring of kRing entries holds both.
+// reads columns t0 .. t0 + kChunk - 1 of its ring, t0 = (s - w kDelay) kChunk. The warp above, whose lane 31
+// is 31 columns behind its lane 0, had written up to t0 + kDelay kChunk - 32 by the barrier before, so
+// kDelay kChunk >= kChunk + 31. Meanwhile it writes the kChunk columns after those, at most
+// (kDelay + 1) kChunk - 32 past t0, so a ring of kRing entries holds both.
 constexpr int kChunk = 32, kDelay = 2, kRing = 128;
 static_assert(kDelay * kChunk >= kChunk + 31 && kRing >= (kDelay + 1) * kChunk, "ring");
 

@@ -10,7 +10,7 @@ namespace fgkl {
 enum class Kind : int {
   kShortF32 = 0,   // one read of at most 248 bases, FP32, rows-per-lane 1..8
   kOneF32 = 1,     // one read, FP32, rows-per-lane 10..20 (even)
-  kOneF64 = 2,     // one read, FP64, rows-per-lane 1..8 and 10..20 (even)
+  kOneF64 = 2,     // one read, FP64, priors from a table, rows-per-lane 1..8 and 10..20 (even)
   kOneF32Pd = 3,   // PD-HMM, one read, FP32, rows-per-lane 1..8 and 10..20 (even)
   kOneF64Pd = 4,   // PD-HMM, one read, FP64, same rows
   kPackedF32Pd = 5,  // PD-HMM, two reads per lane set in FP32x2, rows-per-lane 1..8

@@ -115,7 +115,7 @@ struct FwdRows {
   V k0[R], k1[R], k2[R], k3[R], k4[R], k5[R], k6[R];
   V pm[R], px[R];
   int oc[P::NC][R];
-  const V* table;  // prior table (FP32 kernels)
+  const V* table;  // prior table (policies with kTable)
 
   __device__ V prior(int code, bool isN, int r) const {
     const bool m0 = (code == oc[0][r]) | isN;
@@ -175,7 +175,7 @@ struct BwdRows {
   using S = typename P::S;
   V md[R], dd[R], mm[R], im[R], mi[R], ii[R], pm[R], px[R];
   int oc[P::NC][R];
-  const V* table;  // prior table of the rows below (FP32 kernels)
+  const V* table;  // prior table of the rows below (policies with kTable)
 
   __device__ V prior(int code, bool isN, int r, int lane) const {
     if (Layout<P, R>::kPriorCodes) return table[Layout<P, R>::prior_at(code, r, lane)];
