@@ -519,9 +519,12 @@ Engine::SplitRule Engine::choose_split(const BatchInput& in, const EngineConfig&
   int reads_per_warp = 1;
   if (pd && !cfg.double_precision) {
     if (tuning_.reads_per_warp == 2 && reads_steps / 2 >= kFullSteps * warps) reads_per_warp = rule.pd_reads = 2;
-  } else if (!cfg.double_precision && reads_steps / kQuadReads >= kFullSteps * warps) {
-    rule.quads = true;
-    reads_per_warp = kQuadReads;
+  } else if (!pd) {
+    double reads = 0;
+    for (const Work& w : work) reads += w.tasks;
+    const int most = cfg.double_precision ? 2 : kQuadReads;
+    rule.quads = reads_steps / most >= kFullSteps * warps && (!cfg.double_precision || reads / 2 >= kPairTasks * warps);
+    if (rule.quads) reads_per_warp = most;
   }
   for (Work& w : work) w.tasks = std::ceil(w.tasks / reads_per_warp);
   double total = 0, best = -1;
@@ -760,14 +763,14 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       const int32_t b = i + 1 < order.size() ? static_cast<int32_t>(first_read[g] + order[i + 1]) : -1;
       out.push_back({kind, rows, len_of(order[i]) + (i + 1 < order.size() ? len_of(order[i + 1]) : 0), Task{g, {a, b, -1, -1}, rows, -1, 0}, 0});
     };
-    auto four = [&](size_t i) {
+    auto quad = [&](Kind kind, size_t i, size_t reads) {
       Task t{g, {-1, -1, -1, -1}, quad_rows(len_of(order[i])), -1, 0};
       int len = 0;
-      for (size_t k = 0; k < kQuadReads && i + k < order.size(); ++k) {
+      for (size_t k = 0; k < reads && i + k < order.size(); ++k) {
         t.read[k] = static_cast<int32_t>(first_read[g] + order[i + k]);
         len += len_of(order[i + k]);
       }
-      out.push_back({Kind::kQuadF32, t.rows, len, t, 0});
+      out.push_back({kind, t.rows, len, t, 0});
     };
     // One task per distinct sorted haplotype of read order[i], strip-mined over row blocks.
     const RegionPlan& rp = plans[g];
@@ -798,7 +801,9 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
         one(Kind::kOneF32Pd, single_rows(len_of(order[i])), i);
       for (; i < order.size(); i += 2) two(Kind::kPackedF32Pd, packed_rows(len_of(order[i])), i);
     } else if (cfg.double_precision || plans[g].extra_codes) {
-      for (; i < order.size(); ++i) one(f64, single_rows(len_of(order[i])), i);
+      const bool pairs_fit = cfg.double_precision && split.quads && !extra_codes;
+      for (; i < order.size() && !(pairs_fit && len_of(order[i]) <= kQuadMaxRead); ++i) one(f64, single_rows(len_of(order[i])), i);
+      for (; i < order.size(); i += 2) quad(Kind::kPairF64, i, 2);
     } else {
       // The tile-shape axis: rows_extra moves each read to the next instantiated rows-per-lane
       // (more padding rows, other registers and occupancy; the same bits).
@@ -807,7 +812,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       auto short_up = [&](int rows) { return up && rows < 8 ? rows + 1 : rows; };
       for (; i < order.size() && packed_rows(len_of(order[i])) > 8; ++i) one(Kind::kOneF32, single_up(single_rows(len_of(order[i]))), i);
       for (; i < order.size() && (!split.quads || len_of(order[i]) > kQuadMaxRead); ++i) one(Kind::kShortF32, short_up(packed_rows(len_of(order[i]))), i);
-      for (; i < order.size(); i += kQuadReads) four(i);
+      for (; i < order.size(); i += kQuadReads) quad(Kind::kQuadF32, i, kQuadReads);
     }
   });
   {

@@ -165,7 +165,7 @@ class Engine {
   };
   // The first pass's forms, and the steps above which a region's program is split.
   struct SplitRule {
-    bool quads = false;         // plain FP32 reads of at most kQuadMaxRead bases go kQuadReads to a warp
+    bool quads = false;         // plain reads of at most kQuadMaxRead bases go kQuadReads to a warp, in FP64 two
     int pd_reads = 1;           // FP32 PD-HMM reads of at most 248 bases a warp
     uint64_t limit = ~uint64_t{0};
     int chunks(const ForwardPlan& p) const;
@@ -174,6 +174,10 @@ class Engine {
   // about two haplotypes'. With 16 uneven regions (1,400 steps) four reads a warp and one read a warp
   // take the same time (0.78 and 0.76 ms); with 1,024, 29.6 and 41.2 ms.
   static constexpr double kFullSteps = 600;
+  // And in FP64 the share of the resident warps that two reads a warp must give a task: with 800 tasks of
+  // long programs for 1,184 warps (8 regions of 200 reads x 128 SNP haplotypes) 2.81 ms against 2.63 at one
+  // read a warp; with 1,024 (8 uneven regions) 1.32 against 1.50, with 1,600 4.35 against 4.85.
+  static constexpr double kPairTasks = 0.8;
   SplitRule choose_split(const BatchInput& in, const EngineConfig& cfg, const std::vector<int64_t>& first_read,
                          const std::vector<RegionPlan>& plans) const;
   static constexpr int kAuxStreams = 8;

@@ -345,6 +345,7 @@ bool valid_rows(Kind k, int rows) {
     case Kind::kShortF32:
       return rows >= 1 && rows <= 8;
     case Kind::kQuadF32:
+    case Kind::kPairF64:
       return rows >= 2 && rows <= kQuadMaxRows && rows % 2 == 0;
     case Kind::kOneF32:
       return rows >= 10 && rows <= 20 && rows % 2 == 0;
@@ -431,7 +432,7 @@ cudaError_t long_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cu
 size_t scratch_bytes(Kind k, int rows, int max_slots, int max_nodes, int max_segs) {
   if (is_long(k) || !valid_rows(k, rows)) return 0;
   if (is_pd(k)) return pd_scratch_bytes(pd_form(k), rows, max_slots, max_segs);
-  if (k == Kind::kQuadF32) return quad_scratch_bytes(rows, max_slots, max_nodes, max_segs);
+  if (is_quad(k)) return quad_scratch_bytes(k, rows, max_slots, max_nodes, max_segs);
   return dispatch<SizeF>(k, rows, max_slots, max_nodes, max_segs);
 }
 
@@ -441,7 +442,7 @@ void occupancy(Kind k, int rows, int* blocks, int* threads, int warps) {
   if (is_long(k)) return long_occupancy(k, rows, blocks, threads, warps);
   if (!valid_rows(k, rows) || (warps != 1 && warps != 2 && warps != 4)) return;
   if (is_pd(k)) return pd_occupancy(pd_form(k), rows, blocks, threads, warps);
-  if (k == Kind::kQuadF32) return quad_occupancy(rows, blocks, threads);
+  if (is_quad(k)) return quad_occupancy(k, rows, blocks, threads);
   dispatch<OccF>(k, rows, blocks, threads, warps);
 }
 
@@ -455,7 +456,7 @@ cudaError_t launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStr
   if (is_long(k)) return long_launch(k, rows, blocks, args, stream, warps);
   if (!valid_rows(k, rows) || (warps != 1 && warps != 2 && warps != 4)) return cudaErrorInvalidValue;
   if (is_pd(k)) return pd_launch(pd_form(k), rows, blocks, args, stream, warps);
-  if (k == Kind::kQuadF32) return quad_launch(rows, blocks, args, stream);
+  if (is_quad(k)) return quad_launch(k, rows, blocks, args, stream);
   return dispatch<GoF>(k, rows, blocks, args, stream, warps);
 }
 

@@ -26,9 +26,10 @@ enum class Kind : int {
   kGenericF64Pd = 11,
   kQuadF32 = 12,   // up to four reads, two on each half of the lanes in FP32x2, rows-per-lane 2..14 (even)
   kOneF64Codes = 13,  // as kOneF64, priors by comparing haplotype codes (bytes other than A, C, G, T and N)
+  kPairF64 = 14,   // up to two reads, one on each half of the lanes in FP64, priors from a table, the quad form's rows
 };
-constexpr int kNumKinds = 14;
-// Lanes that hold two reads in the quad form, reads a warp, its largest rows-per-lane and its longest
+constexpr int kNumKinds = 15;
+// Lanes that hold two reads (FP32x2) or one (FP64) in the quad form, reads a warp in FP32x2, its largest rows-per-lane and its longest
 // read (the first row of the first lane is padding).
 constexpr int kQuadLanes = 16, kQuadReads = 4;
 constexpr int kQuadMaxRows = 14;
@@ -91,6 +92,7 @@ __host__ __device__ inline int queue_pair_bin(int len, bool generic) {
 }
 
 inline bool is_long(Kind k) { return k >= Kind::kLongF32 && k <= Kind::kGenericF64Pd; }
+inline bool is_quad(Kind k) { return k == Kind::kQuadF32 || k == Kind::kPairF64; }
 inline bool is_pd(Kind k) {
   return k == Kind::kOneF32Pd || k == Kind::kOneF64Pd || k == Kind::kPackedF32Pd || k == Kind::kLongF32Pd ||
          k == Kind::kLongF64Pd || k == Kind::kGenericF32Pd || k == Kind::kGenericF64Pd;
@@ -133,9 +135,9 @@ void occupancy(Kind k, int rows, int* blocks_per_sm, int* threads_per_block, int
 // Launches one persistent grid of `blocks` blocks.
 cudaError_t launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream, int warps_per_block = 4);
 // The quad form (quad.cpp). Warps per block are its own.
-size_t quad_scratch_bytes(int rows, int max_slots, int max_nodes, int max_segs);
-void quad_occupancy(int rows, int* blocks_per_sm, int* threads_per_block);
-cudaError_t quad_launch(int rows, int blocks, const LaunchArgs& args, cudaStream_t stream);
+size_t quad_scratch_bytes(Kind k, int rows, int max_slots, int max_nodes, int max_segs);
+void quad_occupancy(Kind k, int rows, int* blocks_per_sm, int* threads_per_block);
+cudaError_t quad_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream);
 // PD-HMM instantiations (pd_kernels.cu).
 size_t pd_scratch_bytes(PdForm form, int rows, int max_slots, int max_segs);
 void pd_occupancy(PdForm form, int rows, int* blocks_per_sm, int* threads_per_block, int warps_per_block = 4);

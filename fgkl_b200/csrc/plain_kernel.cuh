@@ -13,13 +13,14 @@
 // (two shuffles a step instead of the bottom row's M, X and Y, and no above-row state to keep, store in
 // snapshots or reload).
 //
-// Two forms. One read on all 32 lanes (G = 32) has the shortest steps and serves small batches, FP64 and
-// long reads. Four reads on two groups of 16 lanes in FP32x2 (the quad form) have half the steps that an
+// Two forms. One read on all 32 lanes (G = 32) has the shortest steps and serves small batches, long reads
+// and the recomputation. Four reads on two groups of 16 lanes in FP32x2 (the quad form) have half the steps that an
 // event spans and half the shuffles, selects and loop overhead a cell; at R = 10 they need 255 registers
 // and 21 KB of shared memory a warp, 8 warps an SM. Measured on 54,000 reads of 151 bases (1,024 uneven
 // regions): 20.5 ms, 2,750 G cells/s (the FP32 pipe 58% active without events, where it reaches 4,080);
 // two reads on 32 lanes in FP32x2 26.6 ms; two on 16 lanes in scalar FP32 at 16 warps an SM 23.2 ms; four
 // on 8 lanes in scalar FP32 23.3 ms.
+// In FP64 the same form holds two reads, one on each half of the lanes.
 //
 // Forward recurrence per cell (GATK LoglessPairHMM, fgkl kernel.rs:1011-1013):
 //   M = prior * (mm*M(i-1,j-1) + im*(X(i-1,j-1) + Y(i-1,j-1)))
@@ -261,7 +262,9 @@ constexpr int block_warps() {
 // warps an SM up to 8 rows.
 // FP64: three blocks of four warps while their registers hold the rows (128 regions in FP64, 5 rows: 7.8 ms,
 // against 8.3 at the 8 warps an SM of one block's full budget; four blocks 7.9); priors from the table
-// instead of by comparison 6.4 ms, and at 6 rows three blocks fit then.
+// instead of by comparison 6.4 ms, and at 6 rows three blocks fit then. Two reads on 16 lanes each take the
+// registers of 8 warps an SM (238 at 10 rows): 128 uneven regions 8.6 -> 7.5 ms, 128 of 128 SNP haplotypes
+// 35.1 -> 28.6 ms.
 constexpr int f64_min_blocks(int rows, bool table) { return rows <= (table ? 6 : 5) ? 3 : 1; }
 template <class P, int R, int G>
 struct MinBlocks {
@@ -270,7 +273,7 @@ struct MinBlocks {
   // A quarter of the SM's registers serves a quarter of its warps.
   static constexpr int kByRegs = 2 * (512 / ((kRegs + 7) / 8 * 8));
   static constexpr int kQuad = kByRegs < kBySmem ? kByRegs : kBySmem;
-  static constexpr int value = G < 32 ? (kQuad > 12 ? 12 : kQuad) : (P::kDouble ? f64_min_blocks(R, P::kTable) : (R <= 8 ? 4 : 2));
+  static constexpr int value = G < 32 ? (P::kDouble ? 4 : (kQuad > 12 ? 12 : kQuad)) : (P::kDouble ? f64_min_blocks(R, P::kTable) : (R <= 8 ? 4 : 2));
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -619,7 +622,7 @@ __device__ __forceinline__ void finalize(const LaunchArgs& a, const Task& task, 
   double* red = reinterpret_cast<double*>(sc.stage);  // [slot][row q], the staging buffers are free now
   constexpr int max_rows = G * R;
   const int slot0 = lane / G * P::NC, top = (lane % G) * R;
-  const int n_join_segs = (P::kDouble && task.hap >= 0) ? 0 : prog.n_segs;
+  const int n_join_segs = (P::kDouble && G == 32 && task.hap >= 0) ? 0 : prog.n_segs;
   // Joins (fgkl kernel.rs:767-791): raw = acc + (Σ_rows F_M*B_M + F_Y*B_Y + init*s) / BACKWARD_SCALE,
   // with the row sum taken in an order fixed by the read row so it does not depend on R or G.
   double yfac[R][P::NC];
@@ -672,7 +675,7 @@ __device__ __forceinline__ void finalize(const LaunchArgs& a, const Task& task, 
     __syncwarp();
   }
   __syncwarp();
-  if (P::kDouble && task.hap >= 0) {
+  if (P::kDouble && G == 32 && task.hap >= 0) {
     // A recomputation task: its one segment's result goes to the haplotype and its duplicates.
     const double raw = sc.raw(0, 0);
     const bool lost = raw != raw;
@@ -735,7 +738,7 @@ __device__ __forceinline__ void run_task(const LaunchArgs& a, const Task& task, 
     rd[c].pad = G * R - rd[c].len;
   }
   const uint8_t* codes = a.v.code_of_byte + region.code_off;
-  if (P::kDouble && task.hap >= 0) {
+  if (P::kDouble && G == 32 && task.hap >= 0) {
     const HapInfo info = a.v.haps[region.hap_off + task.hap];
     Scratch<P, R> sc(scratch, smem, 0, 0, 1);
     forward_pass<P, R, G>(a, prog, rd, codes, lane, sc, a.v.hap_codes + region.seq_off + info.seq, info.len);
@@ -748,7 +751,7 @@ __device__ __forceinline__ void run_task(const LaunchArgs& a, const Task& task, 
     forward_pass<P, R, G>(a, prog, rd, codes, lane, sc, nullptr, 0);
     __syncwarp();
     finalize<P, R, G>(a, task, region, prog, rd, lane, sc);
-    if (P::kDouble && a.only_lost) {
+    if (P::kDouble && G == 32 && a.only_lost) {
       // A dense read's shared FP64 sweep can lose a pair again (a joined result below the backward
       // range): each such distinct haplotype is swept once more here without sharing, which
       // cannot lose it (fgkl lib.rs:476-486).

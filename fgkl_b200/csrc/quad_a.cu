@@ -2,5 +2,5 @@
 #include "quad_kernel.cuh"
 
 namespace fgkl {
-template struct QuadRange<2, 8>;
+template struct QuadRange<false, 2, 8>;
 }  // namespace fgkl

@@ -2,5 +2,5 @@
 #include "quad_kernel.cuh"
 
 namespace fgkl {
-template struct QuadRange<10, 10>;
+template struct QuadRange<false, 10, 10>;
 }  // namespace fgkl

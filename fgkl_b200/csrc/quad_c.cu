@@ -2,5 +2,5 @@
 #include "quad_kernel.cuh"
 
 namespace fgkl {
-template struct QuadRange<12, 14>;
+template struct QuadRange<false, 12, 14>;
 }  // namespace fgkl

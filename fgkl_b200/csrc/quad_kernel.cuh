@@ -17,36 +17,39 @@ void rows_at(int rows, F&& f) {
     rows_at<R + 2, kHi>(rows, f);
 }
 
-template <int R>
+template <bool kDouble>
+using QuadPolicy = std::conditional_t<kDouble, OneF64Table, PackedF32>;
+
+template <bool kDouble, int R>
 constexpr size_t quad_smem() {
-  return kQuadWarps * Layout<PackedF32, R>::kSmemPerWarp;
+  return kQuadWarps * Layout<QuadPolicy<kDouble>, R>::kSmemPerWarp;
 }
 }  // namespace
 
-template <int kLo, int kHi>
-size_t QuadRange<kLo, kHi>::scratch(int rows, int max_slots, int max_nodes, int max_segs) {
+template <bool kDouble, int kLo, int kHi>
+size_t QuadRange<kDouble, kLo, kHi>::scratch(int rows, int max_slots, int max_nodes, int max_segs) {
   size_t bytes = 0;
-  rows_at<kLo, kHi>(rows, [&](auto r) { bytes = scratch_size<PackedF32, decltype(r)::value>(max_slots, max_nodes, max_segs); });
+  rows_at<kLo, kHi>(rows, [&](auto r) { bytes = scratch_size<QuadPolicy<kDouble>, decltype(r)::value>(max_slots, max_nodes, max_segs); });
   return bytes;
 }
 
-template <int kLo, int kHi>
-int QuadRange<kLo, kHi>::occupancy(int rows, int* threads) {
+template <bool kDouble, int kLo, int kHi>
+int QuadRange<kDouble, kLo, kHi>::occupancy(int rows, int* threads) {
   int blocks = 0;
   *threads = kQuadWarps * 32;
   rows_at<kLo, kHi>(rows, [&](auto r) {
     constexpr int R = decltype(r)::value;
     static std::atomic<int> cache[kMaxDevices];
-    blocks = resident_blocks(pairhmm_kernel<PackedF32, R, kQuadLanes>, quad_smem<R>(), kQuadWarps * 32, cache);
+    blocks = resident_blocks(pairhmm_kernel<QuadPolicy<kDouble>, R, kQuadLanes>, quad_smem<kDouble, R>(), kQuadWarps * 32, cache);
   });
   return blocks;
 }
 
-template <int kLo, int kHi>
-cudaError_t QuadRange<kLo, kHi>::launch(int rows, int blocks, const LaunchArgs& a, cudaStream_t s) {
+template <bool kDouble, int kLo, int kHi>
+cudaError_t QuadRange<kDouble, kLo, kHi>::launch(int rows, int blocks, const LaunchArgs& a, cudaStream_t s) {
   rows_at<kLo, kHi>(rows, [&](auto r) {
     constexpr int R = decltype(r)::value;
-    pairhmm_kernel<PackedF32, R, kQuadLanes><<<blocks, kQuadWarps * 32, quad_smem<R>(), s>>>(a);
+    pairhmm_kernel<QuadPolicy<kDouble>, R, kQuadLanes><<<blocks, kQuadWarps * 32, quad_smem<kDouble, R>(), s>>>(a);
   });
   return cudaGetLastError();
 }

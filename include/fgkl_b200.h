@@ -225,9 +225,9 @@ int fgkl_context_get_tuning(const fgkl_context* ctx, fgkl_tuning* tuning);
  * events around each, so each is timed alone; fgkl_batch_launch_profile
  * waits and reports every first-pass and recomputation launch of the last run: kernel kind
  * (0 FP32 for reads of at most 248 bases, 1 FP32, 2 FP64, 3 PD FP32, 4 PD FP64, 5 PD packed FP32, 12
- * FP32 with four reads a warp, 13 FP64 comparing codes; strip-mined: 6 FP32, 7 FP64, 8 PD FP32, 9 PD
- * FP64, 10 and 11 byte-compared PD FP32 and FP64), rows per lane, tasks, blocks, whether it is a
- * recomputation launch, the forward and backward DP cells its tasks compute, and its duration. */
+ * FP32 with four reads a warp, 13 FP64 comparing codes, 14 FP64 with two reads a warp; strip-mined: 6
+ * FP32, 7 FP64, 8 PD FP32, 9 PD FP64, 10 and 11 byte-compared PD FP32 and FP64), rows per lane, tasks,
+ * blocks, whether it is a recomputation launch, the forward and backward DP cells its tasks compute, and its duration. */
 typedef struct fgkl_launch_profile {
   int32_t kind;
   int32_t rows;

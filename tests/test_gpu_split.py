@@ -29,15 +29,16 @@ def regions(lens, n_regions, reads, haps, hap_len, pd=False):
 
 @pytest.mark.parametrize("lens", [(1, 15, 16, 31), (32, 63, 64, 95), (127, 128, 159, 160), (191, 192, 223, 224)])
 @pytest.mark.parametrize("share", [True, False])
-def test_quads_and_single_reads_give_the_same_bits(gpu, lens, share):
+@pytest.mark.parametrize("precision,kind", [(Precision.FLOAT, 12), (Precision.DOUBLE, 14)])
+def test_quads_and_single_reads_give_the_same_bits(gpu, lens, share, precision, kind):
     parts = regions(lens, 24, 40, 14, 300)
     w = synthetic.from_regions(parts)
-    cfg = Config(share_suffixes=share)
+    cfg = Config(precision=precision, share_suffixes=share)
     ctx = BatchContext()
     ctx.set_profiling(True)
     out, _ = ctx.compute(w, cfg)
     kinds = {p["kind"] for p in ctx.launch_profile() if not p["recomputation"]}
-    assert 12 in kinds  # four reads a warp
+    assert kind in kinds  # four reads a warp in FP32, two in FP64
     offs = w.output_offsets()
     for g in (0, 11, 23):
         reads, haps = parts[g]
@@ -46,7 +47,7 @@ def test_quads_and_single_reads_give_the_same_bits(gpu, lens, share):
     keep = slice(0, None, 7)
     ref = O.compute_matrix(reads[keep], haps).reshape(-1, len(haps))
     got = out[offs[5]:offs[6]].reshape(len(reads), len(haps))[keep]
-    assert np.max(np.abs(got - ref)) < TOL[Precision.FLOAT]
+    assert np.max(np.abs(got - ref)) < TOL[precision]
 
 
 @pytest.mark.parametrize("pd", [False, True])
