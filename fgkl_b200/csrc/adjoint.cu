@@ -682,14 +682,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (AdjMinBlocks<P, R>::valu
     if (t >= count) break;
     const int read = a.tasks[t] / a.split, part = a.tasks[t] % a.split;
     const int g = a.v.read_region[read];
-    AdjView v = a.v;
-    if (part > 0) {
-      v.g_ins = a.part + static_cast<size_t>(part - 1) * 4 * a.part_len;
-      v.g_del = v.g_ins + a.part_len;
-      v.g_eps = v.g_del + a.part_len;
-      v.g_err = v.g_eps + a.part_len;
-    }
     const int64_t off = a.v.read_off[read];
+    // The part's gradients, from the first part's: four arrays a part, one part after another.
+    const int64_t g_off = off + static_cast<int64_t>(part) * 4 * a.part_len;
     const int len = static_cast<int>(a.v.read_off[read + 1] - off);
     const int blocks = adj_row_blocks(len, R);
     const int pad0 = 32 * R * blocks - len;
@@ -703,10 +698,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (AdjMinBlocks<P, R>::valu
         for (int r = 0; r < R; ++r) {
           const int q = lane * R + r - (pad0 - 32 * R * blk);
           if (q < 0 || q >= len) continue;
-          atomicExch(reinterpret_cast<unsigned long long*>(v.g_ins + off + q), 0ull);
-          atomicExch(reinterpret_cast<unsigned long long*>(v.g_del + off + q), 0ull);
-          atomicExch(reinterpret_cast<unsigned long long*>(v.g_eps + off + q), 0ull);
-          atomicExch(reinterpret_cast<unsigned long long*>(v.g_err + off + q), 0ull);
+          atomicExch(reinterpret_cast<unsigned long long*>(a.v.g_ins + g_off + q), 0ull);
+          atomicExch(reinterpret_cast<unsigned long long*>(a.v.g_del + g_off + q), 0ull);
+          atomicExch(reinterpret_cast<unsigned long long*>(a.v.g_eps + g_off + q), 0ull);
+          atomicExch(reinterpret_cast<unsigned long long*>(a.v.g_err + g_off + q), 0ull);
         }
       __syncwarp();
     }
@@ -755,7 +750,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (AdjMinBlocks<P, R>::valu
         AdjCoef<P, R> c;
         const int pad = pad0 - 32 * R * blk;
         c.load(a.v, off, len, pad, lane);
-        fwd = adj_forward<P, R>(v, c, off, pad, hap, m, lane, sc, blk, smem, c_fac, init_a);
+        fwd = adj_forward<P, R>(a.v, c, g_off, pad, hap, m, lane, sc, blk, smem, c_fac, init_a);
         __syncwarp();
       }
       const double fwd_raw = ldexp(static_cast<double>(fwd), shift);
@@ -779,10 +774,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (AdjMinBlocks<P, R>::valu
   }
 }
 
-__global__ void adj_reduce_kernel(double* grad, const double* part, size_t n, int parts) {
+__global__ void adj_reduce_kernel(double* grad, size_t n, int parts) {
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
     double g = grad[i];
-    for (int k = 0; k < parts; ++k) g = __dadd_rn(g, part[static_cast<size_t>(k) * n + i]);
+    for (int k = 1; k < parts; ++k) g = __dadd_rn(g, grad[static_cast<size_t>(k) * n + i]);
     grad[i] = g;
   }
 }
@@ -846,9 +841,9 @@ void adj_occupancy(bool dbl, int rows, int* blocks, int* threads) {
 }
 
 cudaError_t adj_reduce(const AdjLaunch& a, cudaStream_t s) {
-  const size_t n = 4 * a.part_len;
+  const size_t n = 4 * static_cast<size_t>(a.part_len);
   if (a.split < 2 || n == 0) return cudaSuccess;
-  adj_reduce_kernel<<<static_cast<int>(std::min<size_t>((n + 255) / 256, 2048)), 256, 0, s>>>(a.v.g_ins, a.part, n, a.split - 1);
+  adj_reduce_kernel<<<static_cast<int>(std::min<size_t>((n + 255) / 256, 2048)), 256, 0, s>>>(a.v.g_ins, n, a.split);
   return cudaGetLastError();
 }
 

@@ -46,8 +46,7 @@ struct AdjLaunch {
   char* scratch;
   size_t scratch_stride; // bytes per warp (adj_scratch_bytes of the launch's largest pair)
   int split;             // parts that a read's haplotypes are shared among
-  double* part;          // gradients of parts 1 .. split - 1, four arrays each (part 0 adds into the view's)
-  size_t part_len;       // read positions: the length of one array
+  int64_t part_len;      // read positions, the length of a gradient array; part k's four arrays lie 4 k of them past the view's
   int* lost_flag;        // per read: set by the first part that loses it in FP32; zeroed before the launch
   int32_t* queue;        // FP32 launches: tasks of reads lost in FP32, for FP64 (per-bin slices), or nullptr
   const int* queue_off;  // per rows-per-lane bin: first queue slot (kAdjRowBins + 1 entries)

@@ -41,7 +41,6 @@ AdjointEngine::~AdjointEngine() {
   cudaFree(d_out_);
   cudaFree(d_small_);
   cudaFree(d_lost_);
-  cudaFree(d_part_);
   cudaFree(d_scratch_);
   for (int i = 0; i < kAux; ++i) {
     if (aux_[i]) cudaStreamSynchronize(aux_[i]);
@@ -196,8 +195,7 @@ int AdjointEngine::prepare(const AdjointInput& in, bool double_precision) {
   n_small_ = static_cast<int>(bins_.size() + rescue_.size()) + 2 * kAdjRowBins + 1;
   if (!grow(d_bytes_, cap_bytes_, n_bytes) || !grow(d_params_, cap_params_, 4 * static_cast<size_t>(grad_len_) + 1) ||
       !grow(d_off_, cap_off_, n_off + 1) || !grow(d_idx_, cap_idx_, n_idx + 1) ||
-      !grow(d_out_, cap_out_, static_cast<size_t>(out_len_) + 4 * static_cast<size_t>(grad_len_) + 1) ||
-      !grow(d_part_, cap_part_, static_cast<size_t>(split_ - 1) * 4 * static_cast<size_t>(grad_len_)) ||
+      !grow(d_out_, cap_out_, static_cast<size_t>(out_len_) + static_cast<size_t>(split_) * 4 * static_cast<size_t>(grad_len_) + 1) ||
       !grow(d_small_, cap_small_, static_cast<size_t>(n_small_) + static_cast<size_t>(total_reads)) || !grow(d_scratch_, cap_scratch_, scratch))
     return fail(FGKL_E_OUT_OF_MEMORY, "device allocation failed");
 
@@ -280,10 +278,8 @@ int AdjointEngine::run() {
   if ((rc = check(cudaMemsetAsync(d_lost_, 0, sizeof(unsigned long long), stream_), "reset counters"))) return rc;
   // The kernels add each pair's gradient terms into the per-position arrays.
   if (grad_len_ > 0 &&
-      (rc = check(cudaMemsetAsync(view_.g_ins, 0, 4 * static_cast<size_t>(grad_len_) * sizeof(double), stream_), "reset gradients")))
+      (rc = check(cudaMemsetAsync(view_.g_ins, 0, static_cast<size_t>(split_) * 4 * static_cast<size_t>(grad_len_) * sizeof(double), stream_), "reset gradients")))
     return rc;
-  const size_t part_bytes = static_cast<size_t>(split_ - 1) * 4 * static_cast<size_t>(grad_len_) * sizeof(double);
-  if (part_bytes > 0 && (rc = check(cudaMemsetAsync(d_part_, 0, part_bytes, stream_), "reset gradients"))) return rc;
   int* lost_flag = d_small_ + n_small_;
   if (n_reads_ > 0 && (rc = check(cudaMemsetAsync(lost_flag, 0, static_cast<size_t>(n_reads_) * sizeof(int), stream_), "reset flags"))) return rc;
   launches_ = 0;
@@ -291,8 +287,7 @@ int AdjointEngine::run() {
   AdjLaunch parts{};
   parts.v = view_;
   parts.split = split_;
-  parts.part = d_part_;
-  parts.part_len = static_cast<size_t>(grad_len_);
+  parts.part_len = grad_len_;
   parts.lost_flag = lost_flag;
   for (int pass = 0; pass < 2; ++pass) {
     const auto& list = pass == 0 ? bins_ : rescue_;

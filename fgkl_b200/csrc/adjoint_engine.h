@@ -75,7 +75,7 @@ class AdjointEngine {
   size_t cap_off_ = 0;
   int32_t* d_idx_ = nullptr;    // read regions | region first hap | count | first read | tasks | queue
   size_t cap_idx_ = 0;
-  double* d_out_ = nullptr;     // likelihoods | 4 gradient arrays
+  double* d_out_ = nullptr;     // likelihoods | 4 gradient arrays a part
   size_t cap_out_ = 0;
   int* d_small_ = nullptr;      // task counters | queue offsets | queue tails
   size_t cap_small_ = 0;
@@ -91,8 +91,6 @@ class AdjointEngine {
   bool side_by_side_ = false;
   int split_ = 1;    // parts that a read's haplotypes are shared among
   int64_t n_reads_ = 0;
-  double* d_part_ = nullptr;  // gradients of the parts beyond the first, four arrays each
-  size_t cap_part_ = 0;
 };
 
 }  // namespace fgkl
