@@ -1,5 +1,7 @@
 #include "engine.h"
 
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -189,11 +191,21 @@ void emit_region(RegionPlan& plan, int chunks) {
 // planning of a batch of a few regions). They run host code only and make no CUDA call. Never destroyed:
 // a helper that waits when the process exits holds nothing. Loops of several callers share the helpers;
 // a caller works on its own loop beside them and never waits for one that has not begun on it, so a
-// process forked from one with helpers, or one that cannot start any, runs its loops by itself.
+// process that cannot start any runs its loops by itself.
 class Helpers {
  public:
+  // The process's own. A forked child has none of its parent's threads, but copies of the lock and the
+  // condition variables that they may have held or waited on, which must not be used again: it gets
+  // helpers of its own.
   static Helpers& get() {
-    static Helpers* const h = new Helpers;
+    static std::atomic<Helpers*> current{nullptr};
+    const pid_t self = getpid();
+    Helpers* h = current.load(std::memory_order_acquire);
+    while (!h || h->owner_ != self) {
+      Helpers* const fresh = new Helpers(self);
+      if (current.compare_exchange_strong(h, fresh, std::memory_order_acq_rel)) return *fresh;
+      delete fresh;  // another thread was first; no helper has been started on this one
+    }
     return *h;
   }
 
@@ -231,6 +243,8 @@ class Helpers {
   };
   static constexpr int kMost = 64;
 
+  explicit Helpers(pid_t owner) : owner_(owner) {}
+
   void do_work(Job& job) {
     try {
       (*job.work)();
@@ -259,6 +273,7 @@ class Helpers {
     --total_;
   }
 
+  const pid_t owner_;  // the process whose threads these are
   std::mutex m_;
   std::condition_variable wake_, done_;
   std::deque<Job*> tickets_;
