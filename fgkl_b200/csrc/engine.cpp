@@ -12,6 +12,7 @@
 #include <deque>
 #include <exception>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -71,7 +72,7 @@ int single_rows(int len) {
 }  // namespace
 
 struct RegionPlan {
-  SortedHaps set;
+  std::unique_ptr<SortedHaps> set;  // until its programs are emitted, as fwd.segs
   ForwardPlan fwd;
   std::vector<ProgramBuild> progs;
   std::vector<HapInfo> haps;
@@ -109,7 +110,22 @@ bool pd_read_classes(const BatchInput& in, int64_t first_read, int n_reads, cons
   return true;
 }
 
-void plan_region(const BatchInput& in, int g, int64_t first_read, int64_t first_hap, bool share, RegionPlan& out) {
+// Emits a planned region's programs: its segments in `chunks` runs at most. Gives the sorted set back.
+void emit_region(RegionPlan& plan, int chunks) {
+  const std::vector<int32_t> bounds = split_segments(plan.fwd, chunks);
+  plan.progs.resize(bounds.size() - 1);
+  try {
+    for (size_t c = 0; c + 1 < bounds.size(); ++c) emit_program(*plan.set, plan.fwd, bounds[c], bounds[c + 1], plan.progs[c]);
+  } catch (const std::exception& e) {
+    plan.error = e.what();
+  }
+  plan.set.reset();
+  plan.fwd.segs = {};
+}
+
+// `whole`: the region's one program is emitted here too and the sorted set, most of a plan's memory, given
+// back; else emit_region follows.
+void plan_region(const BatchInput& in, int g, int64_t first_read, int64_t first_hap, bool share, bool whole, RegionPlan& out) {
   const int n_haps = in.region_haps[g], n_reads = in.region_reads[g];
   std::vector<HapView> views(static_cast<size_t>(n_haps));
   std::vector<const uint8_t*> flags(in.hap_flags ? static_cast<size_t>(n_haps) : 0);
@@ -123,7 +139,8 @@ void plan_region(const BatchInput& in, int g, int64_t first_read, int64_t first_
     out.read_bases += static_cast<uint64_t>(in.read_off[first_read + r + 1] - in.read_off[first_read + r]);
   if (n_haps == 0 || n_reads == 0) return;
   const bool pd = in.hap_flags != nullptr;
-  SortedHaps& s = out.set;
+  out.set = std::make_unique<SortedHaps>();
+  SortedHaps& s = *out.set;
   try {
     s = pd ? SortedHaps::make_pd(views, flags) : SortedHaps::make(views, share);
     out.fwd = forward_plan(s, share && !pd);
@@ -173,17 +190,7 @@ void plan_region(const BatchInput& in, int g, int64_t first_read, int64_t first_
     h.len = s.bases[k].len;
     h.pad_[0] = h.pad_[1] = h.pad_[2] = 0;
   }
-}
-
-// Emits a planned region's programs: its segments in `chunks` runs at most.
-void emit_region(RegionPlan& plan, int chunks) {
-  const std::vector<int32_t> bounds = split_segments(plan.fwd, chunks);
-  plan.progs.resize(bounds.size() - 1);
-  try {
-    for (size_t c = 0; c + 1 < bounds.size(); ++c) emit_program(plan.set, plan.fwd, bounds[c], bounds[c + 1], plan.progs[c]);
-  } catch (const std::exception& e) {
-    plan.error = e.what();
-  }
+  if (whole) emit_region(out, 1);
 }
 
 // The process's helper threads. They are started when a loop asks for them, wait for the next one, and
@@ -478,7 +485,7 @@ int plan_region_cells(const BatchInput& in, const EngineConfig& cfg, uint64_t* c
   parallel_for(N, host_threads(), [&](int64_t gi) {
     const int g = static_cast<int>(gi);
     RegionPlan rp;
-    plan_region(in, g, first_read[g], first_hap[g], cfg.share_suffixes, rp);
+    plan_region(in, g, first_read[g], first_hap[g], cfg.share_suffixes, false, rp);
     uint64_t distinct_len = 0;
     for (int k = 0; k < static_cast<int>(rp.haps.size()); ++k)
       if (rp.haps[k].src == k) distinct_len += static_cast<uint64_t>(rp.haps[k].len);
@@ -497,7 +504,7 @@ int plan_region_cells(const BatchInput& in, const EngineConfig& cfg, uint64_t* c
 
 // How a batch's first pass is spread: see choose_split.
 int Engine::SplitRule::chunks(const ForwardPlan& p) const {
-  const uint64_t steps = p.steps(), n = p.segs.size();
+  const uint64_t steps = p.steps(), n = static_cast<uint64_t>(p.n_segs);
   if (steps <= limit || n < 2) return 1;
   return static_cast<int>(std::min<uint64_t>(n, (steps + limit - 1) / limit));
 }
@@ -524,11 +531,9 @@ Engine::SplitRule Engine::choose_split(const BatchInput& in, const EngineConfig&
   double reads_steps = 0;  // one read a warp
   for (int g = 0; g < N; ++g) {
     const RegionPlan& rp = plans[g];
-    if (rp.fwd.segs.empty()) continue;
-    uint64_t prefix = 0;
-    for (const auto& s : rp.fwd.segs) prefix += static_cast<uint64_t>(s.start);
-    work.push_back({static_cast<double>(rp.fwd.steps()), static_cast<double>(in.region_reads[g]), static_cast<double>(rp.fwd.segs.size()),
-                    static_cast<double>(prefix) / static_cast<double>(rp.fwd.segs.size())});
+    if (rp.fwd.n_segs == 0) continue;
+    work.push_back({static_cast<double>(rp.fwd.steps()), static_cast<double>(in.region_reads[g]), static_cast<double>(rp.fwd.n_segs),
+                    static_cast<double>(rp.fwd.prefixes) / static_cast<double>(rp.fwd.n_segs)});
     reads_steps += work.back().steps * work.back().tasks;
   }
   int reads_per_warp = 1;
@@ -641,16 +646,28 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   // 75 us to plan; a combined batch of per-call requests holds a few).
   std::vector<RegionPlan> plans(static_cast<size_t>(N));
   const bool share = cfg.share_suffixes;
+  // A batch of many reads keeps one program a region (choose_split), so they are emitted while their
+  // regions are planned, and the few regions to split, if any, are planned again: sorted sets kept for all
+  // regions until the split is known cost host time: planning 6,000 regions of 2 reads x 16
+  // haplotypes of 350 bases took 44 ms on 8 cores that way, and takes 30.
+  const bool whole = total_reads >= kWholeReads * 8 * sms_ || N >= kWholeRegions * 8 * sms_;
   parallel_for(N, host_threads(),
-               [&](int64_t g) { plan_region(in, static_cast<int>(g), first_read[g], first_hap[g], share, plans[g]); });
+               [&](int64_t g) { plan_region(in, static_cast<int>(g), first_read[g], first_hap[g], share, whole, plans[g]); });
 
   const bool pd = in.hap_flags != nullptr;
   const SplitRule split = choose_split(in, cfg, first_read, plans);
-  parallel_for(N, host_threads(), [&](int64_t g) {
+  const auto emit = [&](int64_t g) {
     RegionPlan& rp = plans[g];
-    if (rp.error.empty() && !rp.haps.empty()) emit_region(rp, split.chunks(rp.fwd));
-    rp.set = SortedHaps();  // freed here, on the threads that plan
-  });
+    if (!rp.error.empty() || rp.haps.empty()) return;
+    const int chunks = split.chunks(rp.fwd);
+    if (whole && chunks == 1) return;
+    if (whole) {
+      rp = RegionPlan();
+      plan_region(in, static_cast<int>(g), first_read[g], first_hap[g], share, false, rp);
+    }
+    emit_region(rp, chunks);
+  };
+  parallel_for(N, host_threads(), emit);
 
   for (int g = 0; g < N; ++g)
     if (!plans[g].error.empty()) return fail(FGKL_E_UNSUPPORTED, "region " + std::to_string(g) + ": " + plans[g].error);
@@ -1012,7 +1029,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
     std::memset(blob + o_pd_seq + n_pd_seq * sizeof(uint32_t), 0, 16);
     std::memset(blob + o_sigs + n_sigs * sizeof(uint32_t), 0, 16);
     parallel_for(N, std::min(host_threads(), (N + 31) / 32), [&](int64_t g) {
-      const RegionPlan& rp = plans[g];
+      const RegionPlan rp = std::move(plans[g]);  // its last use: freed here, by the threads at work
       const Region& R = regions[g];
       if (!rp.haps.empty()) std::memcpy(blob + o_haps + static_cast<size_t>(R.hap_off) * sizeof(HapInfo), rp.haps.data(), rp.haps.size() * sizeof(HapInfo));
       auto put = [&](const std::vector<uint32_t>& v, int32_t off) {

@@ -178,6 +178,8 @@ class Engine {
   // long programs for 1,184 warps (8 regions of 200 reads x 128 SNP haplotypes) 2.81 ms against 2.63 at one
   // read a warp; with 1,024 (8 uneven regions) 1.32 against 1.50, with 1,600 4.35 against 4.85.
   static constexpr double kPairTasks = 0.8;
+  // Reads, and regions, a resident warp from which hardly any region is split.
+  static constexpr int64_t kWholeReads = 8, kWholeRegions = 2;
   SplitRule choose_split(const BatchInput& in, const EngineConfig& cfg, const std::vector<int64_t>& first_read,
                          const std::vector<RegionPlan>& plans) const;
   static constexpr int kAuxStreams = 8;

@@ -382,7 +382,9 @@ ForwardPlan forward_plan(const SortedHaps& s, bool with_suffix) {
     }
     tree_len[root[i]] = std::max(tree_len[root[i]], g.len);
     p.fwd_columns += static_cast<uint64_t>(g.last() - g.start);
+    p.prefixes += static_cast<uint64_t>(g.start);
   }
+  p.n_segs = m;
   for (int32_t i = 0; i < m; ++i) p.segs[i].tree_len = tree_len[root[i]];
   if (slots.size() >= (s.pd ? kPdPayloadNone : kPayloadNone))
     throw std::invalid_argument("too many snapshot slots for the stream payload");
@@ -398,9 +400,7 @@ std::vector<int32_t> split_segments(const ForwardPlan& p, int32_t chunks) {
   std::vector<int32_t> bounds{0};
   if (chunks > 1 && m > 1) {
     // A chunk costs its segments' columns and the prefix that its first segment resumes from.
-    uint64_t prefix = 0;
-    for (const auto& g : p.segs) prefix += static_cast<uint64_t>(g.start);
-    const double target = (static_cast<double>(p.fwd_columns) + (chunks - 1.0) * static_cast<double>(prefix) / m) / chunks;
+    const double target = (static_cast<double>(p.fwd_columns) + (chunks - 1.0) * static_cast<double>(p.prefixes) / m) / chunks;
     double cost = p.segs[0].last();
     for (int32_t i = 1; i < m; ++i) {
       const double own = p.segs[i].last() - p.segs[i].start;

@@ -109,6 +109,8 @@ struct ForwardPlan {
     int32_t last() const { return cut.column >= 0 ? cut.column : stop; }
   };
   std::vector<Seg> segs;
+  int32_t n_segs = 0;      // of the whole set, and
+  uint64_t prefixes = 0;   // the sum of their starts
   // Columns of the whole set's forward and backward passes, per read row.
   uint64_t fwd_columns = 0, bwd_columns = 0;
   bool has_backward = false;
