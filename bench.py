@@ -332,7 +332,7 @@ def extra_configs(args, device, stream, flush, threads, which=("c2", "c3", "c4",
         dom = max(first, key=lambda x: x["ms"])
         dom_tf = (FLOP_FORWARD * dom["forward_cells"] + FLOP_BACKWARD * dom["backward_cells"]) / (dom["ms"] / 1e3) / 1e12
         step_tf = (FLOP_FORWARD * st.forward_cells + FLOP_BACKWARD * st.backward_cells) / t / 1e12
-        kinds = {0: "OneF32", 12: "PackedF32 quad", 1: "OneF32", 2: "OneF64Table", 13: "OneF64", 14: "OneF64Table pair", 3: "OneF32Pd", 4: "OneF64Pd", 5: "PackedF32Pd"}
+        kinds = {0: "OneF32", 12: "PackedF32 quad", 15: "PackedF32", 1: "OneF32", 2: "OneF64Table", 13: "OneF64", 14: "OneF64Table pair", 3: "OneF32Pd", 4: "OneF64Pd", 5: "PackedF32Pd"}
         kname = "pd_kernel" if dom["kind"] in (3, 4, 5) else "pairhmm_kernel"
         roof = {"bound": "fp32", "unit": "TFLOP/s", "peak": peak, "achieved": dom_tf, "frac": dom_tf / peak,
                 "dominant_launch": {"kernel": f"{kname}<{kinds.get(dom['kind'], dom['kind'])}, {dom['rows']}>",
@@ -623,7 +623,7 @@ def ours(args, rank, world, local, pg):
     peak = max(s_tf.value, p_tf.value)
     achieved = dom_flops / (dom["ms"] / 1e3) / 1e12
     step_achieved = flops / step / 1e12
-    kind_names = {0: "OneF32", 12: "PackedF32 quad", 1: "OneF32", 2: "OneF64Table", 13: "OneF64", 14: "OneF64Table pair", 3: "OneF32Pd", 4: "OneF64Pd", 5: "PackedF32Pd"}
+    kind_names = {0: "OneF32", 12: "PackedF32 quad", 15: "PackedF32", 1: "OneF32", 2: "OneF64Table", 13: "OneF64", 14: "OneF64Table pair", 3: "OneF32Pd", 4: "OneF64Pd", 5: "PackedF32Pd"}
     dominant = {"kernel": f"pairhmm_kernel<{kind_names.get(dom['kind'], dom['kind'])}, {dom['rows']}>",
                 "ms": dom["ms"], "tasks": dom["tasks"], "blocks": dom["blocks"],
                 "forward_cells": dom["forward_cells"], "backward_cells": dom["backward_cells"],

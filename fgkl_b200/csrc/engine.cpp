@@ -513,10 +513,12 @@ int Engine::SplitRule::chunks(const ForwardPlan& p) const {
 // few tasks leaves most of the GPU idle while the longest run: there the reads go one to a warp and each
 // region's segments are spread over several programs, at the cost of the prefixes that these recompute
 // (one region of 64 reads x 16 PD haplotypes: 1.38 -> 0.30 ms with a haplotype a program). A batch with
-// tasks enough for every resident warp keeps one program a region and the forms with the most reads a
-// warp. In between, the step limit is the one that makes the estimate -- the larger of the mean steps a
-// warp gets and the longest program -- smallest (16 uneven regions: 1,400 steps and 0.78 ms; 600 steps
-// 1.11 ms, 3,000 steps 0.98 ms).
+// tasks enough for every resident warp keeps one program a region and the form that takes its regions'
+// reads in the least time: four a warp where the regions have many (1,024 uneven regions: 29.6 ms; one a
+// warp 41.2), two or one where they have few (6,000 regions of 1, 2, 3 and 6 reads: one a warp 1.59, 2.94,
+// 4.26 and 8.31 ms, two 2.49, 2.53, 4.73 and 7.05, four 3.89, 3.99, 4.01 and 7.72). In between, the step limit
+// is the one that makes the estimate -- the larger of the mean steps a warp gets and the longest program --
+// smallest (16 uneven regions: 1,400 steps and 0.78 ms; 600 steps 1.11 ms, 3,000 steps 0.98 ms).
 Engine::SplitRule Engine::choose_split(const BatchInput& in, const EngineConfig& cfg, const std::vector<int64_t>& first_read,
                                        const std::vector<RegionPlan>& plans) const {
   const int N = in.num_regions;
@@ -524,29 +526,76 @@ Engine::SplitRule Engine::choose_split(const BatchInput& in, const EngineConfig&
   const bool pd = in.hap_flags != nullptr;
   SplitRule rule;
   struct Work {
-    double steps, tasks, segs, prefix;
+    double steps, segs, prefix;
+    int short_reads, mid_reads, rest;  // of at most kQuadMaxRead bases, of more that fit 8 rows per lane, longer
+    double tasks;
   };
   std::vector<Work> work;
   work.reserve(static_cast<size_t>(N));
-  double reads_steps = 0;  // one read a warp
+  bool extra_codes = false;  // a batch of FP64 reads takes one form
   for (int g = 0; g < N; ++g) {
     const RegionPlan& rp = plans[g];
     if (rp.fwd.n_segs == 0) continue;
-    work.push_back({static_cast<double>(rp.fwd.steps()), static_cast<double>(in.region_reads[g]), static_cast<double>(rp.fwd.n_segs),
-                    static_cast<double>(rp.fwd.prefixes) / static_cast<double>(rp.fwd.n_segs)});
-    reads_steps += work.back().steps * work.back().tasks;
+    Work w{static_cast<double>(rp.fwd.steps()), static_cast<double>(rp.fwd.n_segs),
+           static_cast<double>(rp.fwd.prefixes) / static_cast<double>(rp.fwd.n_segs), 0, 0, 0, 0};
+    for (int64_t r = first_read[g]; r < first_read[g + 1]; ++r) {
+      const int64_t len = in.read_off[r + 1] - in.read_off[r];
+      ++(rp.generic || len > 8 * 31 || (rp.extra_codes && !cfg.double_precision) ? w.rest : len > kQuadMaxRead ? w.mid_reads : w.short_reads);
+    }
+    extra_codes |= rp.extra_codes;
+    work.push_back(w);
   }
-  int reads_per_warp = 1;
+  // A region's tasks with `reads` a warp, and the time they take for each step, in steps of one read's: only
+  // reads of one region share a warp, and only those that the form holds.
+  struct Count {
+    double tasks, time;
+  };
+  auto count = [&](const Work& w, int reads) -> Count {
+    const int fit = w.short_reads + w.mid_reads;
+    if (reads == 1) return {static_cast<double>(fit + w.rest), static_cast<double>(fit + w.rest)};
+    if (reads == kQuadReads) {
+      // The reads too long for the form go one to a warp or, where they are many, two, an odd one of a region
+      // with a shorter read.
+      const int apart = rule.mid_pairs ? (w.mid_reads + 1) / 2 : w.mid_reads;
+      const int quads = (std::max(0, w.short_reads - (rule.mid_pairs ? w.mid_reads % 2 : 0)) + kQuadReads - 1) / kQuadReads;
+      return {static_cast<double>(w.rest + apart + quads), w.rest + apart * (rule.mid_pairs ? kPairCost : 1.0) + quads * kQuadCost};
+    }
+    const int alone = w.rest + (cfg.double_precision ? w.mid_reads : 0);
+    const int pairs = (fit + w.rest - alone + 1) / 2;
+    return {static_cast<double>(alone + pairs), alone + pairs * (cfg.double_precision ? kF64PairCost : pd ? kPdPairCost : kPairCost)};
+  };
+  double mid_pairs = 0;
+  for (const Work& w : work) mid_pairs += (w.mid_reads + 1) / 2;
+  rule.mid_pairs = mid_pairs >= kPairTasks * warps;
+  // The form whose tasks take the least time in all, among those that give every resident warp work.
+  auto choose = [&](std::initializer_list<int> forms) {
+    int chosen = 1;
+    double least = -1;
+    for (const int reads : forms) {
+      double steps = 0, tasks = 0, time = 0;
+      for (const Work& w : work) {
+        const Count c = count(w, reads);
+        tasks += c.tasks;
+        steps += w.steps * c.tasks;
+        time += w.steps * c.time;
+      }
+      if (reads > 1 && steps < kFullSteps * warps) continue;
+      if (reads == 2 && !pd && tasks < (cfg.double_precision ? kF64PairTasks : kPairTasks) * warps) continue;
+      if (least < 0 || time < least) {
+        least = time;
+        chosen = reads;
+      }
+    }
+    return chosen;
+  };
   if (pd && !cfg.double_precision) {
-    if (tuning_.reads_per_warp == 2 && reads_steps / 2 >= kFullSteps * warps) reads_per_warp = rule.pd_reads = 2;
+    if (tuning_.reads_per_warp == 2) rule.reads = choose({1, 2});
+  } else if (!pd && cfg.double_precision) {
+    if (!extra_codes) rule.reads = choose({1, 2});
   } else if (!pd) {
-    double reads = 0;
-    for (const Work& w : work) reads += w.tasks;
-    const int most = cfg.double_precision ? 2 : kQuadReads;
-    rule.quads = reads_steps / most >= kFullSteps * warps && (!cfg.double_precision || reads / 2 >= kPairTasks * warps);
-    if (rule.quads) reads_per_warp = most;
+    rule.reads = choose({1, 2, kQuadReads});
   }
-  for (Work& w : work) w.tasks = std::ceil(w.tasks / reads_per_warp);
+  for (Work& w : work) w.tasks = count(w, rule.reads).tasks;
   double total = 0, best = -1;
   for (const Work& w : work) total += w.steps * w.tasks;
   for (const double part : {16.0, 4.0, 2.0, 1.4, 1.0, 0.7, 0.5, 0.25, 0.1, 0.02}) {
@@ -829,11 +878,11 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
     } else if (pd) {
       // PD in FP32: reads above 248 bases one per warp, the others in pairs (FP32x2) unless the
       // launch configuration asks for one read per warp.
-      for (; i < order.size() && (packed_rows(len_of(order[i])) > 8 || split.pd_reads == 1); ++i)
+      for (; i < order.size() && (packed_rows(len_of(order[i])) > 8 || split.reads == 1); ++i)
         one(Kind::kOneF32Pd, single_rows(len_of(order[i])), i);
       for (; i < order.size(); i += 2) two(Kind::kPackedF32Pd, packed_rows(len_of(order[i])), i);
     } else if (cfg.double_precision || plans[g].extra_codes) {
-      const bool pairs_fit = cfg.double_precision && split.quads && !extra_codes;
+      const bool pairs_fit = cfg.double_precision && split.reads == 2;
       for (; i < order.size() && !(pairs_fit && len_of(order[i]) <= kQuadMaxRead); ++i) one(f64, single_rows(len_of(order[i])), i);
       for (; i < order.size(); i += 2) quad(Kind::kPairF64, i, 2);
     } else {
@@ -843,7 +892,16 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       auto single_up = [&](int rows) { return up && rows + 2 <= max_rows(Kind::kOneF32) ? rows + 2 : rows; };  // even, 10..20
       auto short_up = [&](int rows) { return up && rows < 8 ? rows + 1 : rows; };
       for (; i < order.size() && packed_rows(len_of(order[i])) > 8; ++i) one(Kind::kOneF32, single_up(single_rows(len_of(order[i]))), i);
-      for (; i < order.size() && (!split.quads || len_of(order[i]) > kQuadMaxRead); ++i) one(Kind::kShortF32, short_up(packed_rows(len_of(order[i]))), i);
+      // Shorter ones by the batch's form, in a batch of quads those too long for it in pairs or alone.
+      const auto fits = [&](size_t k) { return split.reads == kQuadReads && len_of(order[k]) <= kQuadMaxRead; };
+      const bool pairs = split.reads == 2 || (split.reads == kQuadReads && split.mid_pairs);
+      while (i < order.size() && !fits(i)) {
+        if (pairs)
+          two(Kind::kPackedF32, short_up(packed_rows(len_of(order[i]))), i);
+        else
+          one(Kind::kShortF32, short_up(packed_rows(len_of(order[i]))), i);
+        i += pairs ? 2 : 1;
+      }
       for (; i < order.size(); i += kQuadReads) quad(Kind::kQuadF32, i, kQuadReads);
     }
   });
@@ -897,7 +955,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
         tasks.push_back(e.second);
         cost += e.first;
       }
-      const bool fp32 = b.kind == Kind::kShortF32 || b.kind == Kind::kOneF32 || b.kind == Kind::kPackedF32Pd || b.kind == Kind::kOneF32Pd;
+      const bool fp32 = b.kind == Kind::kShortF32 || b.kind == Kind::kPackedF32 || b.kind == Kind::kOneF32 || b.kind == Kind::kPackedF32Pd || b.kind == Kind::kOneF32Pd;
       const bool pipelined = is_long(b.kind);
       b.warps = pipelined ? long_warps(bl.row_blocks) : (fp32 ? tuning_.warps_per_block : kWarpsPerBlock);
       int per_sm = 0, threads = 0;

@@ -134,7 +134,7 @@ class Engine {
   // over (1: one after another; more: bins overlap, the largest first), each first-pass persistent
   // grid as a percentage of the resident-block limit, how many reads an FP32 PD-HMM warp carries
   // (two in FP32x2 at 8 warps per SM, or one at 12), and the first pass's tile shape: rows per lane
-  // of the plain FP32 reads that go one to a warp (the fewest that hold the read, or the next the
+  // of the plain FP32 reads that go one or two to a warp (the fewest that hold the read, or the next the
   // kernels instantiate) and warps per block of the FP32 first-pass kernels but the quad form's. None changes a result bit. Applies from the
   // next prepare().
   struct Tuning {
@@ -165,8 +165,10 @@ class Engine {
   };
   // The first pass's forms, and the steps above which a region's program is split.
   struct SplitRule {
-    bool quads = false;         // plain reads of at most kQuadMaxRead bases go kQuadReads to a warp, in FP64 two
-    int pd_reads = 1;           // FP32 PD-HMM reads of at most 248 bases a warp
+    // Reads a warp: in FP32 2 of at most 248 bases, or, plain, kQuadReads of at most kQuadMaxRead; in FP64,
+    // plain, 2 of at most kQuadMaxRead.
+    int reads = 1;
+    bool mid_pairs = false;  // with quads, the FP32 reads of up to 248 bases too long for them: two a warp
     uint64_t limit = ~uint64_t{0};
     int chunks(const ForwardPlan& p) const;
   };
@@ -174,10 +176,17 @@ class Engine {
   // about two haplotypes'. With 16 uneven regions (1,400 steps) four reads a warp and one read a warp
   // take the same time (0.78 and 0.76 ms); with 1,024, 29.6 and 41.2 ms.
   static constexpr double kFullSteps = 600;
-  // And in FP64 the share of the resident warps that two reads a warp must give a task: with 800 tasks of
+  // And the share of the resident warps that two plain reads a warp must give a task. In FP64: with 800 tasks of
   // long programs for 1,184 warps (8 regions of 200 reads x 128 SNP haplotypes) 2.81 ms against 2.63 at one
-  // read a warp; with 1,024 (8 uneven regions) 1.32 against 1.50, with 1,600 4.35 against 4.85.
-  static constexpr double kPairTasks = 0.8;
+  // read a warp; with 1,024 (8 uneven regions) 1.32 against 1.50, with 1,600 4.35 against 4.85. In FP32: with
+  // 1,080 tasks (40 regions of 54 reads) of 100, 151 and 230 bases 0.67, 0.71 and 1.08 ms against 0.55, 0.67
+  // and 1.11; with 1,728 0.73, 0.88 and 1.51 against 0.89, 1.01 and 1.59.
+  // With 432 tasks (16 regions of 54 reads of 230 bases) 0.63 ms against 0.57.
+  static constexpr double kF64PairTasks = 0.8, kPairTasks = 1.0;
+  // Time a step of a task with several reads takes, in steps of one read's in the same precision and model
+  // (6,000 regions, 5 rows per lane, 10 in the forms on 16 lanes: one FP32 read a warp 0.231 us a task, two
+  // 0.392, four 0.644 to 0.70; one FP64 read 0.32, two 0.52; one PD-HMM read 0.33, two 0.57).
+  static constexpr double kPairCost = 1.7, kQuadCost = 2.9, kF64PairCost = 1.6, kPdPairCost = 1.75;
   // Reads, and regions, a resident warp from which hardly any region is split.
   static constexpr int64_t kWholeReads = 8, kWholeRegions = 2;
   SplitRule choose_split(const BatchInput& in, const EngineConfig& cfg, const std::vector<int64_t>& first_read,

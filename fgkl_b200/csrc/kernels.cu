@@ -273,6 +273,20 @@ auto dispatch(Kind k, int rows, Args&&... args) -> decltype(F<OneF32, 1>::run(ar
           break;
       }
       break;
+    case Kind::kPackedF32:
+      switch (rows) {
+        FGKL_CASE(PackedF32, 1)
+        FGKL_CASE(PackedF32, 2)
+        FGKL_CASE(PackedF32, 3)
+        FGKL_CASE(PackedF32, 4)
+        FGKL_CASE(PackedF32, 5)
+        FGKL_CASE(PackedF32, 6)
+        FGKL_CASE(PackedF32, 7)
+        FGKL_CASE(PackedF32, 8)
+        default:
+          break;
+      }
+      break;
     case Kind::kOneF32:
       switch (rows) {
         FGKL_CASE(OneF32, 10)
@@ -343,6 +357,7 @@ bool valid_rows(Kind k, int rows) {
   if (is_long(k)) return valid_long_rows(k, rows);
   switch (k) {
     case Kind::kShortF32:
+    case Kind::kPackedF32:
       return rows >= 1 && rows <= 8;
     case Kind::kQuadF32:
     case Kind::kPairF64:

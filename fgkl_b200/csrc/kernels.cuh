@@ -27,8 +27,9 @@ enum class Kind : int {
   kQuadF32 = 12,   // up to four reads, two on each half of the lanes in FP32x2, rows-per-lane 2..14 (even)
   kOneF64Codes = 13,  // as kOneF64, priors by comparing haplotype codes (bytes other than A, C, G, T and N)
   kPairF64 = 14,   // up to two reads, one on each half of the lanes in FP64, priors from a table, the quad form's rows
+  kPackedF32 = 15,  // two reads of at most 248 bases on all lanes in FP32x2, rows-per-lane 1..8
 };
-constexpr int kNumKinds = 15;
+constexpr int kNumKinds = 16;
 // Lanes that hold two reads (FP32x2) or one (FP64) in the quad form, reads a warp in FP32x2, its largest rows-per-lane and its longest
 // read (the first row of the first lane is padding).
 constexpr int kQuadLanes = 16, kQuadReads = 4;

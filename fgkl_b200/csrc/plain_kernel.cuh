@@ -13,13 +13,15 @@
 // (two shuffles a step instead of the bottom row's M, X and Y, and no above-row state to keep, store in
 // snapshots or reload).
 //
-// Two forms. One read on all 32 lanes (G = 32) has the shortest steps and serves small batches, long reads
+// Three forms. One read on all 32 lanes (G = 32) has the shortest steps and serves small batches, long reads
 // and the recomputation. Four reads on two groups of 16 lanes in FP32x2 (the quad form) have half the steps that an
 // event spans and half the shuffles, selects and loop overhead a cell; at R = 10 they need 255 registers
 // and 21 KB of shared memory a warp, 8 warps an SM. Measured on 54,000 reads of 151 bases (1,024 uneven
 // regions): 20.5 ms, 2,750 G cells/s (the FP32 pipe 58% active without events, where it reaches 4,080);
 // two reads on 32 lanes in FP32x2 26.6 ms; two on 16 lanes in scalar FP32 at 16 warps an SM 23.2 ms; four
-// on 8 lanes in scalar FP32 23.3 ms.
+// on 8 lanes in scalar FP32 23.3 ms. Two reads on 32 lanes serve full batches where the quad form does not
+// fit: regions whose reads leave its slots empty, and reads of 224 to 248 bases (512 regions of 54 reads of
+// 236 bases: 9.8 ms, one a warp 10.4).
 // In FP64 the same form holds two reads, one on each half of the lanes.
 //
 // Forward recurrence per cell (GATK LoglessPairHMM, fgkl kernel.rs:1011-1013):
@@ -266,6 +268,7 @@ constexpr int block_warps() {
 // registers of 8 warps an SM (238 at 10 rows): 128 uneven regions 8.6 -> 7.5 ms, 128 of 128 SNP haplotypes
 // 35.1 -> 28.6 ms.
 constexpr int f64_min_blocks(int rows, bool table) { return rows <= (table ? 6 : 5) ? 3 : 1; }
+// Two FP32 reads on 32 lanes: four blocks up to 4 rows, three up to 7, two at 8.
 template <class P, int R, int G>
 struct MinBlocks {
   static constexpr int kRegs = (7 * R * P::NC + 42) > 255 ? 255 : 7 * R * P::NC + 42;
@@ -273,7 +276,8 @@ struct MinBlocks {
   // A quarter of the SM's registers serves a quarter of its warps.
   static constexpr int kByRegs = 2 * (512 / ((kRegs + 7) / 8 * 8));
   static constexpr int kQuad = kByRegs < kBySmem ? kByRegs : kBySmem;
-  static constexpr int value = G < 32 ? (P::kDouble ? 4 : (kQuad > 12 ? 12 : kQuad)) : (P::kDouble ? f64_min_blocks(R, P::kTable) : (R <= 8 ? 4 : 2));
+  static constexpr int kPair = R <= 4 ? 4 : (R <= 7 ? 3 : 2);
+  static constexpr int value = G < 32 ? (P::kDouble ? 4 : (kQuad > 12 ? 12 : kQuad)) : (P::kDouble ? f64_min_blocks(R, P::kTable) : P::NC == 2 ? kPair : (R <= 8 ? 4 : 2));
 };
 
 // ---------------------------------------------------------------------------------------------

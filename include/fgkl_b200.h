@@ -198,7 +198,7 @@ typedef struct fgkl_tuning {
   int32_t grid_percent;     /* each first-pass persistent grid, % of the kernel's resident-block limit, 10-100 */
   int32_t reads_per_warp;   /* FP32 PD-HMM reads of at most 248 bases: 2 (FP32x2 pairs, the default, where
                                the batch fills the GPU with them) or 1 */
-  int32_t rows_extra;       /* tile shape: 1 runs plain FP32 reads that go one to a warp one rows-per-lane
+  int32_t rows_extra;       /* tile shape: 1 runs plain FP32 reads that go one or two to a warp one rows-per-lane
                                step above the fewest that hold them (0, the default: the fewest) */
   int32_t warps_per_block;  /* tile shape: warps per block of the FP32 first-pass kernels (other than the one
                                with four reads a warp), 1, 2 or 4 (default) */
@@ -225,7 +225,7 @@ int fgkl_context_get_tuning(const fgkl_context* ctx, fgkl_tuning* tuning);
  * events around each, so each is timed alone; fgkl_batch_launch_profile
  * waits and reports every first-pass and recomputation launch of the last run: kernel kind
  * (0 FP32 for reads of at most 248 bases, 1 FP32, 2 FP64, 3 PD FP32, 4 PD FP64, 5 PD packed FP32, 12
- * FP32 with four reads a warp, 13 FP64 comparing codes, 14 FP64 with two reads a warp; strip-mined: 6
+ * FP32 with four reads a warp, 13 FP64 comparing codes, 14 FP64 with two reads a warp, 15 FP32 with two; strip-mined: 6
  * FP32, 7 FP64, 8 PD FP32, 9 PD FP64, 10 and 11 byte-compared PD FP32 and FP64), rows per lane, tasks,
  * blocks, whether it is a recomputation launch, the forward and backward DP cells its tasks compute, and its duration. */
 typedef struct fgkl_launch_profile {

@@ -41,3 +41,58 @@ def test_a_long_region_among_very_many_is_planned_again_and_split(gpu, pd):
     assert sum(p["tasks"] for p in launches(ctx)) > 2399 + 7  # the long region's reads have several tasks each
     for g in (0, 1699, 1700, 1701, 2399):
         same_as_alone(w, out, g, FLOAT, pd)
+
+
+def regions_of(lens, haps, hap_len, n):
+    """`n` regions of reads of `lens[i % len(lens)]` bases, from 40 different ones."""
+    made = []
+    for s in range(40):
+        reads, hs = [], None
+        for i, m in enumerate(lens[s % len(lens)]):
+            r, h = synthetic.reference_region(300 + s, i + 1, m, haps, hap_len).region(0)
+            hs = hs or h  # one seed, one haplotype set
+            reads.append(r[i])
+        made.append((reads, hs))
+    return [made[i % 40] for i in range(n)]
+
+
+@pytest.mark.parametrize("precision,reads,kind", [
+    (Precision.FLOAT, 1, 0), (Precision.FLOAT, 2, 15), (Precision.FLOAT, 3, 12), (Precision.FLOAT, 6, 15), (Precision.FLOAT, 8, 12),
+    (Precision.DOUBLE, 1, 2), (Precision.DOUBLE, 2, 14), (Precision.DOUBLE, 3, 2)])
+def test_full_batches_of_small_regions_take_the_form_that_their_reads_fill(gpu, precision, reads, kind):
+    """Only reads of one region share a warp: a region of one read leaves three quarters of a four-read
+    task empty, and one of two reads half."""
+    cfg = Config(precision=precision)
+    w = synthetic.from_regions(regions_of([(151,) * reads], 12, 300, 1300))
+    ctx = BatchContext()
+    ctx.set_profiling(True)
+    out, _ = ctx.compute(w, cfg)
+    assert {p["kind"] for p in launches(ctx)} == {kind}
+    for g in (0, 17, 39):
+        same_as_alone(w, out, g, cfg)
+
+
+def test_two_reads_a_warp_at_the_edges_of_its_rows(gpu):
+    edges = [1, 2] + [31 * r + d for r in range(1, 9) for d in (-1, 0, 1) if 31 * r + d <= 248]
+    lens = [(edges[i % len(edges)], edges[(7 * i + 3) % len(edges)]) for i in range(40)]
+    w = synthetic.from_regions(regions_of(lens, 16, 320, 1300))
+    ctx = BatchContext()
+    ctx.set_profiling(True)
+    out, _ = ctx.compute(w, FLOAT)
+    assert {p["kind"] for p in launches(ctx)} == {15} and {p["rows"] for p in launches(ctx)} == set(range(1, 9))
+    for g in range(40):
+        same_as_alone(w, out, g, FLOAT)
+
+
+@pytest.mark.parametrize("n_regions,kind", [(160, 0), (700, 15)])
+def test_reads_too_long_for_four_a_warp_go_beside_them(gpu, n_regions, kind):
+    """Alone where there are few in the batch, in pairs where there are many (an odd one of a region with a
+    shorter read)."""
+    lens = [(100,) * 20 + (224,) * 7 + (248,) * 6, (223,) * 9 + (249,) * 3 + (240,)]
+    w = synthetic.from_regions(regions_of(lens, 16, 320, n_regions))
+    ctx = BatchContext()
+    ctx.set_profiling(True)
+    out, _ = ctx.compute(w, FLOAT)
+    assert {p["kind"] for p in launches(ctx)} == {12, kind, 1}
+    for g in (0, 1, 38, 39):
+        same_as_alone(w, out, g, FLOAT)
