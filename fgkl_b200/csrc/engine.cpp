@@ -305,6 +305,57 @@ void parallel_for(int64_t n, int threads, F&& fn) {
 
 int host_threads() { return std::max(1, static_cast<int>(std::thread::hardware_concurrency())); }
 
+// The pairs of a strip-mined launch, by their numbers of row blocks.
+struct LongPairs {
+  struct Of {  // the pairs of one number of row blocks
+    double pairs = 0, columns = 0, longest = 0;
+  };
+  std::vector<Of> by_blocks;
+  void add(int blocks, int columns) {
+    const size_t at = static_cast<size_t>(std::min(blocks, 4095));  // beyond it all the same
+    if (at >= by_blocks.size()) by_blocks.resize(at + 1);
+    Of& o = by_blocks[at];
+    o.pairs += 1;
+    o.columns += columns;
+    o.longest = std::max(o.longest, static_cast<double>(columns));
+  }
+};
+
+// Warps a block of a strip-mined launch of these pairs, on `sms` SMs. A pair's row blocks on W warps take
+// ceil(blocks / W) rounds of n + 32 + 64 (W - 1) steps: more warps shorten a pair, fewer waste no steps on
+// starting one behind another, nor on rounds that they do not fill. The W with the smallest estimate -- the larger
+// of the warps' steps in all at the rate of a busy GPU and the longest pair --, the fewest among equals; a busy
+// SM's rate is that of 8 warps (in FP64 of 4.5, one a scheduler and a little). Passes over 6 haplotypes a
+// region, 8 warps a block or a read's row blocks, and as chosen: 32 regions of 48 reads of 1,000 bases, PD, the
+// FP32 pass 28.9 -> 12.2 ms; 64 regions, plain, 10.3 -> 8.8; 64 regions of reads of 640 bases beside one of
+// 3,200, both passes, 8.7 -> 6.4.
+int choose_long_warps(Kind kind, int rows, int sms, const LongPairs& of) {
+  const int blocks = static_cast<int>(of.by_blocks.size()) - 1, most = blocks > kLongWarps ? kLongWarps : std::max(1, blocks);
+  const bool f64 = kind == Kind::kLongF64 || kind == Kind::kLongF64Pd || kind == Kind::kGenericF64Pd;
+  const double kBusy = f64 ? 4.5 : 8.0;
+  int best = 1;
+  double least = -1;
+  for (int w = 1; w <= most; ++w) {
+    int per_sm = 0, threads = 0;
+    long_occupancy(kind, rows, &per_sm, &threads, w);
+    if (per_sm <= 0) continue;
+    double sum = 0, longest = 0;
+    for (int b = 1; b <= blocks; ++b) {
+      const LongPairs::Of& o = of.by_blocks[static_cast<size_t>(b)];
+      if (o.pairs == 0) continue;
+      const double rounds = (b + w - 1) / w, fill = 32 + 64 * (std::min(w, b) - 1);
+      sum += rounds * (o.columns + o.pairs * fill) * w;
+      longest = std::max(longest, rounds * (o.longest + fill));
+    }
+    const double time = std::max(sum / (sms * std::min(kBusy, static_cast<double>(per_sm * w))), longest);
+    if (least < 0 || time < least) {
+      least = time;
+      best = w;
+    }
+  }
+  return best;
+}
+
 // Copies `bytes` bytes in `chunks` pieces on several threads.
 void parallel_copy(uint8_t* dst, const uint8_t* src, size_t bytes) {
   constexpr size_t kChunk = size_t{4} << 20;
@@ -798,7 +849,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   struct BinList {
     std::vector<std::pair<uint64_t, Task>> list;
     uint64_t fwd_cells = 0, bwd_cells = 0;  // forward, backward DP cells
-    int row_blocks = 0;                     // strip-mined: the most a read has
+    LongPairs pairs;                        // strip-mined
   };
   std::vector<BinList> by_bin(static_cast<size_t>(kKinds) * kBinRows);
   auto bin_at = [&](Kind kind, int rows) -> BinList& { return by_bin[static_cast<size_t>(kind) * kBinRows + rows]; };
@@ -919,7 +970,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       if (t.task.hap >= 0) {
         // An unshared strip-mined pair: read length x haplotype length forward cells.
         bl.list.push_back({t.cost, t.task});
-        bl.row_blocks = std::max(bl.row_blocks, long_blocks(t.len, t.rows));
+        bl.pairs.add(long_blocks(t.len, t.rows), static_cast<int>(rp.haps[t.task.hap].len));
         bl.fwd_cells += static_cast<uint64_t>(rp.haps[t.task.hap].len) * static_cast<uint64_t>(t.len);
         continue;
       }
@@ -957,7 +1008,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       }
       const bool fp32 = b.kind == Kind::kShortF32 || b.kind == Kind::kPackedF32 || b.kind == Kind::kOneF32 || b.kind == Kind::kPackedF32Pd || b.kind == Kind::kOneF32Pd;
       const bool pipelined = is_long(b.kind);
-      b.warps = pipelined ? long_warps(bl.row_blocks) : (fp32 ? tuning_.warps_per_block : kWarpsPerBlock);
+      b.warps = pipelined ? choose_long_warps(b.kind, b.rows, sms_, bl.pairs) : (fp32 ? tuning_.warps_per_block : kWarpsPerBlock);
       int per_sm = 0, threads = 0;
       occupancy(b.kind, b.rows, &per_sm, &threads, b.warps);
       b.warps = threads / 32;

@@ -64,7 +64,7 @@ __host__ __device__ inline int long_rows(int len, bool wide) {
   return best;
 }
 __host__ __device__ inline int long_blocks(int len, int rows) { return (len + 32 * rows - 1) / (32 * rows); }
-// Warps a block of the plain strip-mined kernels: one a row block up to kLongWarps; more row blocks run in
+// Warps a block of the strip-mined kernels at most: one a row block up to kLongWarps; more row blocks run in
 // rounds of about equal size.
 constexpr int kLongWarps = 8;
 inline int long_warps(int row_blocks) {

@@ -96,3 +96,24 @@ def test_reads_too_long_for_four_a_warp_go_beside_them(gpu, n_regions, kind):
     assert {p["kind"] for p in launches(ctx)} == {12, kind, 1}
     for g in (0, 1, 38, 39):
         same_as_alone(w, out, g, FLOAT)
+
+
+@pytest.mark.parametrize("pd", [False, True])
+@pytest.mark.parametrize("precision", [Precision.FLOAT, Precision.DOUBLE])
+def test_long_reads_of_a_full_batch_keep_the_bits_of_a_call(gpu, pd, precision):
+    """Many pairs of long reads run on one warp each, their row blocks in rounds; a call's few pairs run them on
+    several warps."""
+    cfg = Config(precision=precision)
+    make = synthetic.reference_pd_region if pd else synthetic.reference_region
+    made = []
+    for s, n in enumerate((625, 641, 1030, 2100)):
+        reads, haps = make(700 + s, 24, n, 3, n + 80).region(0)
+        made.append(([r for r in reads if len(r.bases) > 620][:9] or reads[:2], haps))
+    w = synthetic.from_regions([made[i % 4] for i in range(160)])
+    out, _ = BatchContext().compute(w, cfg)
+    offs = w.output_offsets()
+    for g in (0, 1, 2, 3, 156, 159):
+        reads, haps = made[g % 4]
+        alone = (PdPairHmm if pd else PairHmm)(cfg).compute_log10_likelihoods(reads[:1], haps)
+        assert alone.tobytes() == out[offs[g]:offs[g] + len(haps)].tobytes()
+        assert np.max(np.abs(alone.reshape(-1) - O.compute_matrix(reads[:1], haps).reshape(-1))) < TOL[precision]
