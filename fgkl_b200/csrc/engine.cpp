@@ -671,6 +671,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   DeviceGuard device_guard(device_);
   const auto t_start = std::chrono::steady_clock::now();
   cfg_ = cfg;
+  pd_ = in.hap_flags != nullptr;
   error_.clear();
   planned_ = BatchStats{};
   bins_.clear();
@@ -780,8 +781,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   int64_t n_haps = 0, n_stream = kStreamPad, n_segs = 0, n_sweeps = 0, n_seq = 0, n_pd_seq = 0, n_sigs = 0;
   int max_slots = 1, max_nodes = 1, max_segs = 1;
   std::vector<int64_t> queue_cap(kQueueBins, 0);
-  int max_read_len = 1;
-  for (int64_t r = 0; r < total_reads; ++r) max_read_len = std::max(max_read_len, static_cast<int>(in.read_off[r + 1] - in.read_off[r]));
+  std::vector<int> queue_len(kQueueBins, 1);  // the longest read of each bin
   int max_hap_len = 1;  // scratch of the strip-mined kinds: one carry column per haplotype base
   for (int g = 0; g < N; ++g) {
     const RegionPlan& rp = plans[g];
@@ -832,11 +832,18 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
     if (rp.n_distinct > 0)
       for (int64_t r = first_read[g]; r < first_read[g + 1]; ++r) {
         const int len = static_cast<int>(in.read_off[r + 1] - in.read_off[r]);
-        const int bin = queue_bin(len, rp.generic), pair_bin = queue_pair_bin(len, rp.generic);
-        queue_cap[bin] += rp.n_distinct;
-        if (pair_bin != bin) queue_cap[pair_bin] += rp.n_distinct;
+        const int bin = queue_bin(len, rp.generic);
+        for (const bool few : {false, true}) {
+          const int pair_bin = queue_pair_bin(len, rp.generic, pd, few);
+          if (few && queue_bin_group(pair_bin) < 3) continue;  // the same bin either way
+          queue_cap[pair_bin] += rp.n_distinct;
+          queue_len[pair_bin] = std::max(queue_len[pair_bin], len);
+        }
+        // Whole-program tasks, where single pairs go to another bin.
+        if (queue_bin_group(bin) == 0 && queue_pair_bin(len, rp.generic, pd, false) != bin) queue_cap[bin] += static_cast<int64_t>(rp.progs.size());
       }
   }
+  for (int q = 3 * kRowBins; q < kQueueBins; ++q) queue_cap[q] = std::min<int64_t>(queue_cap[q], few_pairs_most(sms_));
   if (n_stream > INT32_MAX || n_seq > INT32_MAX || n_pd_seq > INT32_MAX || n_haps > INT32_MAX)
     return fail(FGKL_E_INVALID_ARGUMENT, "batch too large for 32-bit plan offsets; split it");
 
@@ -1041,17 +1048,22 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
     queue_off[kQueueBins] = static_cast<int>(acc);
   }
   if (queue_on) {
-    for (int q = 1; q < kQueueBins; ++q) {
+    // The bins of several warps a pair first: their pairs take the longest.
+    for (int i = 0; i < kQueueBins; ++i) {
+      const int q = (i + 3 * kRowBins) % kQueueBins;
       const int cap = queue_off[q + 1] - queue_off[q];
       if (cap == 0) continue;
       // Queue bin -> the FP64 form of the pairs it holds (queue_bin).
       const int r = queue_bin_rows(q);
-      const Kind kind = q >= 2 * kRowBins ? Kind::kGenericF64Pd
-                                          : (q >= kRowBins ? (pd ? Kind::kLongF64Pd : Kind::kLongF64) : (pd ? Kind::kOneF64Pd : f64));
+      const int group = queue_bin_group(q);
+      const Kind kind = group == 0 ? (pd ? Kind::kOneF64Pd : f64)
+                                   : (group == 2 || group == 4 ? Kind::kGenericF64Pd : (pd ? Kind::kLongF64Pd : Kind::kLongF64));
       int per_sm = 0, threads = 0;
       const bool pipelined = is_long(kind);
       Bin b{kind, r, queue_off[q], cap, 0, 0, 0};
-      if (pipelined) b.warps = long_warps(long_blocks(max_read_len, r));
+      // Many pairs: two warps a pair, so that the longest does not run on alone for long (1,000 pairs of 700
+      // bases 1.62 ms against 1.45 at one, 300 of 1,200 bases 1.86 against 2.25), one for short ones.
+      if (pipelined) b.warps = group < 3 ? (long_blocks(queue_len[q], r) > (group == 1 ? 2 : 4) ? 2 : 1) : long_warps(long_blocks(queue_len[q], r));
       occupancy(kind, r, &per_sm, &threads, b.warps);
       if (per_sm <= 0) return fail(FGKL_E_CUDA, "recomputation kernel unavailable on this device");
       b.queue_bin = q;
@@ -1279,7 +1291,7 @@ int Engine::run() {
   };
   if ((rc = pass(bins_, false))) return rc;
   if (!rescue_bins_.empty()) {
-    CollectArgs c{view_, d_queue_, queue_off_, queue_tail, cfg_.double_precision ? 0 : 1};
+    CollectArgs c{view_, d_queue_, queue_off_, queue_tail, cfg_.double_precision ? 0 : 1, pd_ ? 1 : 0, sms_};
     if ((rc = check(launch_collect(c, n_regions_, stream_), "lost-pair collection"))) return rc;
     planned_.kernel_launches++;
   }

@@ -211,6 +211,7 @@ class Engine {
   cudaEvent_t fork_ = nullptr;
   std::string error_;
   EngineConfig cfg_;
+  bool pd_ = false;  // the prepared batch is PD-HMM
   BatchStats planned_;
 
   // Device buffers (grow-only).

@@ -13,6 +13,14 @@ namespace fgkl {
 
 namespace {
 
+// Queues a lost pair in a bin; whether the bin had room.
+__device__ __forceinline__ bool queue_pair(const CollectArgs& a, int bin, int read, int hap, int prog) {
+  const int slot = atomicAdd(a.queue_tail + bin, 1);
+  if (slot >= a.queue_off[bin + 1] - a.queue_off[bin]) return false;
+  a.queue[a.queue_off[bin] + slot] = Task{static_cast<int32_t>(blockIdx.x), {read, -1, -1, -1}, queue_bin_rows(bin), hap, prog};
+  return true;
+}
+
 // Queues what the first pass lost for FP64 recomputation, in the queue bin of the read's form and
 // rows-per-lane (queue_bin), one warp per read. After an FP32 pass, a read of a shared program lost
 // against at least a third of its haplotypes (duplicates counted, fgkl lib.rs:495-505) is queued once,
@@ -24,6 +32,7 @@ __global__ void __launch_bounds__(256) collect_kernel(CollectArgs a) {
   if (a.v.counters->lost_pairs == 0) return;
   const Region region = a.v.regions[blockIdx.x];
   const bool generic = (region.flags & kRegionGeneric) != 0;
+  const unsigned long long lost_wide = a.v.counters->lost_wide;
   const int lane = threadIdx.x & 31;
   for (int r = threadIdx.x >> 5; r < region.n_reads; r += blockDim.x >> 5) {
     const double* row = a.v.out + region.out_off + static_cast<int64_t>(r) * region.n_haps;
@@ -60,17 +69,20 @@ __global__ void __launch_bounds__(256) collect_kernel(CollectArgs a) {
       if (lane == 0) atomicAdd(&a.v.counters->rescue_reads, static_cast<unsigned long long>(lost_distinct));
       continue;
     }
-    const int pair_bin = queue_pair_bin(len, generic);
-    const int pair_cap = a.queue_off[pair_bin + 1] - a.queue_off[pair_bin];
+    // Where many are lost, the longest reads' pairs go to several warps each all the same, as many as those
+    // bins hold: on one warp such a pair runs on by itself when the others are done.
+    const int wide_bin = queue_pair_bin(len, generic, a.pd != 0, true);
+    const bool grouped = queue_bin_group(wide_bin) >= 3;
+    const int row_blocks = long_blocks(len, queue_bin_rows(wide_bin));
+    const bool few = lost_wide <= static_cast<unsigned long long>(few_pairs(a.sms, row_blocks));
+    const bool longest = !few && grouped && row_blocks > kLongWarps;
+    const int pair_bin = few || !grouped ? wide_bin : queue_pair_bin(len, generic, a.pd != 0, false);
     for (int k = lane; k < region.n_haps; k += 32) {
       const HapInfo info = a.v.haps[region.hap_off + k];
       if (info.src != k || !isnan(row[info.order])) continue;
-      const int slot = atomicAdd(a.queue_tail + pair_bin, 1);
-      if (slot < pair_cap) {
-        a.queue[a.queue_off[pair_bin] + slot] =
-            Task{static_cast<int32_t>(blockIdx.x), {read, -1, -1, -1}, queue_bin_rows(pair_bin), k, region.prog};
-        atomicAdd(&a.v.counters->rescue_reads, 1ull);
-      }
+      bool queued = longest && queue_pair(a, wide_bin, read, k, region.prog);
+      if (!queued) queued = queue_pair(a, pair_bin, read, k, region.prog);
+      if (queued) atomicAdd(&a.v.counters->rescue_reads, 1ull);
     }
   }
 }
@@ -213,7 +225,10 @@ __global__ void __launch_bounds__(kLongWarps * 32, (P::kDouble || R > 12 ? 1 : 2
         a.v.out[region.out_off + static_cast<int64_t>(read_local) * region.n_haps + h.order] = result;
         lost_count += lost;
       }
-      if (lost_count) atomicAdd(&a.v.counters->lost_pairs, lost_count);
+      if (lost_count) {
+        atomicAdd(&a.v.counters->lost_pairs, lost_count);
+        atomicAdd(&a.v.counters->lost_wide, lost_count);
+      }
     }
     __syncthreads();
   }

@@ -52,13 +52,15 @@ __host__ __device__ constexpr int long_rows_count(bool wide) { return wide ? 4 :
 // padding rows (ties: the smaller). Blocks = ceil(len / (32 * R)). `wide`: the plain FP32 kind.
 __host__ __device__ inline int long_rows(int len, bool wide) {
   int best = 8;
-  long long best_rows = -1;
-  for (int i = 0; i < long_rows_count(wide); ++i) {
-    const int r = long_rows_value(i, wide);
-    const long long rows = (static_cast<long long>(len) + 32 * r - 1) / (32 * r) * (32 * r);
-    if (best_rows < 0 || rows < best_rows) {
+  unsigned best_rows = 0;
+#pragma unroll
+  for (int i = 0; i < kNumLongRows; ++i) {
+    if (i >= long_rows_count(wide)) break;
+    const unsigned r = static_cast<unsigned>(long_rows_value(i, wide));
+    const unsigned rows = (static_cast<unsigned>(len) + 32 * r - 1) / (32 * r) * (32 * r);
+    if (best_rows == 0 || rows < best_rows) {
       best_rows = rows;
-      best = r;
+      best = static_cast<int>(r);
     }
   }
   return best;
@@ -72,10 +74,12 @@ inline int long_warps(int row_blocks) {
   return rounds > 0 ? (row_blocks + rounds - 1) / rounds : 1;
 }
 
-// Recomputation queue bins: rows-per-lane 1..20 of single-block reads, then kRowBins + R for
-// strip-mined reads and 2 * kRowBins + R for the pairs of byte-compared PD regions.
+// Recomputation queue bins, by group and rows-per-lane: reads whose rows one warp holds (0), strip-mined on
+// one or two warps a pair (1; 2 for the pairs of byte-compared PD regions), and strip-mined on a warp a row
+// block, for the runs that lose few pairs (3, and 4 byte-compared).
 constexpr int kRowBins = 21;
-constexpr int kQueueBins = 3 * kRowBins;
+constexpr int kQueueGroups = 5;
+constexpr int kQueueBins = kQueueGroups * kRowBins;
 __host__ __device__ inline int queue_bin(int len, bool generic) {
   if (generic) return 2 * kRowBins + long_rows(len, false);
   if (len > kMaxBlockRead) return kRowBins + long_rows(len, false);
@@ -84,13 +88,29 @@ __host__ __device__ inline int queue_bin(int len, bool generic) {
   return rows;
 }
 __host__ __device__ inline int queue_bin_rows(int bin) { return bin % kRowBins; }
-// The bin of a single lost pair of a read: as queue_bin up to 248 bases; above, the strip-mined form's, whose
-// row blocks run side by side on a few warps (one block of 10 to 20 rows a lane in FP64 spills registers and
-// is one warp's work). A read's whole-program tasks stay in queue_bin's.
-__host__ __device__ inline int queue_pair_bin(int len, bool generic) {
+__host__ __device__ inline int queue_bin_group(int bin) { return bin / kRowBins; }
+// The bin of a single lost pair of a read (a read's whole-program tasks are queue_bin's). `few`: the run lost few
+// pairs of reads above 248 bases (few_pairs), so that a pair's row blocks have warps to run side by side on;
+// else the warps are worth more on pairs of their own (1 pair of 540 bases 0.27 against 0.39 ms, 1,000 pairs
+// 1.05 against 0.87). In a single block 10 to 14 rows a lane of the plain FP64 form are the faster even then
+// (32 pairs of 350 bases: 0.17 against 0.18 ms); those of the PD form spill registers, and reads of 12 and
+// more, or that two strip-mined blocks hold with hardly any padding, go strip-mined even when many are lost
+// (1,000 pairs of 480 bases: 1.15 against 2.01 ms; 9,134 of 250 bases 3.2 against 4.5; but 5,977 of 300 bases,
+// padded to 384 rows, 3.2 against 3.0).
+__host__ __device__ inline int queue_pair_bin(int len, bool generic, bool pd, bool few) {
   const int bin = queue_bin(len, generic);
-  return bin < kRowBins && bin > 8 ? kRowBins + long_rows(len, false) : bin;
+  const int group = queue_bin_group(bin);
+  if (group == 0 && bin <= 8) return bin;
+  if (few && (group > 0 || bin >= (pd ? 10 : 16))) return (group == 2 ? 4 : 3) * kRowBins + long_rows(len, false);
+  return group == 0 && pd && (bin >= 12 || len <= 256) ? kRowBins + long_rows(len, false) : bin;
 }
+// Lost pairs of reads above 248 bases up to which they are few for a read of this many strip-mined row blocks:
+// with more, several warps a pair no longer pay (148 SMs: pairs of 700 bases 0.43 ms at six warps a pair and
+// 0.93 at one with 148 pairs, 0.69 and 0.94 with 200, 0.98 and 0.96 with 300; PD pairs of 250 bases at two
+// warps 0.29 against 0.37 at one with 400 pairs, 0.58 against 0.47 with 1,000).
+__host__ __device__ inline int few_pairs(int sms, int row_blocks) { return row_blocks <= 2 ? 4 * sms : sms + sms / 2; }
+// The most pairs that a bin of several warps a pair holds.
+inline int few_pairs_most(int sms) { return few_pairs(sms, 1); }
 
 inline bool is_long(Kind k) { return k >= Kind::kLongF32 && k <= Kind::kGenericF64Pd; }
 inline bool is_quad(Kind k) { return k == Kind::kQuadF32 || k == Kind::kPairF64; }
@@ -125,6 +145,8 @@ struct CollectArgs {
   int* queue_tail;       // per bin: tasks queued
   int dense;             // 1 after an FP32 pass: a read lost against a third of its haplotypes or more
                          // is queued once, as a whole-program FP64 task (fgkl lib.rs:495-520)
+  int pd;                // 1 in a PD-HMM batch
+  int sms;               // of the device (few_pairs)
 };
 
 // Rows per lane the instantiations cover.

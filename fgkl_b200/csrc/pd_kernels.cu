@@ -434,7 +434,10 @@ __device__ __forceinline__ void pd_finalize(const LaunchArgs& a, const Task& tas
       lost_count += lost;
     }
   }
-  if (lost_count && !dense) atomicAdd(&a.v.counters->lost_pairs, lost_count);
+  if (lost_count && !dense) {
+    atomicAdd(&a.v.counters->lost_pairs, lost_count);
+    if (R > 8) atomicAdd(&a.v.counters->lost_wide, lost_count);
+  }
 }
 
 // Resident blocks of 4 warps the register budget is cut for. Two reads a warp at 5 rows: three (168
@@ -635,7 +638,10 @@ __global__ void __launch_bounds__(kLongWarps * 32, 1) pd_long_kernel(LaunchArgs 
         a.v.out[region.out_off + static_cast<int64_t>(read_local) * region.n_haps + h.order] = result;
         lost_count += lost;
       }
-      if (lost_count) atomicAdd(&a.v.counters->lost_pairs, lost_count);
+      if (lost_count) {
+        atomicAdd(&a.v.counters->lost_pairs, lost_count);
+        atomicAdd(&a.v.counters->lost_wide, lost_count);
+      }
     }
     __syncthreads();
   }

@@ -720,7 +720,10 @@ __device__ __forceinline__ void finalize(const LaunchArgs& a, const Task& task, 
       lost_count += lost;
     }
   }
-  if (lost_count && !dense) atomicAdd(&a.v.counters->lost_pairs, lost_count);
+  if (lost_count && !dense) {
+    atomicAdd(&a.v.counters->lost_pairs, lost_count);
+    if (G == 32 && R > 8) atomicAdd(&a.v.counters->lost_wide, lost_count);
+  }
 }
 
 // One task at its R rows per lane.

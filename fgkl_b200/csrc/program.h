@@ -147,8 +147,9 @@ struct Task {
 // Per-pass counters written by the kernels.
 struct Counters {
   unsigned long long lost_pairs;   // pairs handed to the double-precision recomputation
+  unsigned long long lost_wide;    // those of them whose reads have more than 248 bases, or strip-mined
   unsigned long long rescue_reads; // (read, distinct haplotype) pairs queued for recomputation
-  unsigned long long pad_[2];
+  unsigned long long pad_;
 };
 
 // Flattened batch: everything a kernel needs, as device pointers.
