@@ -781,7 +781,9 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   int64_t n_haps = 0, n_stream = kStreamPad, n_segs = 0, n_sweeps = 0, n_seq = 0, n_pd_seq = 0, n_sigs = 0;
   int max_slots = 1, max_nodes = 1, max_segs = 1;
   std::vector<int64_t> queue_cap(kQueueBins, 0);
-  std::vector<int> queue_len(kQueueBins, 1);  // the longest read of each bin
+  std::vector<int64_t> many_cap(kQueueBins, 0);  // pairs of the bins that only a run losing many fills
+  std::vector<int> queue_len(kQueueBins, 1);     // the longest read of each bin
+  int64_t wide_pairs = 0;                        // what Counters::lost_wide counts, if all were lost
   int max_hap_len = 1;  // scratch of the strip-mined kinds: one carry column per haplotype base
   for (int g = 0; g < N; ++g) {
     const RegionPlan& rp = plans[g];
@@ -833,16 +835,19 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       for (int64_t r = first_read[g]; r < first_read[g + 1]; ++r) {
         const int len = static_cast<int>(in.read_off[r + 1] - in.read_off[r]);
         const int bin = queue_bin(len, rp.generic);
-        for (const bool few : {false, true}) {
-          const int pair_bin = queue_pair_bin(len, rp.generic, pd, few);
-          if (few && queue_bin_group(pair_bin) < 3) continue;  // the same bin either way
-          queue_cap[pair_bin] += rp.n_distinct;
-          queue_len[pair_bin] = std::max(queue_len[pair_bin], len);
+        const int few = queue_pair_bin(len, rp.generic, pd, true), many = queue_pair_bin(len, rp.generic, pd, false);
+        queue_cap[few] += rp.n_distinct;
+        if (few != many) {
+          many_cap[many] += rp.n_distinct;
+          if (queue_bin_group(bin) == 0) queue_cap[bin] += static_cast<int64_t>(rp.progs.size());  // whole-program tasks
         }
-        // Whole-program tasks, where single pairs go to another bin.
-        if (queue_bin_group(bin) == 0 && queue_pair_bin(len, rp.generic, pd, false) != bin) queue_cap[bin] += static_cast<int64_t>(rp.progs.size());
+        for (const int q : {few, many}) queue_len[q] = std::max(queue_len[q], len);
+        if (len > 8 * 31 || rp.generic) wide_pairs += R.n_haps;
       }
   }
+  // A batch that cannot lose more than a few pairs has no use for the other bins.
+  if (wide_pairs > few_pairs(sms_, kLongWarps))
+    for (int q = 0; q < kQueueBins; ++q) queue_cap[q] += many_cap[q];
   for (int q = 3 * kRowBins; q < kQueueBins; ++q) queue_cap[q] = std::min<int64_t>(queue_cap[q], few_pairs_most(sms_));
   if (n_stream > INT32_MAX || n_seq > INT32_MAX || n_pd_seq > INT32_MAX || n_haps > INT32_MAX)
     return fail(FGKL_E_INVALID_ARGUMENT, "batch too large for 32-bit plan offsets; split it");
@@ -1083,7 +1088,9 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
                           : whole         ? scratch_bytes(b.kind, b.rows, max_slots, max_nodes, max_segs)
                                           : scratch_bytes(b.kind, b.rows, 0, 0, 1));
       b.scratch_off = off;
-      off += static_cast<size_t>(b.blocks) * b.warps * b.stride;
+      // A block of a strip-mined launch has one carry column (allocated in fours: calls of a few pairs more or
+      // less fit one buffer), the others' warps a record set each.
+      off += (is_long(b.kind) ? align_up(static_cast<size_t>(b.blocks), 4) : static_cast<size_t>(b.blocks) * b.warps) * b.stride;
     }
     scratch_total = std::max(scratch_total, off);
   }

@@ -157,7 +157,7 @@ class Engine {
     int task_off;  // into the device task array
     int n_tasks;
     int blocks;
-    size_t stride;       // scratch bytes per warp
+    size_t stride;       // scratch bytes per warp, strip-mined per block
     size_t scratch_off;  // this bin's slice of the scratch
     uint64_t fwd_cells = 0, bwd_cells = 0;  // DP cells its tasks compute (first pass)
     int queue_bin = 0;   // recomputation bins: the queue bin (queue_bin) the tasks come from

@@ -132,7 +132,7 @@ struct LaunchArgs {
   const int* count;      // device-side task count (recomputation queues), or nullptr
   int* task_counter;     // zeroed before the launch
   char* scratch;
-  size_t scratch_stride; // bytes per warp
+  size_t scratch_stride; // bytes per warp, strip-mined per block
   int min_accept_plain;  // 1: results below the single-precision threshold are lost
   int only_lost;         // recomputation: a whole-program task writes only pairs whose result is NaN
 };

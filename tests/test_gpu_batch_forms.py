@@ -3,7 +3,7 @@ choice leaves each pair's bits as a call of its region alone gives them."""
 import numpy as np
 import pytest
 
-from fgkl_b200 import BatchContext, Config, PairHmm, PdPairHmm, Precision, synthetic
+from fgkl_b200 import BatchContext, Config, PairHmm, PdPairHmm, Precision, Read, set_allocation_limit, synthetic
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -117,3 +117,28 @@ def test_long_reads_of_a_full_batch_keep_the_bits_of_a_call(gpu, pd, precision):
         alone = (PdPairHmm if pd else PairHmm)(cfg).compute_log10_likelihoods(reads[:1], haps)
         assert alone.tobytes() == out[offs[g]:offs[g] + len(haps)].tobytes()
         assert np.max(np.abs(alone.reshape(-1) - O.compute_matrix(reads[:1], haps).reshape(-1))) < TOL[precision]
+
+
+@pytest.mark.parametrize("precision,value_bytes", [(Precision.FLOAT, 4), (Precision.DOUBLE, 8)])
+def test_strip_mined_pairs_take_one_carry_column_each(gpu, precision, value_bytes):
+    """A pair's row blocks hand on two values a haplotype column, whatever the warps that run them: four pairs of
+    eight row blocks against 200,000 columns (and as much again in FP64 for those that may be lost) fit buffers
+    in which a column for each of their warps would not."""
+    columns, reads = 200_000, 4
+    rng = np.random.default_rng(5)
+    hap = np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, columns)]
+    b = [hap[at:at + 1000].tobytes() for at in (100, 50_000, 90_000, 198_000)]
+    q = lambda v: bytes([v]) * 1000
+    w = synthetic.from_regions([([Read(s, q(30), q(45), q(45), q(10)) for s in b], [hap.tobytes()])])
+    cfg = Config(precision=precision)
+    free = BatchContext()
+    out, _ = free.compute(w, cfg)
+    one = 2 * value_bytes * columns
+    lost = 2 * 8 * columns
+    assert reads * lost + (1 << 20) < 8 * reads * one  # what eight warps a pair would take
+    prev = set_allocation_limit(reads * lost + (1 << 20))
+    try:
+        tight, _ = BatchContext().compute(w, cfg)
+    finally:
+        set_allocation_limit(prev)
+    assert tight.tobytes() == out.tobytes()
