@@ -908,7 +908,8 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       out.push_back({kind, rows, len_of(order[i]) + (i + 1 < order.size() ? len_of(order[i + 1]) : 0), Task{g, {a, b, -1, -1}, rows, -1, 0}, 0});
     };
     auto quad = [&](Kind kind, size_t i, size_t reads) {
-      Task t{g, {-1, -1, -1, -1}, quad_rows(len_of(order[i])), -1, 0};
+      const int rows = quad_rows(len_of(order[i]));
+      Task t{g, {-1, -1, -1, -1}, kind == Kind::kQuadF32 && tuning_.rows_extra != 0 && rows < kQuadMaxRows ? rows + 2 : rows, -1, 0};
       int len = 0;
       for (size_t k = 0; k < reads && i + k < order.size(); ++k) {
         t.read[k] = static_cast<int32_t>(first_read[g] + order[i + k]);
@@ -1018,7 +1019,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
         tasks.push_back(e.second);
         cost += e.first;
       }
-      const bool fp32 = b.kind == Kind::kShortF32 || b.kind == Kind::kPackedF32 || b.kind == Kind::kOneF32 || b.kind == Kind::kPackedF32Pd || b.kind == Kind::kOneF32Pd;
+      const bool fp32 = b.kind == Kind::kShortF32 || b.kind == Kind::kPackedF32 || b.kind == Kind::kQuadF32 || b.kind == Kind::kOneF32 || b.kind == Kind::kPackedF32Pd || b.kind == Kind::kOneF32Pd;
       const bool pipelined = is_long(b.kind);
       b.warps = pipelined ? choose_long_warps(b.kind, b.rows, sms_, bl.pairs) : (fp32 ? tuning_.warps_per_block : kWarpsPerBlock);
       int per_sm = 0, threads = 0;
@@ -1312,6 +1313,12 @@ void Engine::set_tuning(const Tuning& t) {
   tuning_.reads_per_warp = t.reads_per_warp == 1 ? 1 : 2;
   tuning_.rows_extra = t.rows_extra ? 1 : 0;
   tuning_.warps_per_block = (t.warps_per_block == 1 || t.warps_per_block == 2) ? t.warps_per_block : kWarpsPerBlock;
+}
+
+std::vector<std::array<int, 4>> Engine::first_pass() const {
+  std::vector<std::array<int, 4>> out;
+  for (const Bin& b : bins_) out.push_back({static_cast<int>(b.kind), b.rows, b.blocks, b.warps});
+  return out;
 }
 
 int Engine::time_run(int repeats, double* ms) {

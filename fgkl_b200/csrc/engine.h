@@ -5,6 +5,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <array>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -134,9 +135,9 @@ class Engine {
   // over (1: one after another; more: bins overlap, the largest first), each first-pass persistent
   // grid as a percentage of the resident-block limit, how many reads an FP32 PD-HMM warp carries
   // (two in FP32x2 at 8 warps per SM, or one at 12), and the first pass's tile shape: rows per lane
-  // of the plain FP32 reads that go one or two to a warp (the fewest that hold the read, or the next the
-  // kernels instantiate) and warps per block of the FP32 first-pass kernels but the quad form's. None changes a result bit. Applies from the
-  // next prepare().
+  // of the plain FP32 reads (the fewest that hold the read, or the next the kernels instantiate) and warps
+  // per block of the FP32 first-pass kernels (the quad form's have one, or two for any more). None changes a
+  // result bit. Applies from the next prepare().
   struct Tuning {
     int streams = 8;
     int grid_percent = 100;
@@ -149,6 +150,8 @@ class Engine {
   // Times the prepared batch's kernels (direct launches on the stream, after one untimed run):
   // the median of `repeats` runs, in milliseconds. Host-synchronous.
   int time_run(int repeats, double* ms);
+  // The prepared batch's first-pass launches: kind, rows per lane, blocks and warps per block of each.
+  std::vector<std::array<int, 4>> first_pass() const;
 
  private:
   struct Bin {

@@ -472,7 +472,7 @@ void occupancy(Kind k, int rows, int* blocks, int* threads, int warps) {
   if (is_long(k)) return long_occupancy(k, rows, blocks, threads, warps);
   if (!valid_rows(k, rows) || (warps != 1 && warps != 2 && warps != 4)) return;
   if (is_pd(k)) return pd_occupancy(pd_form(k), rows, blocks, threads, warps);
-  if (is_quad(k)) return quad_occupancy(k, rows, blocks, threads);
+  if (is_quad(k)) return quad_occupancy(k, rows, blocks, threads, warps);
   dispatch<OccF>(k, rows, blocks, threads, warps);
 }
 
@@ -486,7 +486,7 @@ cudaError_t launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStr
   if (is_long(k)) return long_launch(k, rows, blocks, args, stream, warps);
   if (!valid_rows(k, rows) || (warps != 1 && warps != 2 && warps != 4)) return cudaErrorInvalidValue;
   if (is_pd(k)) return pd_launch(pd_form(k), rows, blocks, args, stream, warps);
-  if (is_quad(k)) return quad_launch(k, rows, blocks, args, stream);
+  if (is_quad(k)) return quad_launch(k, rows, blocks, args, stream, warps);
   return dispatch<GoF>(k, rows, blocks, args, stream, warps);
 }
 

@@ -157,10 +157,10 @@ size_t scratch_bytes(Kind k, int rows, int max_slots, int max_nodes, int max_seg
 void occupancy(Kind k, int rows, int* blocks_per_sm, int* threads_per_block, int warps_per_block = 4);
 // Launches one persistent grid of `blocks` blocks.
 cudaError_t launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream, int warps_per_block = 4);
-// The quad form (quad.cpp). Warps per block are its own.
+// The quad form (quad.cpp): one warp a block, or two for any more.
 size_t quad_scratch_bytes(Kind k, int rows, int max_slots, int max_nodes, int max_segs);
-void quad_occupancy(Kind k, int rows, int* blocks_per_sm, int* threads_per_block);
-cudaError_t quad_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream);
+void quad_occupancy(Kind k, int rows, int* blocks_per_sm, int* threads_per_block, int warps_per_block);
+cudaError_t quad_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream, int warps_per_block);
 // PD-HMM instantiations (pd_kernels.cu).
 size_t pd_scratch_bytes(PdForm form, int rows, int max_slots, int max_segs);
 void pd_occupancy(PdForm form, int rows, int* blocks_per_sm, int* threads_per_block, int warps_per_block = 4);

@@ -17,12 +17,12 @@ size_t quad_scratch_bytes(Kind k, int rows, int max_slots, int max_nodes, int ma
   return quad_range(k, rows, [&](auto q) { return q.scratch(rows, max_slots, max_nodes, max_segs); });
 }
 
-void quad_occupancy(Kind k, int rows, int* blocks, int* threads) {
-  *blocks = quad_range(k, rows, [&](auto q) { return q.occupancy(rows, threads); });
+void quad_occupancy(Kind k, int rows, int* blocks, int* threads, int warps) {
+  *blocks = quad_range(k, rows, [&](auto q) { return q.occupancy(rows, warps, threads); });
 }
 
-cudaError_t quad_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream) {
-  return quad_range(k, rows, [&](auto q) { return q.launch(rows, blocks, args, stream); });
+cudaError_t quad_launch(Kind k, int rows, int blocks, const LaunchArgs& args, cudaStream_t stream, int warps) {
+  return quad_range(k, rows, [&](auto q) { return q.launch(rows, blocks, args, stream, warps); });
 }
 
 }  // namespace fgkl

@@ -8,8 +8,8 @@ namespace fgkl {
 template <bool kDouble, int kLo, int kHi>
 struct QuadRange {
   static size_t scratch(int rows, int max_slots, int max_nodes, int max_segs);
-  static int occupancy(int rows, int* threads);
-  static cudaError_t launch(int rows, int blocks, const LaunchArgs& a, cudaStream_t s);
+  static int occupancy(int rows, int warps, int* threads);
+  static cudaError_t launch(int rows, int blocks, const LaunchArgs& a, cudaStream_t s, int warps);
 };
 
 }  // namespace fgkl

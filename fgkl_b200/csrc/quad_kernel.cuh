@@ -21,9 +21,12 @@ template <bool kDouble>
 using QuadPolicy = std::conditional_t<kDouble, OneF64Table, PackedF32>;
 
 template <bool kDouble, int R>
-constexpr size_t quad_smem() {
-  return kQuadWarps * Layout<QuadPolicy<kDouble>, R>::kSmemPerWarp;
+constexpr size_t quad_smem(int warps) {
+  return warps * Layout<QuadPolicy<kDouble>, R>::kSmemPerWarp;
 }
+
+// Warps of a block when `warps` are asked for.
+constexpr int quad_warps(int warps) { return warps < kQuadWarps ? warps : kQuadWarps; }
 }  // namespace
 
 template <bool kDouble, int kLo, int kHi>
@@ -34,22 +37,25 @@ size_t QuadRange<kDouble, kLo, kHi>::scratch(int rows, int max_slots, int max_no
 }
 
 template <bool kDouble, int kLo, int kHi>
-int QuadRange<kDouble, kLo, kHi>::occupancy(int rows, int* threads) {
+int QuadRange<kDouble, kLo, kHi>::occupancy(int rows, int warps, int* threads) {
   int blocks = 0;
-  *threads = kQuadWarps * 32;
+  warps = quad_warps(warps);
+  *threads = warps * 32;
   rows_at<kLo, kHi>(rows, [&](auto r) {
     constexpr int R = decltype(r)::value;
-    static std::atomic<int> cache[kMaxDevices];
-    blocks = resident_blocks(pairhmm_kernel<QuadPolicy<kDouble>, R, kQuadLanes>, quad_smem<kDouble, R>(), kQuadWarps * 32, cache);
+    static std::atomic<int> cache[kQuadWarps][kMaxDevices];
+    blocks = resident_blocks(pairhmm_kernel<QuadPolicy<kDouble>, R, kQuadLanes>, quad_smem<kDouble, R>(warps), warps * 32, cache[warps - 1],
+                             quad_smem<kDouble, R>(kQuadWarps));
   });
   return blocks;
 }
 
 template <bool kDouble, int kLo, int kHi>
-cudaError_t QuadRange<kDouble, kLo, kHi>::launch(int rows, int blocks, const LaunchArgs& a, cudaStream_t s) {
+cudaError_t QuadRange<kDouble, kLo, kHi>::launch(int rows, int blocks, const LaunchArgs& a, cudaStream_t s, int warps) {
+  warps = quad_warps(warps);
   rows_at<kLo, kHi>(rows, [&](auto r) {
     constexpr int R = decltype(r)::value;
-    pairhmm_kernel<QuadPolicy<kDouble>, R, kQuadLanes><<<blocks, kQuadWarps * 32, quad_smem<kDouble, R>(), s>>>(a);
+    pairhmm_kernel<QuadPolicy<kDouble>, R, kQuadLanes><<<blocks, warps * 32, quad_smem<kDouble, R>(warps), s>>>(a);
   });
   return cudaGetLastError();
 }

@@ -198,10 +198,10 @@ typedef struct fgkl_tuning {
   int32_t grid_percent;     /* each first-pass persistent grid, % of the kernel's resident-block limit, 10-100 */
   int32_t reads_per_warp;   /* FP32 PD-HMM reads of at most 248 bases: 2 (FP32x2 pairs, the default, where
                                the batch fills the GPU with them) or 1 */
-  int32_t rows_extra;       /* tile shape: 1 runs plain FP32 reads that go one or two to a warp one rows-per-lane
-                               step above the fewest that hold them (0, the default: the fewest) */
-  int32_t warps_per_block;  /* tile shape: warps per block of the FP32 first-pass kernels (other than the one
-                               with four reads a warp), 1, 2 or 4 (default) */
+  int32_t rows_extra;       /* tile shape: 1 runs plain FP32 reads one rows-per-lane step above the fewest
+                               that hold them (0, the default: the fewest) */
+  int32_t warps_per_block;  /* tile shape: warps per block of the FP32 first-pass kernels, 1, 2 or 4 (default);
+                               2 is the most of the one with four reads a warp */
   double ms;                /* autotuner: median device time of one run of the batch with this configuration */
 } fgkl_tuning;
 

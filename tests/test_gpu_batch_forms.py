@@ -142,3 +142,29 @@ def test_strip_mined_pairs_take_one_carry_column_each(gpu, precision, value_byte
     finally:
         set_allocation_limit(prev)
     assert tight.tobytes() == out.tobytes()
+
+
+def test_tile_shapes_reach_four_reads_a_warp(gpu):
+    """Rows per lane one step up (the form has even values) and one warp a block, with the same bits; the
+    autotuner gives a shape that leaves every launch as it was the time of the configuration it is tried on."""
+    w = synthetic.from_regions(regions_of([(100,) * 12, (223,) * 9, (30,) * 8], 16, 320, 400))
+    base = BatchContext()
+    base.set_profiling(True)
+    out, _ = base.compute(w, FLOAT)
+    assert {p["kind"] for p in launches(base)} == {12}
+    for rows_extra, warps in ((1, 4), (0, 1), (0, 2), (1, 1)):
+        ctx = BatchContext()
+        ctx.set_tuning(8, 100, 2, rows_extra, warps)
+        ctx.set_profiling(True)
+        shaped, _ = ctx.compute(w, FLOAT)
+        assert shaped.tobytes() == out.tobytes()
+        up = {min(14, p["rows"] + 2 * rows_extra) for p in launches(base)}
+        assert {p["rows"] for p in launches(ctx)} == up
+        # A launch has a block for each two tasks, or each, as long as they are resident together.
+        small = [(a["blocks"], b["blocks"]) for a in launches(base) for b in launches(ctx) if a["rows"] == b["rows"]]
+        assert warps > 1 or rows_extra or any(b > a for a, b in small)
+    chosen, tried = BatchContext().autotune(w, FLOAT, repeats=1)
+    best = min(t["ms"] for t in tried[:16])
+    by_shape = {(t["rows_extra"], t["warps_per_block"]): t["ms"] for t in tried[16:]}
+    assert by_shape[0, 2] == best  # two warps are what the default's four come to
+    assert chosen["ms"] == min(t["ms"] for t in tried)
