@@ -151,53 +151,76 @@ int AdjointEngine::prepare(const AdjointInput& in, bool double_precision) {
   int64_t split = total_reads > 0 ? (2 * 12 * static_cast<int64_t>(sms_)) / total_reads : 1;
   split = std::min<int64_t>(split, most_haps);
   if (grad_len_ > 0) split = std::min<int64_t>(split, 1 + static_cast<int64_t>(kPartBudget / (4 * sizeof(double) * static_cast<size_t>(grad_len_))));
-  split_ = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(split, INT32_MAX / std::max<int64_t>(1, total_reads))));
-  std::vector<int32_t> tasks;
-  for (auto& [rows, list] : by_rows) {
+  const int most_parts = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(split, INT32_MAX / std::max<int64_t>(1, total_reads))));
+  for (auto& [rows, list] : by_rows)
     std::stable_sort(list.begin(), list.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-    Bin b{dbl_, rows, static_cast<int>(tasks.size()), static_cast<int>(list.size()) * split_, 0, 0};
-    for (auto& e : list)
-      for (int k = 0; k < split_; ++k) tasks.push_back(e.second * split_ + k);
-    bins_.push_back(b);
-  }
-  std::vector<int> queue_off(kAdjRowBins + 1, 0);
-  for (int r = 0; r < kAdjRowBins; ++r) queue_off[r + 1] = queue_off[r] + (dbl_ ? 0 : per_rows[r] * split_);
-  if (!dbl_)
-    for (int r = 1; r < kAdjRowBins; ++r)
-      if (per_rows[r]) rescue_.push_back(Bin{true, r, queue_off[r], per_rows[r] * split_, 0, 0});
-  // The bins of a pass run side by side where a scratch of its own for each fits kSideBudget (a bin of a few
-  // reads leaves most of the GPU idle), else one after another on one scratch. A bin's grid shrinks only
-  // when its warps' scratch would exceed the budget (very long pairs).
-  size_t scratch = 256, side = 0;
-  for (auto* list : {&bins_, &rescue_}) {
-    size_t sum = 0;
-    for (Bin& b : *list) {
-      int per_sm = 0, threads = 0;
-      adj_occupancy(b.dbl, b.rows, &per_sm, &threads);
-      if (per_sm <= 0) return fail(FGKL_E_CUDA, "adjoint kernel unavailable on this device");
-      const int64_t want = std::min<int64_t>((b.n_tasks + kWarps - 1) / kWarps, static_cast<int64_t>(per_sm) * sms_);
-      b.stride = align_up(std::max<size_t>(need[b.rows], 256));
-      const int64_t by_budget = static_cast<int64_t>(kScratchBudget / (kWarps * b.stride));
-      b.blocks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, by_budget)));
-      scratch = std::max(scratch, static_cast<size_t>(b.blocks) * kWarps * b.stride);
-      b.scratch_off = sum;
-      sum += static_cast<size_t>(b.blocks) * kWarps * b.stride;
+  std::vector<int32_t> tasks;
+  std::vector<int> queue_off;
+  // Lays the batch out with `parts` parts a read and, where `side_limit` bytes of scratch allow, the bins of a
+  // pass side by side, and allocates its device buffers. FGKL_E_OUT_OF_MEMORY where they do not fit.
+  const auto lay_out = [&](int parts, size_t side_limit) -> int {
+    split_ = parts;
+    bins_.clear();
+    rescue_.clear();
+    tasks.clear();
+    for (auto& [rows, list] : by_rows) {
+      Bin b{dbl_, rows, static_cast<int>(tasks.size()), static_cast<int>(list.size()) * split_, 0, 0};
+      for (auto& e : list)
+        for (int k = 0; k < split_; ++k) tasks.push_back(e.second * split_ + k);
+      bins_.push_back(b);
     }
-    side = std::max(side, sum);
-  }
-  side_by_side_ = side <= kSideBudget;
-  if (side_by_side_) scratch = std::max(scratch, side);
+    queue_off.assign(kAdjRowBins + 1, 0);
+    for (int r = 0; r < kAdjRowBins; ++r) queue_off[r + 1] = queue_off[r] + (dbl_ ? 0 : per_rows[r] * split_);
+    if (!dbl_)
+      for (int r = 1; r < kAdjRowBins; ++r)
+        if (per_rows[r]) rescue_.push_back(Bin{true, r, queue_off[r], per_rows[r] * split_, 0, 0});
+    // The bins of a pass run side by side where a scratch of its own for each fits the limit (a bin of a few
+    // reads leaves most of the GPU idle), else one after another on one scratch. A bin's grid shrinks only
+    // when its warps' scratch would exceed the budget (very long pairs).
+    size_t scratch = 256, side = 0;
+    for (auto* list : {&bins_, &rescue_}) {
+      size_t sum = 0;
+      for (Bin& b : *list) {
+        int per_sm = 0, threads = 0;
+        adj_occupancy(b.dbl, b.rows, &per_sm, &threads);
+        if (per_sm <= 0) return fail(FGKL_E_CUDA, "adjoint kernel unavailable on this device");
+        const int64_t want = std::min<int64_t>((b.n_tasks + kWarps - 1) / kWarps, static_cast<int64_t>(per_sm) * sms_);
+        b.stride = align_up(std::max<size_t>(need[b.rows], 256));
+        const int64_t by_budget = static_cast<int64_t>(kScratchBudget / (kWarps * b.stride));
+        b.blocks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, by_budget)));
+        scratch = std::max(scratch, static_cast<size_t>(b.blocks) * kWarps * b.stride);
+        b.scratch_off = sum;
+        sum += static_cast<size_t>(b.blocks) * kWarps * b.stride;
+      }
+      side = std::max(side, sum);
+    }
+    side_by_side_ = side <= side_limit;
+    if (side_by_side_) scratch = std::max(scratch, side);
 
-  // Device buffers.
-  const size_t n_bytes = static_cast<size_t>(grad_len_) + static_cast<size_t>(hap_bytes) + 16;
-  const size_t n_off = static_cast<size_t>(total_reads + 1 + total_haps + 1 + N);
-  const size_t n_idx = static_cast<size_t>(total_reads + 3 * N) + tasks.size() + static_cast<size_t>(queue_off[kAdjRowBins]);
-  n_small_ = static_cast<int>(bins_.size() + rescue_.size()) + 2 * kAdjRowBins + 1;
-  if (!grow(d_bytes_, cap_bytes_, n_bytes) || !grow(d_params_, cap_params_, 4 * static_cast<size_t>(grad_len_) + 1) ||
-      !grow(d_off_, cap_off_, n_off + 1) || !grow(d_idx_, cap_idx_, n_idx + 1) ||
-      !grow(d_out_, cap_out_, static_cast<size_t>(out_len_) + static_cast<size_t>(split_) * 4 * static_cast<size_t>(grad_len_) + 1) ||
-      !grow(d_small_, cap_small_, static_cast<size_t>(n_small_) + static_cast<size_t>(total_reads)) || !grow(d_scratch_, cap_scratch_, scratch))
-    return fail(FGKL_E_OUT_OF_MEMORY, "device allocation failed");
+    const size_t n_bytes = static_cast<size_t>(grad_len_) + static_cast<size_t>(hap_bytes) + 16;
+    const size_t n_off = static_cast<size_t>(total_reads + 1 + total_haps + 1 + N);
+    const size_t n_idx = static_cast<size_t>(total_reads + 3 * N) + tasks.size() + static_cast<size_t>(queue_off[kAdjRowBins]);
+    n_small_ = static_cast<int>(bins_.size() + rescue_.size()) + 2 * kAdjRowBins + 1;
+    if (!grow(d_bytes_, cap_bytes_, n_bytes) || !grow(d_params_, cap_params_, 4 * static_cast<size_t>(grad_len_) + 1) ||
+        !grow(d_off_, cap_off_, n_off + 1) || !grow(d_idx_, cap_idx_, n_idx + 1) ||
+        !grow(d_out_, cap_out_, static_cast<size_t>(out_len_) + static_cast<size_t>(split_) * 4 * static_cast<size_t>(grad_len_) + 1) ||
+        !grow(d_small_, cap_small_, static_cast<size_t>(n_small_) + static_cast<size_t>(total_reads)) || !grow(d_scratch_, cap_scratch_, scratch))
+      return fail(FGKL_E_OUT_OF_MEMORY, "device allocation failed");
+    return FGKL_OK;
+  };
+  int laid = lay_out(most_parts, kSideBudget);
+  if (laid == FGKL_E_OUT_OF_MEMORY && (split_ > 1 || side_by_side_)) {
+    // The memory is short: one part a read and one bin after another take the least. What the parts made
+    // large is given back first.
+    cudaFree(d_out_);
+    cudaFree(d_scratch_);
+    d_out_ = nullptr;
+    d_scratch_ = nullptr;
+    cap_out_ = cap_scratch_ = 0;
+    error_.clear();
+    laid = lay_out(1, 0);
+  }
+  if (laid) return laid;
 
   std::vector<int32_t> region_hap(N), region_nhap(N), region_read(N);
   for (int g = 0; g < N; ++g) {
