@@ -22,8 +22,8 @@ constexpr int kWarpsPerBlock = 4;
 __host__ __device__ constexpr int warps_index(int warps) { return warps <= 1 ? 0 : (warps == 2 ? 1 : 2); }
 
 // ---------------------------------------------------------------------------------------------
-// Arithmetic policies. kTable: priors come from a table by haplotype code. up and down move a value one lane within groups of G lanes (the first, respectively
-// last, lane of a group receives its own).
+// Arithmetic policies. kTable: priors come from a table by haplotype code. up and down move a value one
+// lane within groups of G lanes (the first, respectively last, lane of a group receives its own).
 // ---------------------------------------------------------------------------------------------
 
 struct PackedF32 {

@@ -30,8 +30,8 @@ enum class Kind : int {
   kPackedF32 = 15,  // two reads of at most 248 bases on all lanes in FP32x2, rows-per-lane 1..8
 };
 constexpr int kNumKinds = 16;
-// Lanes that hold two reads (FP32x2) or one (FP64) in the quad form, reads a warp in FP32x2, its largest rows-per-lane and its longest
-// read (the first row of the first lane is padding).
+// Lanes that hold two reads (FP32x2) or one (FP64) in the quad form, reads a warp in FP32x2, its largest
+// rows-per-lane and its longest read (the first row of the first lane is padding).
 constexpr int kQuadLanes = 16, kQuadReads = 4;
 constexpr int kQuadMaxRows = 14;
 constexpr int kQuadMaxRead = kQuadLanes * kQuadMaxRows - 1;

@@ -79,7 +79,7 @@ constexpr size_t pd_scratch_size(int n_slots, int n_segs) {
 // Forward coefficients of the lane's rows and each row's read class. As in the plain kernel, what row r + 1
 // takes from row r is held with row r (k0..k3, k5), because the lane computes both values that its bottom
 // row hands to the lane below.
-template <class P, int R, int G>
+template <class P, int R>
 struct PdRows {
   using V = typename P::V;
   using S = typename P::S;
@@ -111,7 +111,7 @@ struct PdRows {
   }
 
   __device__ void load(const BatchView& v, const ReadRef* rd, int lane, const uint8_t* classes) {
-    const int top = (lane % G) * R;
+    const int top = lane * R;
 #pragma unroll
     for (int r = 0; r <= R; ++r) {
 #pragma unroll
@@ -143,7 +143,7 @@ struct PdRows {
     load(v, rd, lane, classes);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int q = (lane % G) * R + r - rd[0].pad;
+      const int q = lane * R + r - rd[0].pad;
       uint32_t d = 0;
       if (rd[0].len > 0 && q >= 0 && q < rd[0].len) {
         const uint32_t b = v.bases[rd[0].off + q];
@@ -181,8 +181,8 @@ struct PdState {
 // exact for every column, so the whole warp takes it. keep(r): what to do with the branch values of row r
 // before its column; de: the lane's column carries DEL_END, and each row's values take the max with its
 // branch values once its X is computed, so that the next row's X reads U = max(B(up), V(up)).
-template <class P, int R, int G, bool kSlow, class Prior, class Keep>
-__device__ __forceinline__ void pd_rows_down(const PdRows<P, R, G>& pr, PdState<P, R>& st, const typename P::V& an, typename P::V qX,
+template <class P, int R, bool kSlow, class Prior, class Keep>
+__device__ __forceinline__ void pd_rows_down(const PdRows<P, R>& pr, PdState<P, R>& st, const typename P::V& an, typename P::V qX,
                                              typename P::V T, bool de, Prior&& prior, Keep&& keep) {
   using V = typename P::V;
 #pragma unroll
@@ -207,24 +207,23 @@ __device__ __forceinline__ void pd_rows_down(const PdRows<P, R, G>& pr, PdState<
 
 // One PD forward step: events, then the column. kEv = false compiles the event code out, for steps where no
 // lane of the warp has an event. kCarry = true gives lane 0 the row above from the state's carry values
-// (strip-mined reads); otherwise a group's first lane starts with a padding row, for which the row above is
+// (strip-mined reads); otherwise lane 0 starts with a padding row, for which the row above is
 // zero. kGeneric = true decides priors by comparing bytes (PdRows::prior_generic) instead of by class bits.
-template <class P, int R, int G, bool kEv = true, bool kCarry = false, bool kGeneric = false>
+template <class P, int R, bool kEv = true, bool kCarry = false, bool kGeneric = false>
 __device__ __forceinline__ void pd_step(const LaunchArgs& a, const Program& prog, const ReadRef* rd, int lane,
-                                        const PdRows<P, R, G>& pr, const typename P::V& an, PdScratch<P, R>& sc,
+                                        const PdRows<P, R>& pr, const typename P::V& an, PdScratch<P, R>& sc,
                                         PdState<P, R>& st, int synth_len, uint32_t ev, uint32_t sig) {
   using V = typename P::V;
   using S = typename P::S;
   using L = PdLayout<P, R>;
-  const int gl = lane % G;
-  V qX = P::template up<G>(st.xs), T = P::template up<G>(st.ts);
-  if (gl == 0) {
+  V qX = P::up(st.xs), T = P::up(st.ts);
+  if (lane == 0) {
     qX = kCarry ? st.cX : P::zero();
     T = kCarry ? st.cT : P::zero();
   }
-  // END and ACC act in the group's last lane alone (the read's last row); the other lanes pass them by
+  // END and ACC act in the last lane alone (the read's last row); the other lanes pass them by
   // without entering the event code, which every lane otherwise reaches at its own step.
-  if (kEv && (ev & (gl == G - 1 ? kEvMask : (kEvMask & ~(EV_END | EV_ACC))))) {
+  if (kEv && (ev & (lane == 31 ? kEvMask : (kEvMask & ~(EV_END | EV_ACC))))) {
     if (ev & EV_SNAP) {
       const uint32_t slot = ev >> kPdPayloadShift;
       V* dst[2] = {slot != kPdPayloadNone ? sc.slot(static_cast<int>(slot), lane) : nullptr,
@@ -245,9 +244,9 @@ __device__ __forceinline__ void pd_step(const LaunchArgs& a, const Program& prog
         o[6 * R] = st.acc;
       }
     }
-    if ((ev & EV_END) && gl == G - 1) {
+    if ((ev & EV_END) && lane == 31) {
 #pragma unroll
-      for (int c = 0; c < P::NC; ++c) sc.raw(st.seg_i, lane / G * P::NC + c) = static_cast<double>(P::get(st.acc, c));
+      for (int c = 0; c < P::NC; ++c) sc.raw(st.seg_i, c) = static_cast<double>(P::get(st.acc, c));
     }
     if (ev & EV_BEGIN) {
       ++st.seg_i;
@@ -278,7 +277,7 @@ __device__ __forceinline__ void pd_step(const LaunchArgs& a, const Program& prog
         for (int r = 0; r < R; ++r) {
           st.M[r] = st.X[r] = st.BM[r] = st.BX[r] = st.BY[r] = P::zero();
 #pragma unroll
-          for (int c = 0; c < P::NC; ++c) P::put(st.Y[r], c, gl * R + r < rd[c].pad ? in_s : S(0));
+          for (int c = 0; c < P::NC; ++c) P::put(st.Y[r], c, lane * R + r < rd[c].pad ? in_s : S(0));
         }
         st.acc = P::zero();
       }
@@ -295,7 +294,7 @@ __device__ __forceinline__ void pd_step(const LaunchArgs& a, const Program& prog
       // haplotype's end): a column carrying either flag keeps V(left) as the branch values unless
       // inside a deletion, one predicate a lane.
       const bool keep = mat && s_later != kPdInsideDel;
-      pd_rows_down<P, R, G, true>(pr, st, an, qX, T, de, prior, [&](int r) {
+      pd_rows_down<P, R, true>(pr, st, an, qX, T, de, prior, [&](int r) {
         if (keep) {
           st.BM[r] = st.M[r];
           st.BX[r] = st.X[r];
@@ -304,10 +303,10 @@ __device__ __forceinline__ void pd_step(const LaunchArgs& a, const Program& prog
       });
     } else {
       // Some lane's first read row is in another state than its later rows.
-      pd_rows_down<P, R, G, true>(pr, st, an, qX, T, de, prior, [&](int r) {
+      pd_rows_down<P, R, true>(pr, st, an, qX, T, de, prior, [&](int r) {
         bool inside[P::NC];
 #pragma unroll
-        for (int c = 0; c < P::NC; ++c) inside[c] = ((gl * R + r == rd[c].pad) ? s_first : s_later) == kPdInsideDel;
+        for (int c = 0; c < P::NC; ++c) inside[c] = ((lane * R + r == rd[c].pad) ? s_first : s_later) == kPdInsideDel;
         if (mat) {
           st.BM[r] = P::sel(inside[0], inside[P::NC - 1], st.BM[r], st.M[r]);
           st.BX[r] = P::sel(inside[0], inside[P::NC - 1], st.BX[r], st.X[r]);
@@ -316,7 +315,7 @@ __device__ __forceinline__ void pd_step(const LaunchArgs& a, const Program& prog
       });
     }
   } else {
-    pd_rows_down<P, R, G, false>(pr, st, an, qX, T, false, prior, [](int) {});
+    pd_rows_down<P, R, false>(pr, st, an, qX, T, false, prior, [](int) {});
   }
 }
 
@@ -330,14 +329,13 @@ __device__ __forceinline__ uint32_t pd_synth_entry(const uint32_t* seq, int len,
   return e;
 }
 
-template <class P, int R, int G>
+template <class P, int R>
 __device__ __forceinline__ void pd_forward_pass(const LaunchArgs& a, const Program& prog, const ReadRef* rd, const uint8_t* classes,
                                                 const uint32_t* sigs, int lane, PdScratch<P, R>& sc, const uint32_t* synth_seq,
                                                 int synth_len) {
   using V = typename P::V;
   using S = typename P::S;
-  const int gl = lane % G;
-  PdRows<P, R, G> pr;
+  PdRows<P, R> pr;
   pr.load(a.v, rd, lane, classes);
   V an;
 #pragma unroll
@@ -349,46 +347,46 @@ __device__ __forceinline__ void pd_forward_pass(const LaunchArgs& a, const Progr
   if (P::kDouble && synth_len > 0) {
     const int n = synth_len;
     auto at = [&](int t) {
-      const uint32_t e = pd_synth_entry(synth_seq, n, t - gl);
-      pd_step<P, R, G>(a, prog, rd, lane, pr, an, sc, st, synth_len, e, __ldg(sigs + (e & kCodeMask)));
+      const uint32_t e = pd_synth_entry(synth_seq, n, t - lane);
+      pd_step<P, R>(a, prog, rd, lane, pr, an, sc, st, synth_len, e, __ldg(sigs + (e & kCodeMask)));
     };
     int t = 0;
-    for (; t < G; ++t) at(t);
+    for (; t < 32; ++t) at(t);
     // Every lane strictly inside the haplotype: no events. An entry is loaded two steps ahead and its
     // signature one, so neither load waits on the other.
-    const uint32_t* seq = synth_seq - gl;
+    const uint32_t* seq = synth_seq - lane;
     if (t < n) {
       auto entry = [&](int i) { return i < n ? __ldg(seq + i) : 0u; };
       uint32_t e0 = entry(t), e1 = entry(t + 1), g0 = __ldg(sigs + (e0 & kCodeMask));
 #pragma unroll 2
       for (; t < n; ++t) {
         const uint32_t e2 = entry(t + 2), g1 = __ldg(sigs + (e1 & kCodeMask));
-        pd_step<P, R, G, false>(a, prog, rd, lane, pr, an, sc, st, synth_len, e0, g0);
+        pd_step<P, R, false>(a, prog, rd, lane, pr, an, sc, st, synth_len, e0, g0);
         e0 = e1;
         e1 = e2;
         g0 = g1;
       }
     }
-    for (; t < n + G; ++t) at(t);
+    for (; t < n + 32; ++t) at(t);
   } else {
     const int n = prog.fwd_len;
-    const uint32_t* stream = a.v.stream + prog.fwd_off - gl;
+    const uint32_t* stream = a.v.stream + prog.fwd_off - lane;
     // Two steps an iteration; one where no lane has an event runs a body without event code.
-    const uint32_t keep = gl == G - 1 ? kEvMask : (kEvMask & ~(EV_END | EV_ACC));
+    const uint32_t keep = lane == 31 ? kEvMask : (kEvMask & ~(EV_END | EV_ACC));
     uint32_t n0 = __ldg(stream), n1 = __ldg(stream + 1);
     uint32_t g0 = __ldg(sigs + (n0 & kCodeMask)), g1 = __ldg(sigs + (n1 & kCodeMask));
-    for (int t = 0; t < n + G; t += 2) {
+    for (int t = 0; t < n + 32; t += 2) {
       const uint32_t e0 = n0, e1 = n1, s0 = g0, s1 = g1;
       n0 = __ldg(stream + t + 2);
       n1 = __ldg(stream + t + 3);
       g0 = __ldg(sigs + (n0 & kCodeMask));
       g1 = __ldg(sigs + (n1 & kCodeMask));
       if (__any_sync(kFull, (e0 | e1) & keep)) {
-        pd_step<P, R, G>(a, prog, rd, lane, pr, an, sc, st, 0, e0, s0);
-        pd_step<P, R, G>(a, prog, rd, lane, pr, an, sc, st, 0, e1, s1);
+        pd_step<P, R>(a, prog, rd, lane, pr, an, sc, st, 0, e0, s0);
+        pd_step<P, R>(a, prog, rd, lane, pr, an, sc, st, 0, e1, s1);
       } else {
-        pd_step<P, R, G, false>(a, prog, rd, lane, pr, an, sc, st, 0, e0, s0);
-        pd_step<P, R, G, false>(a, prog, rd, lane, pr, an, sc, st, 0, e1, s1);
+        pd_step<P, R, false>(a, prog, rd, lane, pr, an, sc, st, 0, e0, s0);
+        pd_step<P, R, false>(a, prog, rd, lane, pr, an, sc, st, 0, e1, s1);
       }
     }
   }
@@ -396,7 +394,7 @@ __device__ __forceinline__ void pd_forward_pass(const LaunchArgs& a, const Progr
 }
 
 // Thresholds, log10 and the caller's layout (fgkl kernel.rs:897-914 via pd_kernel.rs:262-270).
-template <class P, int R, int G>
+template <class P, int R>
 __device__ __forceinline__ void pd_finalize(const LaunchArgs& a, const Task& task, const Region& region, const Program& prog, int lane,
                             PdScratch<P, R>& sc) {
   using C = Consts<P::kDouble>;
@@ -421,7 +419,7 @@ __device__ __forceinline__ void pd_finalize(const LaunchArgs& a, const Task& tas
     if (own < 0 || own >= prog.n_segs) continue;
     const double factor = a.v.segs[prog.seg_off + own].factor;
 #pragma unroll
-    for (int c = 0; c < 32 / G * P::NC; ++c) {
+    for (int c = 0; c < P::NC; ++c) {
       if (task.read[c] < 0) continue;
       const int read_local = task.read[c] - region.read_off;
       double* dst = a.v.out + region.out_off + static_cast<int64_t>(read_local) * region.n_haps + info.order;
@@ -450,7 +448,7 @@ struct PdMinBlocks {
   static constexpr int value = P::kDouble ? (R <= 5 ? 3 : 1) : (P::NC == 2 ? (R <= 5 ? 3 : 2) : (R <= 6 ? 4 : R <= 9 ? 3 : 2));
 };
 
-template <class P, int R, int G>
+template <class P, int R>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, (PdMinBlocks<P, R>::value)) pd_kernel(LaunchArgs a) {
   using V = typename P::V;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -470,7 +468,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (PdMinBlocks<P, R>::value
     ReadRef rd[P::NC];
 #pragma unroll
     for (int c = 0; c < P::NC; ++c) {
-      const int id = task.read[lane / G * P::NC + c];
+      const int id = task.read[c];
       if (id >= 0) {
         rd[c].off = a.v.read_off[id];
         rd[c].len = static_cast<int>(a.v.read_off[id + 1] - rd[c].off);
@@ -478,7 +476,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (PdMinBlocks<P, R>::value
         rd[c].off = 0;
         rd[c].len = 0;
       }
-      rd[c].pad = G * R - rd[c].len;
+      rd[c].pad = 32 * R - rd[c].len;
     }
     const uint8_t* classes = a.v.code_of_byte + region.code_off;
     const uint32_t* sigs = a.v.pd_sigs + region.sig_off;
@@ -486,12 +484,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (PdMinBlocks<P, R>::value
     if (P::kDouble && task.hap >= 0) {
       const HapInfo info = a.v.haps[region.hap_off + task.hap];
       PdScratch<P, R> sc(scratch, smem, 0);
-      pd_forward_pass<P, R, G>(a, prog, rd, classes, sigs, lane, sc, a.v.pd_entries + region.seq_off + info.seq, info.len);
-      pd_finalize<P, R, G>(a, task, region, prog, lane, sc);
+      pd_forward_pass<P, R>(a, prog, rd, classes, sigs, lane, sc, a.v.pd_entries + region.seq_off + info.seq, info.len);
+      pd_finalize<P, R>(a, task, region, prog, lane, sc);
     } else {
       PdScratch<P, R> sc(scratch, smem, prog.n_slots);
-      pd_forward_pass<P, R, G>(a, prog, rd, classes, sigs, lane, sc, nullptr, 0);
-      pd_finalize<P, R, G>(a, task, region, prog, lane, sc);
+      pd_forward_pass<P, R>(a, prog, rd, classes, sigs, lane, sc, nullptr, 0);
+      pd_finalize<P, R>(a, task, region, prog, lane, sc);
     }
     __syncwarp();
   }
@@ -521,7 +519,7 @@ constexpr size_t pd_long_smem_per_warp() {
 // One superstep of a warp: steps t0 .. t0 + kChunk - 1. kInner: every lane is strictly inside the haplotype
 // throughout, so no events and no bounds.
 template <class P, int R, bool kGeneric, bool kInner>
-__device__ __forceinline__ void pd_long_superstep(const LaunchArgs& a, const ReadRef* rd, int lane, const PdRows<P, R, 32>& pr,
+__device__ __forceinline__ void pd_long_superstep(const LaunchArgs& a, const ReadRef* rd, int lane, const PdRows<P, R>& pr,
                                                   typename P::V an, PdScratch<P, R>& sc, PdState<P, R>& st, const uint32_t* seq,
                                                   const uint32_t* sigs, int n, int t0, const Carry<P>* in, Carry<P>* out,
                                                   int out_mask) {
@@ -540,7 +538,7 @@ __device__ __forceinline__ void pd_long_superstep(const LaunchArgs& a, const Rea
     const Carry<P> c = in[t & (kRing - 1)];
     st.cX = c.x;
     st.cT = c.t;
-    pd_step<P, R, 32, !kInner, true, kGeneric>(a, prog, rd, lane, pr, an, sc, st, n, e, sig);
+    pd_step<P, R, !kInner, true, kGeneric>(a, prog, rd, lane, pr, an, sc, st, n, e, sig);
     const int p = t - 31;  // lane 31's column
     if (lane == 31 && out && (kInner || (p >= 0 && p < n))) out[p & out_mask] = Carry<P>{st.xs, st.ts};
   }
@@ -582,7 +580,7 @@ __global__ void __launch_bounds__(kLongWarps * 32, 1) pd_long_kernel(LaunchArgs 
     for (int b0 = 0; b0 < blocks; b0 += warps) {
       const int in_round = min(warps, blocks - b0), b = b0 + w;
       const bool on = w < in_round;
-      PdRows<P, R, 32> pr;
+      PdRows<P, R> pr;
       PdState<P, R> st;
       st.clear();
       Carry<P> next{S(0), S(0)};  // the first warp's input for column t0 + kChunk + lane
@@ -650,14 +648,14 @@ __global__ void __launch_bounds__(kLongWarps * 32, 1) pd_long_kernel(LaunchArgs 
 template <class P, int R>
 void pd_occ(int* blocks, int warps) {
   static std::atomic<int> cache[3][kMaxDevices];
-  *blocks = resident_blocks(pd_kernel<P, R, 32>, warps * PdLayout<P, R>::kSmemPerWarp, warps * 32, cache[warps_index(warps)],
+  *blocks = resident_blocks(pd_kernel<P, R>, warps * PdLayout<P, R>::kSmemPerWarp, warps * 32, cache[warps_index(warps)],
                             kWarpsPerBlock * PdLayout<P, R>::kSmemPerWarp);
 }
 
 template <class P, int R>
 cudaError_t pd_go(int blocks, const LaunchArgs& a, cudaStream_t s, int warps) {
   const size_t smem = warps * PdLayout<P, R>::kSmemPerWarp;
-  pd_kernel<P, R, 32><<<blocks, warps * 32, smem, s>>>(a);
+  pd_kernel<P, R><<<blocks, warps * 32, smem, s>>>(a);
   return cudaGetLastError();
 }
 

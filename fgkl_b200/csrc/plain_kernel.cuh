@@ -43,8 +43,9 @@
 // column (SNAP, END, NODE) and then the loads for its own (BEGIN, SWEEP). Start states come from a
 // per-warp staging buffer in shared memory, one record per lane: the previous segment writes it
 // directly when it is the snapshot's last writer, otherwise the state is prefetched from global
-// scratch with cp.async at the previous segment's BEGIN, after that BEGIN has read the record. Joins only store their forward column; the products
-// with the backward node are summed after the sweep, warp-wide, in an order fixed by the read row.
+// scratch with cp.async at the previous segment's BEGIN, after that BEGIN has read the record. Joins only
+// store their forward column; the products with the backward node are summed after the sweep, warp-wide, in
+// an order fixed by the read row.
 #include <cuda_pipeline.h>
 #include <cuda_runtime.h>
 
@@ -584,7 +585,7 @@ __device__ __forceinline__ void forward_pass(const LaunchArgs& a, const Program&
     // code, which the compiler schedules across the steps (two steps an iteration: 10% slower without
     // events); in the others one copy of the step with event code runs four times (four copies: 11%
     // slower on uneven regions, for their size).
-        constexpr int kSteps = 4;
+    constexpr int kSteps = 4;
     const uint32_t keep = gl == G - 1 ? kEvMask : (kEvMask & ~(EV_END | EV_ACC));
     uint32_t next[kSteps];
 #pragma unroll

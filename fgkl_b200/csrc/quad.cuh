@@ -1,5 +1,5 @@
-// The quad form's kernels of kLo to kHi rows per lane, in FP32x2 or (kDouble) one read a half in FP64, each range instantiated in its quad_*.cu so that they
-// compile side by side.
+// The quad form's kernels of kLo to kHi rows per lane, in FP32x2 or (kDouble) one read a half in FP64, each
+// range instantiated in its quad_*.cu so that they compile side by side.
 #pragma once
 #include "kernels.cuh"
 
