@@ -835,6 +835,10 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       for (int64_t r = first_read[g]; r < first_read[g + 1]; ++r) {
         const int len = static_cast<int>(in.read_off[r + 1] - in.read_off[r]);
         const int bin = queue_bin(len, rp.generic);
+        if (bin <= 8) {
+          queue_cap[bin] += rp.n_distinct;
+          continue;
+        }
         const int few = queue_pair_bin(len, rp.generic, pd, true), many = queue_pair_bin(len, rp.generic, pd, false);
         queue_cap[few] += rp.n_distinct;
         if (few != many) {
@@ -842,7 +846,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
           if (queue_bin_group(bin) == 0) queue_cap[bin] += static_cast<int64_t>(rp.progs.size());  // whole-program tasks
         }
         for (const int q : {few, many}) queue_len[q] = std::max(queue_len[q], len);
-        if (len > 8 * 31 || rp.generic) wide_pairs += R.n_haps;
+        wide_pairs += R.n_haps;
       }
   }
   // A batch that cannot lose more than a few pairs has no use for the other bins.
@@ -1158,7 +1162,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
     std::memset(blob + o_pd_seq + n_pd_seq * sizeof(uint32_t), 0, 16);
     std::memset(blob + o_sigs + n_sigs * sizeof(uint32_t), 0, 16);
     parallel_for(N, std::min(host_threads(), (N + 31) / 32), [&](int64_t g) {
-      const RegionPlan rp = std::move(plans[g]);  // its last use: freed here, by the threads at work
+      const RegionPlan& rp = plans[g];
       const Region& R = regions[g];
       if (!rp.haps.empty()) std::memcpy(blob + o_haps + static_cast<size_t>(R.hap_off) * sizeof(HapInfo), rp.haps.data(), rp.haps.size() * sizeof(HapInfo));
       auto put = [&](const std::vector<uint32_t>& v, int32_t off) {
@@ -1199,6 +1203,8 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
     return rc;
   if ((rc = check(cudaMemcpyAsync(d_in_, st, s_out, cudaMemcpyHostToDevice, copy_), "upload plan"))) return rc;
   if ((rc = check(cudaEventRecord(uploaded_, copy_), "upload event"))) return rc;
+  // The plans of many regions are freed by several threads, while the copies run.
+  if (N >= 512) parallel_for(N, std::min(host_threads(), 16), [&](int64_t g) { plans[g] = RegionPlan(); });
   // Uploaded from the caller's own memory: done before returning, so the caller may reuse it.
   if (direct_reads) {
     upload_guard.s = nullptr;
