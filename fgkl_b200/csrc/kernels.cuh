@@ -91,9 +91,9 @@ __host__ __device__ inline int queue_bin_rows(int bin) { return bin % kRowBins; 
 __host__ __device__ inline int queue_bin_group(int bin) { return bin / kRowBins; }
 // The bin of a single lost pair of a read (a read's whole-program tasks are queue_bin's). `few`: the run lost few
 // pairs of reads above 248 bases (few_pairs), so that a pair's row blocks have warps to run side by side on;
-// else the warps are worth more on pairs of their own (1 pair of 540 bases 0.27 against 0.39 ms, 1,000 pairs
+// else the warps are worth more on pairs of their own (32 pairs of 540 bases 0.27 against 0.39 ms, 1,000 pairs
 // 1.05 against 0.87). In a single block 10 to 14 rows a lane of the plain FP64 form are the faster even then
-// (32 pairs of 350 bases: 0.17 against 0.18 ms); those of the PD form spill registers, and reads of 12 and
+// (16 pairs of 350 bases: 0.17 against 0.18 ms); those of the PD form spill registers, and reads of 12 and
 // more, or that two strip-mined blocks hold with hardly any padding, go strip-mined even when many are lost
 // (1,000 pairs of 480 bases: 1.15 against 2.01 ms; 9,134 of 250 bases 3.2 against 4.5; but 5,977 of 300 bases,
 // padded to 384 rows, 3.2 against 3.0).

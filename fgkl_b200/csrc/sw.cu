@@ -18,11 +18,11 @@
 // Ignore strategies an alternate that occurs exactly in the reference short-circuits to one match
 // (lib.rs:602-607, the last occurrence), found first by the warp testing 32 start positions at a time.
 //
-// The integer ALU pipe bounds the fill (80% active). Measured on 16,384 pairs of 500 x 500 bases: 25 ALU
-// operations a cell, 8 rows a lane 6.31 ms; tagged cells (below) and the traceback by the warp 5.14 ms;
-// steps inside the matrix without edge cases, the end cell's row and column kept only where a strategy
-// looks there 4.43 ms; 16 rows a lane, so that 500 rows are one block and a step's overhead is shared by
-// twice the cells, 3.7 ms (1,100 G cells/s).
+// The integer ALU pipe bounds the fill (85% active; 80% in the plain form). Measured on 16,384 pairs of 500 x
+// 500 bases: 25 ALU operations a cell, 8 rows a lane 6.31 ms; tagged cells (below) and the traceback by the
+// warp 5.14 ms; steps inside the matrix without edge cases, the end cell's row and column kept only where a
+// strategy looks there 4.43 ms; 16 rows a lane, so that 500 rows are one block and a step's overhead is shared
+// by twice the cells, 3.7 ms (1,100 G cells/s).
 #include <algorithm>
 #include <climits>
 #include <cstdint>
