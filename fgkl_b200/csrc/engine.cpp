@@ -591,7 +591,8 @@ Engine::SplitRule Engine::choose_split(const BatchInput& in, const EngineConfig&
            static_cast<double>(rp.fwd.prefixes) / static_cast<double>(rp.fwd.n_segs), 0, 0, 0, 0};
     for (int64_t r = first_read[g]; r < first_read[g + 1]; ++r) {
       const int64_t len = in.read_off[r + 1] - in.read_off[r];
-      ++(rp.generic || len > 8 * 31 || (rp.extra_codes && !cfg.double_precision) ? w.rest : len > kQuadMaxRead ? w.mid_reads : w.short_reads);
+      const bool apart = rp.generic || len > 8 * 31 || (rp.extra_codes && !cfg.double_precision);
+      ++(apart ? w.rest : len > kQuadMaxRead ? w.mid_reads : w.short_reads);
     }
     extra_codes |= rp.extra_codes;
     work.push_back(w);
@@ -856,7 +857,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
   if (n_stream > INT32_MAX || n_seq > INT32_MAX || n_pd_seq > INT32_MAX || n_haps > INT32_MAX)
     return fail(FGKL_E_INVALID_ARGUMENT, "batch too large for 32-bit plan offsets; split it");
 
-  // Tasks: reads sorted longest first; FP32 packs consecutive pairs below 256 bases. A task costs
+  // Tasks: a region's reads sorted longest first and packed in that order by the batch's form. A task costs
   // its region's stream length times its rows, so within a bin (one rows value) the costliest
   // regions' tasks come first: regions are visited in that order (ties by index), which lists each
   // bin's tasks longest first without sorting them.
@@ -944,8 +945,7 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       // PD in FP64: one read per warp.
       for (; i < order.size(); ++i) one(Kind::kOneF64Pd, single_rows(len_of(order[i])), i);
     } else if (pd) {
-      // PD in FP32: reads above 248 bases one per warp, the others in pairs (FP32x2) unless the
-      // launch configuration asks for one read per warp.
+      // PD in FP32: reads above 248 bases one per warp, the others by the batch's form, one or two (FP32x2).
       for (; i < order.size() && (packed_rows(len_of(order[i])) > 8 || split.reads == 1); ++i)
         one(Kind::kOneF32Pd, single_rows(len_of(order[i])), i);
       for (; i < order.size(); i += 2) two(Kind::kPackedF32Pd, packed_rows(len_of(order[i])), i);
@@ -1023,7 +1023,8 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
         tasks.push_back(e.second);
         cost += e.first;
       }
-      const bool fp32 = b.kind == Kind::kShortF32 || b.kind == Kind::kPackedF32 || b.kind == Kind::kQuadF32 || b.kind == Kind::kOneF32 || b.kind == Kind::kPackedF32Pd || b.kind == Kind::kOneF32Pd;
+      const bool fp32 = b.kind == Kind::kShortF32 || b.kind == Kind::kPackedF32 || b.kind == Kind::kQuadF32 ||
+                        b.kind == Kind::kOneF32 || b.kind == Kind::kPackedF32Pd || b.kind == Kind::kOneF32Pd;
       const bool pipelined = is_long(b.kind);
       b.warps = pipelined ? choose_long_warps(b.kind, b.rows, sms_, bl.pairs) : (fp32 ? tuning_.warps_per_block : kWarpsPerBlock);
       int per_sm = 0, threads = 0;
@@ -1073,7 +1074,8 @@ int Engine::prepare(const BatchInput& in, const EngineConfig& cfg) {
       Bin b{kind, r, queue_off[q], cap, 0, 0, 0};
       // Many pairs: two warps a pair, so that the longest does not run on alone for long (1,000 pairs of 700
       // bases 1.62 ms against 1.45 at one, 300 of 1,200 bases 1.86 against 2.25), one for short ones.
-      if (pipelined) b.warps = group < 3 ? (long_blocks(queue_len[q], r) > (group == 1 ? 2 : 4) ? 2 : 1) : long_warps(long_blocks(queue_len[q], r));
+      const int row_blocks = pipelined ? long_blocks(queue_len[q], r) : 0;
+      if (pipelined) b.warps = group >= 3 ? long_warps(row_blocks) : (row_blocks > (group == 1 ? 2 : 4) ? 2 : 1);
       occupancy(kind, r, &per_sm, &threads, b.warps);
       if (per_sm <= 0) return fail(FGKL_E_CUDA, "recomputation kernel unavailable on this device");
       b.queue_bin = q;

@@ -22,7 +22,7 @@ __device__ __forceinline__ bool queue_pair(const CollectArgs& a, int bin, int re
 }
 
 // Queues what the first pass lost for FP64 recomputation, in the queue bin of the read's form and
-// rows-per-lane (queue_bin), one warp per read. After an FP32 pass, a read of a shared program lost
+// rows-per-lane (queue_bin, queue_pair_bin), one warp per read. After an FP32 pass, a read of a shared program lost
 // against at least a third of its haplotypes (duplicates counted, fgkl lib.rs:495-505) is queued once,
 // as a whole-program task that fills in every lost pair of the read with one shared sweep, when that
 // sweep is the cheaper one; any other lost pair is queued as (read, distinct sorted haplotype), swept
